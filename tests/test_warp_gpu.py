@@ -72,6 +72,29 @@ def test_orders_match_the_oracle_with_large_displacements(O):
             assert np.array_equal(host(w), ref, equal_nan=True), (order, pad)
 
 
+@pytest.mark.parametrize("fdim", [(1, 1, 1), (3, 5, 2), (4, 4, 4), (37, 6, 5)])
+@pytest.mark.parametrize("order", [0, 1, 3])
+def test_windows_on_volumes_near_the_window_size(O, fdim, order):
+    """Floating volumes from one voxel to one where some warps lie wholly inside: every window that
+    leaves the volume, wherever it does, and positions on voxels, faces and far outside."""
+    rng = np.random.default_rng(fdim[0])
+    c = make_case(shape=(6, 7, 40), seed=38)
+    pix = (1.0, 1.0, 1.0)
+    g = nrb.make_geometry(c.rdim, c.rpix, c.rxyz, fdim, pix, nrb.identity_header(pix), c.cdim, c.cpix, c.cxyz)
+    flo = rng.normal(0, 100, int(np.prod(fdim))).astype(np.float32)
+    pos = np.stack([rng.uniform(-4, n + 3, c.nvox) for n in fdim]).astype(np.float32)
+    pos[:, :64] = np.round(pos[:, :64])
+    pos[:, 64:96] = 1.0e9
+    mid = slice(96, c.nvox // 2)  # warps whose windows can all be inside
+    for a, n in enumerate(fdim):
+        pos[a, mid] = rng.uniform(min(1, n - 1), max(1, n - 3), mid.stop - mid.start)
+    for pad in (math.nan, 2.5):
+        w = torch.empty(c.nvox, dtype=torch.float32, device="cuda")
+        nrb.resample_image_order(g, dev(flo), dev(pos.ravel()), w, order, padding=pad)
+        ref = O.resample_order(flo, fdim, np.eye(4, dtype=np.float32), pos.ravel(), c.rdim, order, pad=pad)
+        assert np.array_equal(host(w), ref, equal_nan=True)
+
+
 def test_mask_leaves_voxels_untouched(O):
     c = make_case(seed=34, disp=2.0)
     g = c.geometry()
