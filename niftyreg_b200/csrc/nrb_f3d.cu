@@ -21,7 +21,7 @@ namespace nrb {
 
 // defined in nrb_ops.cu
 nrb_status smooth_and_downsample(const float *in, const int32_t idim[3], float *out, const int32_t odim[3],
-                                 const float new_xyz[16], const float old_ijk[16], float *tmp, cudaStream_t st);
+                                 const float new_xyz[16], const float old_ijk[16], cudaStream_t st);
 nrb_status grid_identity(const int32_t cdim[3], const float cxyz[16], float *cpp, cudaStream_t st);
 nrb_status grid_refine(const int32_t odim[3], const float *old, const int32_t ndim[3], float *out, cudaStream_t st);
 nrb_status rescale_with(float *img, int64_t n, float lo, float hi, float *fred, cudaStream_t st);
@@ -882,8 +882,6 @@ nrb_status build_pyramids(const float *ref, const float *flo, const ImageDesc& r
     NRB_CUDA(cudaMemcpyAsync(ref_pyr[levels - 1].p, ref, rf.n() * 4, cudaMemcpyDefault, st));
     NRB_CUDA(cudaMemcpyAsync(flo_pyr[levels - 1].p, flo, ff.n() * 4, cudaMemcpyDefault, st));
     if (levels == 1) return NRB_OK;
-    DevBuf tmp;
-    NRB_TRY(tmp.alloc(4 * std::max(rf.n(), ff.n()), st));
     for (int l = levels - 2; l >= 0; --l) {
         // each image halves along its own axes
         hdr[l] = halve(hdr[l + 1]);
@@ -892,15 +890,14 @@ nrb_status build_pyramids(const float *ref, const float *flo, const ImageDesc& r
         NRB_TRY(ref_pyr[l].alloc(hdr[l].n(), st));
         hdr[l].xyz(nxyz);
         hdr[l + 1].ijk(oijk);
-        NRB_TRY(smooth_and_downsample(ref_pyr[l + 1].p, hdr[l + 1].dim, ref_pyr[l].p, hdr[l].dim, nxyz, oijk, tmp.p,
-                                      st));
+        NRB_TRY(smooth_and_downsample(ref_pyr[l + 1].p, hdr[l + 1].dim, ref_pyr[l].p, hdr[l].dim, nxyz, oijk, st));
         NRB_TRY(flo_pyr[l].alloc(fhdr[l].n(), st));
         fhdr[l].xyz(nxyz);
         fhdr[l + 1].ijk(oijk);
         NRB_TRY(smooth_and_downsample(flo_pyr[l + 1].p, fhdr[l + 1].dim, flo_pyr[l].p, fhdr[l].dim, nxyz, oijk,
-                                      tmp.p, st));
+                                      st));
     }
-    return NRB_OK;  // tmp is freed in stream order
+    return NRB_OK;
 }
 
 // The pair's description for a batched level (its walks, buffers, NMI tables, node stage) and
@@ -2353,16 +2350,13 @@ extern "C" nrb_status nrb_image_pyramid(const float *img, const int32_t dim[3], 
     cudaStream_t st = as_stream(stream);
     NRB_CUDA(cudaMemcpyAsync(out + off[levels - 1], img, h[levels - 1].n() * sizeof(float), cudaMemcpyDeviceToDevice,
                              st));
-    if (levels == 1) return NRB_OK;
-    DevBuf tmp;
-    NRB_TRY(tmp.alloc(4 * h[levels - 1].n(), st));
     for (int l = levels - 2; l >= 0; --l) {
         float nxyz[16], oijk[16];
         h[l].xyz(nxyz);
         h[l + 1].ijk(oijk);
-        NRB_TRY(smooth_and_downsample(out + off[l + 1], h[l + 1].dim, out + off[l], h[l].dim, nxyz, oijk, tmp.p, st));
+        NRB_TRY(smooth_and_downsample(out + off[l + 1], h[l + 1].dim, out + off[l], h[l].dim, nxyz, oijk, st));
     }
-    return NRB_OK;  // tmp is freed in stream order
+    return NRB_OK;
 }
 
 // reg_spline_refineControlPointGrid3D's node values (reg-lib/cpu/_reg_localTrans.cpp:1930-2119):

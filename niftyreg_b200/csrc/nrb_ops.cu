@@ -617,62 +617,311 @@ __global__ void k_downsample(int nx, int ny, int nz, int ox, int oy, int oz, Mat
     }
 }
 
+// The smoothing, normalisation and downsampling of one pyramid level in one pass. A block of
+// 32 x 8 threads owns 32 x 8 output columns over a run of output slices: it walks the input slices
+// they need, convolves each along x at the sampled columns and along y at the sampled rows in
+// shared memory (only the values a sampled output reads), and every thread keeps the last
+// 2 * SMOOTH_R + 1 results of its column in registers for the z pass, whose output it divides and
+// stores. Sums are k_conv_axis's, tap for tap; a tap outside the volume adds weight * 0. While no
+// value is NaN the density of an output depends on its indices alone (three short sums); a block
+// that meets a NaN starts its run over with (value, density) pairs.
+//
+// One read of the input and one write of the output, where the three axis passes, the normalisation
+// and the sampling moved 60 bytes per input voxel (and 16 bytes per voxel of temporaries were
+// mapped for each call). Bound by instruction issue now (72% active, 38% of the copy bandwidth):
+// 512x512x320 -> 256x256x160 takes 193 us, the separate passes took about 4 ms. Tiles of 32 x 8
+// outputs: the rows' halo is 6% and the columns' 25%, read from L2, and 256 threads with 64
+// registers keep four blocks per SM in flight across the two barriers of a slice.
+constexpr int SMOOTH_R = 2, SMOOTH_TAPS = 2 * SMOOTH_R + 1, SMOOTH_X = 32, SMOOTH_Y = 8;
+constexpr int SMOOTH_IN_X = 2 * SMOOTH_X + 2 * SMOOTH_R, SMOOTH_IN_Y = 2 * SMOOTH_Y + 2 * SMOOTH_R;
+constexpr int SMOOTH_THREADS = SMOOTH_X * SMOOTH_Y;
+constexpr int SMOOTH_LOADS = (SMOOTH_IN_X * SMOOTH_IN_Y + SMOOTH_THREADS - 1) / SMOOTH_THREADS;
+
+struct SmoothParams {
+    int n[3], o[3], s[3];    // input dims, output dims, shift per axis (0 or 1): output i samples i << s
+    int zrun;                // output slices per block
+    float k[SMOOTH_TAPS];
+};
+
+// sum of the weights of the taps of position p inside [0, n), each times d (a pass over densities)
+__device__ __forceinline__ float smooth_density(const float *k, int p, int n, float d) {
+    float s = 0.f;
+#pragma unroll
+    for (int t = 0; t < SMOOTH_TAPS; ++t)
+        if ((unsigned)(p + t - SMOOTH_R) < (unsigned)n) s = fmaf(k[t], d, s);
+    return s;
+}
+
+// One block's run; returns false (with nothing final written) when !kNan and an input value is NaN
+template <bool kNan, bool kHalve>
+__device__ __forceinline__ bool smooth_run(const SmoothParams& P, const float *__restrict__ in, float *__restrict__ out,
+                                           float (*tile)[SMOOTH_IN_Y * SMOOTH_IN_X], float (*xs)[SMOOTH_IN_Y * SMOOTH_X]) {
+    const int tid = threadIdx.x, lx = tid % SMOOTH_X, ly = tid / SMOOTH_X;
+    const int ox0 = blockIdx.x * SMOOTH_X, oy0 = blockIdx.y * SMOOTH_Y, oz0 = blockIdx.z * P.zrun;
+    const int oz1 = min(oz0 + P.zrun, P.o[2]);
+    const int sx = kHalve ? 1 : P.s[0], sy = kHalve ? 1 : P.s[1], sz = kHalve ? 1 : P.s[2];
+    const int ix0 = (ox0 << sx) - SMOOTH_R, iy0 = (oy0 << sy) - SMOOTH_R;
+    const int wx = ((SMOOTH_X - 1) << sx) + SMOOTH_TAPS, wy = ((SMOOTH_Y - 1) << sy) + SMOOTH_TAPS;
+    const int x = ox0 + lx, y = oy0 + ly;
+    const bool mine = x < P.o[0] && y < P.o[1];
+    const long long plane = (long long)P.n[0] * P.n[1];
+    // the elements of a slice's tile this thread loads: offset in the slice, and byte offset in the
+    // tile (-1: outside the volume or the tile, never written, so the zero stored here stays)
+    int src[SMOOTH_LOADS], dst[SMOOTH_LOADS];
+#pragma unroll
+    for (int l = 0; l < SMOOTH_LOADS; ++l) {
+        const int e = tid + l * SMOOTH_THREADS;
+        const int r = e / wx, c = e - r * wx;
+        const int gx = ix0 + c, gy = iy0 + r;
+        const bool inside = r < wy && (unsigned)gx < (unsigned)P.n[0] && (unsigned)gy < (unsigned)P.n[1];
+        src[l] = inside ? gy * P.n[0] + gx : 0;
+        dst[l] = inside ? 4 * (r * SMOOTH_IN_X + c) : -1;
+        asm volatile("" : "+r"(src[l]), "+r"(dst[l]));  // kept in registers, not recomputed per slice
+    }
+    for (int e = tid; e < SMOOTH_IN_Y * SMOOTH_IN_X; e += SMOOTH_THREADS) tile[0][e] = tile[1][e] = 0.f;
+    __syncthreads();
+    // the density over x and y, and that of a column whose z taps are all inside
+    const float dxy = kNan ? 0.f : smooth_density(P.k, y << sy, P.n[1], smooth_density(P.k, x << sx, P.n[0], 1.f));
+    const float dmid = kNan ? 0.f : smooth_density(P.k, SMOOTH_R, SMOOTH_TAPS, dxy);
+    float v[SMOOTH_TAPS], d[SMOOTH_TAPS];
+#pragma unroll
+    for (int t = 0; t < SMOOTH_TAPS; ++t) v[t] = d[t] = 0.f;
+    const int z0 = (oz0 << sz) - SMOOTH_R, z1 = ((oz1 - 1) << sz) + SMOOTH_R;
+    float next[SMOOTH_LOADS];
+    auto fetch = [&](int z) {
+        if ((unsigned)z >= (unsigned)P.n[2]) return;
+        const float *p = in + z * plane;
+#pragma unroll
+        for (int l = 0; l < SMOOTH_LOADS; ++l)
+            if (dst[l] >= 0) next[l] = __ldg(p + src[l]);
+    };
+    auto slot = [&](int q, int l) -> float& { return *reinterpret_cast<float *>(reinterpret_cast<char *>(tile[q]) + dst[l]); };
+#pragma unroll
+    for (int l = 0; l < SMOOTH_LOADS; ++l) next[l] = 0.f;
+    fetch(z0);
+    int nan = 0;
+    for (int z = z0; z <= z1; ++z) {
+        const bool inz = (unsigned)z < (unsigned)P.n[2];
+#pragma unroll
+        for (int l = 0; l < SMOOTH_LOADS; ++l) {
+            if (dst[l] < 0) continue;
+            const bool use = inz && (!kNan || next[l] == next[l]);
+            slot(0, l) = use ? next[l] : 0.f;
+            if (kNan) slot(1, l) = use ? 1.f : 0.f;
+        }
+        if (z < z1) fetch(z + 1);  // in flight while this slice is convolved
+        // a NaN shows in the sums of the slice it is in (the check of a slice is read one later)
+        if (kNan) __syncthreads();
+        else if (__syncthreads_or(nan)) return false;
+        // along x at the sampled columns of every row of the tile
+#pragma unroll
+        for (int u = 0; u < (SMOOTH_IN_Y + SMOOTH_Y - 1) / SMOOTH_Y; ++u) {
+            const int r = ly + u * SMOOTH_Y;
+            if (r >= wy) break;
+#pragma unroll
+            for (int q = 0; q < (kNan ? 2 : 1); ++q) {
+                const float *row = tile[q] + r * SMOOTH_IN_X + (lx << sx);
+                float in5[SMOOTH_TAPS + 1];
+                if (kHalve) {  // 8-byte aligned: three loads without a bank conflict for the five taps
+#pragma unroll
+                    for (int t = 0; t < SMOOTH_TAPS + 1; t += 2) {
+                        const float2 w = *reinterpret_cast<const float2 *>(row + t);
+                        in5[t] = w.x;
+                        in5[t + 1] = w.y;
+                    }
+                } else {
+#pragma unroll
+                    for (int t = 0; t < SMOOTH_TAPS; ++t) in5[t] = row[t];
+                }
+                float s = 0.f;
+#pragma unroll
+                for (int t = 0; t < SMOOTH_TAPS; ++t) s = fmaf(P.k[t], in5[t], s);
+                xs[q][r * SMOOTH_X + lx] = s;
+            }
+        }
+        __syncthreads();
+        // along y at the sampled rows, into the column's window
+#pragma unroll
+        for (int t = 0; t + 1 < SMOOTH_TAPS; ++t) {
+            v[t] = v[t + 1];
+            if (kNan) d[t] = d[t + 1];
+        }
+#pragma unroll
+        for (int q = 0; q < (kNan ? 2 : 1); ++q) {
+            const float *col = xs[q] + (ly << sy) * SMOOTH_X + lx;
+            float s = 0.f;
+#pragma unroll
+            for (int t = 0; t < SMOOTH_TAPS; ++t) s = fmaf(P.k[t], col[t * SMOOTH_X], s);
+            (q == 0 ? v : d)[SMOOTH_TAPS - 1] = s;
+            nan |= s != s;
+        }
+        // along z: the window is centred on slice z - SMOOTH_R
+        const int zc = z - SMOOTH_R;
+        if (zc < (oz0 << sz) || (zc & sz) != 0 || !mine) continue;
+        float num = 0.f, den = 0.f;
+#pragma unroll
+        for (int t = 0; t < SMOOTH_TAPS; ++t) {
+            num = fmaf(P.k[t], v[t], num);
+            if (kNan) den = fmaf(P.k[t], d[t], den);
+        }
+        if (!kNan) den = zc >= SMOOTH_R && zc + SMOOTH_R < P.n[2] ? dmid : smooth_density(P.k, zc, P.n[2], dxy);
+        float r = num / den;
+        if (kNan) {
+            const float o = __ldg(in + zc * plane + (long long)(y << sy) * P.n[0] + (x << sx));
+            if (o != o) r = o;  // _reg_tools.cpp:1100-1110
+        }
+        out[((long long)(zc >> sz) * P.o[1] + y) * P.o[0] + x] = r;
+    }
+    if (!kNan && __syncthreads_or(nan)) return false;
+    return true;
+}
+
+template <bool kHalve>
+__global__ void __launch_bounds__(SMOOTH_THREADS, 4)
+k_smooth_downsample(const __grid_constant__ SmoothParams P, const float *__restrict__ in, float *__restrict__ out) {
+    __shared__ __align__(16) float tile[2][SMOOTH_IN_Y * SMOOTH_IN_X];
+    __shared__ float xs[2][SMOOTH_IN_Y * SMOOTH_X];
+    if (smooth_run<false, kHalve>(P, in, out, tile, xs)) return;
+    __syncthreads();
+    smooth_run<true, kHalve>(P, in, out, tile, xs);
+}
+
 // ---------------------------------------------------------------------------------------------
 // reductions and element-wise updates
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(NRB_RED_THREADS)
+// [0, n) of `img` as `head` elements before its first 16-byte boundary, `nvec` whole float4s and a
+// tail of at most three.
+struct VecSpan {
+    long long head, nvec, n;
+    __device__ __forceinline__ VecSpan(const float *img, long long count): n(count) {
+        head = min(count, (long long)((16 - (reinterpret_cast<uintptr_t>(img) & 15)) & 15) / 4);
+        nvec = (count - head) / 4;
+    }
+};
+
+// min and max are exact in any order, so the split is free: it is chosen to keep loads in flight
+__global__ void __launch_bounds__(2 * NRB_RED_THREADS, 4)
 k_minmax(long long n, const float *__restrict__ img, float *__restrict__ pmin, float *__restrict__ pmax) {
-    __shared__ float smin[NRB_RED_THREADS], smax[NRB_RED_THREADS];
+    __shared__ float smin[2 * NRB_RED_THREADS / 32], smax[2 * NRB_RED_THREADS / 32];
+    const VecSpan S(img, n);
+    const long long gtid = blockIdx.x * (long long)blockDim.x + threadIdx.x, gs = (long long)gridDim.x * blockDim.x;
     float mn = FLT_MAX, mx = -FLT_MAX;
-    for (long long i = blockIdx.x * (long long)NRB_RED_THREADS + threadIdx.x; i < n;
-         i += (long long)gridDim.x * NRB_RED_THREADS) {
-        const float v = img[i];
+    auto take = [&](float v) {
         if (v == v) {
             mn = fminf(mn, v);
             mx = fmaxf(mx, v);
         }
-    }
-    smin[threadIdx.x] = mn;
-    smax[threadIdx.x] = mx;
-    __syncthreads();
-    for (int s = NRB_RED_THREADS / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            smin[threadIdx.x] = fminf(smin[threadIdx.x], smin[threadIdx.x + s]);
-            smax[threadIdx.x] = fmaxf(smax[threadIdx.x], smax[threadIdx.x + s]);
+    };
+    const float4 *vec = reinterpret_cast<const float4 *>(img + S.head);
+    long long i = gtid;
+    for (; i + gs < S.nvec; i += 2 * gs) {
+        float4 q[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) q[u] = __ldg(vec + i + u * gs);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            take(q[u].x);
+            take(q[u].y);
+            take(q[u].z);
+            take(q[u].w);
         }
-        __syncthreads();
     }
+    for (; i < S.nvec; i += gs) {
+        const float4 q = __ldg(vec + i);
+        take(q.x);
+        take(q.y);
+        take(q.z);
+        take(q.w);
+    }
+    if (gtid < S.head) take(img[gtid]);
+    const long long tail = S.head + 4 * S.nvec + gtid;
+    if (tail < n) take(img[tail]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        smin[threadIdx.x >> 5] = mn;
+        smax[threadIdx.x >> 5] = mx;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        pmin[blockIdx.x] = smin[0];
-        pmax[blockIdx.x] = smax[0];
+        for (int w = 1; w < (int)blockDim.x / 32; ++w) {
+            mn = fminf(mn, smin[w]);
+            mx = fmaxf(mx, smax[w]);
+        }
+        pmin[blockIdx.x] = mn;
+        pmax[blockIdx.x] = mx;
     }
 }
 
 // reg_intensityRescale_core (reg-lib/cpu/_reg_tools.cpp:92-174): double-precision rescale of
 // the finite values; every block combines the min/max partials itself.
-__global__ void k_rescale(long long n, float *__restrict__ img, const float *__restrict__ pmin,
-                          const float *__restrict__ pmax, int np, float new_min, float new_max) {
-    __shared__ float mm[2];
-    if (threadIdx.x == 0) {
-        float mn = FLT_MAX, mx = -FLT_MAX;
-        for (int i = 0; i < np; ++i) {
-            mn = fminf(mn, pmin[i]);
-            mx = fmaxf(mx, pmax[i]);
-        }
-        mm[0] = mn;
-        mm[1] = mx;
+//
+// The quotient by the range is the correctly rounded one from the rounded reciprocal and one
+// residual step (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990): three FP64 operations per voxel instead of a division.
+// It needs a finite, normal range and quotient; other ranges (infinite values, a constant image)
+// are divided. Four floats per load and store. 512x512x320: min/max 54 us, rescale 140 us (74% of
+// the copy bandwidth; FP64 division and single floats before).
+__global__ void __launch_bounds__(256)
+k_rescale(long long n, float *__restrict__ img, const float *__restrict__ pmin, const float *__restrict__ pmax, int np,
+          float new_min, float new_max) {
+    __shared__ float smin[8], smax[8];
+    float mn = FLT_MAX, mx = -FLT_MAX;
+    for (int i = threadIdx.x; i < np; i += blockDim.x) {
+        mn = fminf(mn, pmin[i]);
+        mx = fmaxf(mx, pmax[i]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        smin[threadIdx.x >> 5] = mn;
+        smax[threadIdx.x >> 5] = mx;
     }
     __syncthreads();
-    const double cur = (double)(mm[1] - mm[0]), nd = (double)(new_max - new_min), lo = (double)mm[0];
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        double v = (double)img[i];
-        if (v == v) {
-            v = (v - lo) / cur;
-            v = v * nd + new_min;
-        }
-        img[i] = (float)v;
+    mn = smin[0];
+    mx = smax[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) {
+        mn = fminf(mn, smin[w]);
+        mx = fmaxf(mx, smax[w]);
     }
+    const double cur = (double)(mx - mn), nd = (double)(new_max - new_min), lo = (double)mn;
+    const bool by_reciprocal = cur > 1e-30 && cur < 1e38;
+    const double inv = 1.0 / cur;
+    auto one = [&](float f) {
+        double v = (double)f;
+        if (v == v) {
+            const double a = v - lo;
+            if (by_reciprocal) {
+                const double q = a * inv;
+                v = fma(fma(-cur, q, a), inv, q);
+            } else {
+                v = a / cur;
+            }
+            v = fma(v, nd, (double)new_min);
+        }
+        return (float)v;
+    };
+    const VecSpan S(img, n);
+    const long long gtid = blockIdx.x * (long long)blockDim.x + threadIdx.x, gs = (long long)gridDim.x * blockDim.x;
+    float4 *vec = reinterpret_cast<float4 *>(img + S.head);
+    for (long long i = gtid; i < S.nvec; i += gs) {
+        float4 q = vec[i];
+        q.x = one(q.x);
+        q.y = one(q.y);
+        q.z = one(q.z);
+        q.w = one(q.w);
+        vec[i] = q;
+    }
+    if (gtid < S.head) img[gtid] = one(img[gtid]);
+    const long long tail = S.head + 4 * S.nvec + gtid;
+    if (tail < n) img[tail] = one(img[tail]);
 }
 
 // reg_getMaximalLength (reg-lib/cpu/_reg_tools.cpp:335-355): float lengths, max is exact in any
@@ -1592,10 +1841,10 @@ extern "C" nrb_status nrb_approx_bending_energy_gradient(nrb_workspace *ws, cons
 
 // fred holds two partial arrays of NRB_RED_BLOCKS floats (min | max)
 static nrb_status rescale_impl(float *img, int64_t n, float lo, float hi, float *fred, cudaStream_t st) {
-    const int np = (int)std::max<long long>(1, std::min<long long>((n + NRB_RED_THREADS - 1) / NRB_RED_THREADS, NRB_RED_BLOCKS));
-    k_minmax<<<np, NRB_RED_THREADS, 0, st>>>(n, img, fred, fred + NRB_RED_BLOCKS);
+    const int np = (int)std::max<long long>(1, std::min<long long>((n + 8 * NRB_RED_THREADS - 1) / (8 * NRB_RED_THREADS), NRB_RED_BLOCKS));
+    k_minmax<<<np, 2 * NRB_RED_THREADS, 0, st>>>(n, img, fred, fred + NRB_RED_BLOCKS);
     NRB_LAUNCHED("k_minmax");
-    k_rescale<<<grid_for(n, 256), 256, 0, st>>>(n, img, fred, fred + NRB_RED_BLOCKS, np, lo, hi);
+    k_rescale<<<grid_for((n + 3) / 4, 256, 8), 256, 0, st>>>(n, img, fred, fred + NRB_RED_BLOCKS, np, lo, hi);
     NRB_LAUNCHED("k_rescale");
     return NRB_OK;
 }
@@ -1702,20 +1951,74 @@ extern "C" nrb_status nrb_conjugate_gradient(nrb_workspace *ws, float *grad, flo
 // ---------------------------------------------------------------------------------------------
 namespace nrb {
 
+// Whether new_xyz followed by old_ijk, rounded (k_downsample), takes every voxel i of the new image
+// to i << shift: the composed map is within 0.05 voxel of that at the corners (it is affine), and the
+// float evaluation's error stays far below the rest of the rounding margin. True for every header
+// the pyramid derives by halving; a degenerate matrix fails it and takes the separate passes.
+static bool samples_every_other(const int32_t idim[3], const int32_t odim[3], const float new_xyz[16],
+                                const float old_ijk[16], int shift[3]) {
+    double mm = 0, ij = 0;
+    for (int i = 0; i < 12; ++i) {
+        if (!std::isfinite(new_xyz[i]) || !std::isfinite(old_ijk[i])) return false;
+        mm += std::fabs((double)new_xyz[i]) * (i % 4 < 3 ? odim[i % 4] : 1);
+        ij = std::max(ij, std::fabs((double)old_ijk[i]));
+    }
+    double off = 0;
+    for (int i = 0; i < 3; ++i) off = std::max(off, std::fabs((double)old_ijk[4 * i + 3]));
+    if (!(16.0 * std::ldexp(1.0, -24) * (3.0 * ij * mm + off) < 0.2)) return false;
+    for (int i = 0; i < 3; ++i) {
+        shift[i] = odim[i] == idim[i] ? 0 : 1;
+        if (((long long)(odim[i] - 1) << shift[i]) >= idim[i]) return false;
+        double t = old_ijk[4 * i + 3];
+        for (int k = 0; k < 3; ++k) t += (double)old_ijk[4 * i + k] * new_xyz[4 * k + 3];
+        double dev = std::fabs(t);
+        for (int j = 0; j < 3; ++j) {
+            double m = 0;
+            for (int k = 0; k < 3; ++k) m += (double)old_ijk[4 * i + k] * new_xyz[4 * k + j];
+            dev += std::fabs(m - (i == j ? 1 << shift[i] : 0)) * (odim[j] - 1);
+        }
+        if (!(dev < 0.05)) return false;
+    }
+    return true;
+}
+
 // Gaussian smoothing of reg_downsampleImage (sigma = -0.7355 voxel, all three axes in one
 // reg_tools_kernelConvolution call, density normalised once at the end), then nearest-neighbour
-// downsampling. tmp needs 4 * nvox(in) floats.
+// downsampling.
 nrb_status smooth_and_downsample(const float *in, const int32_t idim[3], float *out, const int32_t odim[3],
-                                 const float new_xyz[16], const float old_ijk[16], float *tmp, cudaStream_t st) {
+                                 const float new_xyz[16], const float old_ijk[16], cudaStream_t st) {
     const double temp = 0.7355;  // |sigma|, voxel units
     const int radius = (int)(temp * 3.0f);
+    static_assert((int)(0.7355 * 3.0f) == SMOOTH_R, "the fused smoothing is written for this radius");
     std::vector<float> k(2 * radius + 1);
     for (int i = -radius; i <= radius; ++i)
         k[radius + i] = (float)(std::exp(-(double)(i * i) / (2.0 * temp * temp)) / (temp * 2.506628274631));
-    float *dk = nullptr;
-    NRB_CUDA(tmp_alloc(&dk, k.size() * 4, st));
-    NRB_CUDA(cudaMemcpyAsync(dk, k.data(), k.size() * 4, cudaMemcpyHostToDevice, st));
+    SmoothParams P;
+    // slices are addressed with 32-bit offsets in the fused pass
+    if ((long long)idim[0] * idim[1] < (1LL << 31) && samples_every_other(idim, odim, new_xyz, old_ijk, P.s)) {
+        for (int i = 0; i < 3; ++i) {
+            P.n[i] = idim[i];
+            P.o[i] = odim[i];
+        }
+        for (int i = 0; i < SMOOTH_TAPS; ++i) P.k[i] = k[i];
+        const dim3 cols((odim[0] + SMOOTH_X - 1) / SMOOTH_X, (odim[1] + SMOOTH_Y - 1) / SMOOTH_Y);
+        // runs of output slices: two rounds of resident blocks when the volume has that many, no
+        // run shorter than 4 slices (the 2 * SMOOTH_R slices a run re-reads)
+        const long long want = std::max<long long>(1, 2LL * 4 * sm_count() / ((long long)cols.x * cols.y));
+        P.zrun = std::max(4, (int)((odim[2] + want - 1) / want));
+        const unsigned runs = (unsigned)((odim[2] + P.zrun - 1) / P.zrun);
+        if (cols.y <= 65535 && runs <= 65535) {
+            auto kernel = P.s[0] && P.s[1] && P.s[2] ? k_smooth_downsample<true> : k_smooth_downsample<false>;
+            kernel<<<dim3(cols.x, cols.y, runs), SMOOTH_THREADS, 0, st>>>(P, in, out);
+            NRB_LAUNCHED("k_smooth_downsample");
+            return NRB_OK;
+        }
+    }
+    float *dk = nullptr, *tmp = nullptr;
     const long long nv = nvox(idim);
+    NRB_CUDA(tmp_alloc(&dk, k.size() * 4, st));
+    NRB_CUDA(tmp_alloc(&tmp, 4 * nv * sizeof(float), st));
+    NRB_CUDA(cudaMemcpyAsync(dk, k.data(), k.size() * 4, cudaMemcpyHostToDevice, st));
     float *v0 = tmp, *d0 = tmp + nv, *v1 = tmp + 2 * nv, *d1 = tmp + 3 * nv;
     const int g = grid_for(nv, 256);
     k_conv_axis<<<g, 256, 0, st>>>(idim[0], idim[1], idim[2], 0, in, nullptr, dk, radius, v0, d0);
@@ -1731,6 +2034,7 @@ nrb_status smooth_and_downsample(const float *in, const int32_t idim[3], float *
                                                     to_mat34(new_xyz), to_mat34(old_ijk), v1, out);
     NRB_LAUNCHED("k_downsample");
     NRB_CUDA(cudaFreeAsync(dk, st));
+    NRB_CUDA(cudaFreeAsync(tmp, st));
     return NRB_OK;
 }
 

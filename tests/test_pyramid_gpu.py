@@ -83,6 +83,85 @@ def test_pyramid_levels_match_reference(name):
         assert err <= 1e-6, (l, err)
 
 
+def _level64(img, down):
+    """One level of the pyramid in double: the normalised Gaussian (sigma 0.7355, radius 2, float
+    weights) along x, y and z over the finite values, every `down`-th voxel kept, NaN kept."""
+    k = np.exp(-np.arange(-2, 3) ** 2 / (2 * 0.7355 ** 2)) / (0.7355 * 2.506628274631)
+    k = k.astype(np.float32).astype(np.float64)
+    ok = ~np.isnan(img)
+    num, den = np.where(ok, img, 0).astype(np.float64), ok.astype(np.float64)
+    for axis in (2, 1, 0):
+        num, den = (np.apply_along_axis(lambda a: np.convolve(a, k, "same"), axis, q) for q in (num, den))
+    with np.errstate(invalid="ignore", divide="ignore"):
+        out = np.where(ok, num / den, np.nan)
+    return out[::down[0], ::down[1], ::down[2]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(64, 64, 64), (65, 67, 129), (63, 72, 200), (5, 64, 66)])
+def test_pyramid_level_on_tile_edges(shape):
+    """One halving at the edges of the smoothing's tiles (32 x 8 outputs, runs along z), axes that
+    keep their size, with and without NaN voxels; 1e-6 of the largest magnitude as above. Outputs
+    out of a NaN's reach are the same floats with it as without it, and so are all outputs of an
+    origin whose coordinates are too large for the fused pass (2^20 mm: still exact, so the
+    separate passes sample the same voxels)."""
+    import torch
+    ensure_built()
+    nz, ny, nx = shape
+    rng = np.random.default_rng(nz)
+    img = rng.normal(300, 100, shape).astype(np.float32)
+    bad = img.copy()
+    bad[nz // 2, ny // 3, nx // 2] = np.nan
+    bad[0, 0, 0] = np.nan
+    down = [2 if n // 2 >= 32 else 1 for n in shape]
+    got = {}
+    for name, data, origin in (("plain", img, 0.0), ("nan", bad, 0.0), ("far", bad, 2.0 ** 20)):
+        xyz = nrb.identity_header((1.0, 1.0, 1.0), (origin,) * 3)
+        dims, _, total = nrb.image_pyramid_headers((nx, ny, nz), (1.0, 1.0, 1.0), xyz, 2)
+        out = torch.empty(total, dtype=torch.float32, device="cuda")
+        nrb.image_pyramid(torch.from_numpy(data.ravel()).cuda(), (nx, ny, nz), (1.0, 1.0, 1.0), xyz, 2, out)
+        n = int(np.prod(dims[0]))
+        got[name] = out.cpu().numpy()[:n].reshape(dims[0][::-1])
+        want = _level64(data, down)
+        assert got[name].shape == want.shape
+        assert np.array_equal(np.isnan(got[name]), np.isnan(want))
+        assert np.nanmax(np.abs(got[name] - want)) <= 1e-6 * np.nanmax(np.abs(want)), name
+    assert np.array_equal(got["nan"], got["far"], equal_nan=True)
+    reach = np.zeros(shape, bool)
+    for z, y, x in np.argwhere(np.isnan(bad)):
+        reach[max(0, z - 2):z + 3, max(0, y - 2):y + 3, max(0, x - 2):x + 3] = True
+    keep = ~reach[::down[0], ::down[1], ::down[2]]
+    assert np.array_equal(got["plain"][keep], got["nan"][keep])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 17, 2049, 1000003])
+@pytest.mark.parametrize("offset", [0, 1, 3])
+def test_rescale_at_odd_lengths_and_alignments(n, offset):
+    """nrb_intensity_rescale against the oracle, bit for bit: lengths around the vector width, bases
+    off the 16-byte boundary, NaN values, a constant image (0 / 0), infinite values; the floats on
+    either side of the range stay as they were."""
+    import torch
+    ensure_built()
+    O = oracle.Restated()
+    rng = np.random.default_rng(n + offset)
+    for kind in ("values", "constant", "infinite"):
+        img = np.full(n, 3.0, np.float32) if kind == "constant" else rng.normal(0, 500, n).astype(np.float32)
+        if kind == "values" and n > 4:
+            img[rng.random(n) < 0.1] = np.nan
+        if kind == "infinite":
+            img[n // 2] = np.inf
+        buf = np.full(n + 8, -5.0, np.float32)
+        buf[offset:offset + n] = img
+        t = torch.from_numpy(buf).cuda()
+        nrb.intensity_rescale(t[offset:], n, 2.0, 65.0)
+        out = t.cpu().numpy()
+        with np.errstate(invalid="ignore"):
+            want = O.intensity_rescale(img, 2.0, 65.0)
+        assert np.array_equal(out[offset:offset + n], want, equal_nan=True), kind
+        assert np.all(out[:offset] == -5.0) and np.all(out[offset + n:] == -5.0)
+
+
 REFINES = {
     # reference (nz, ny, nx), pixdim, spacing mm at the coarse level
     "even": ((64, 64, 64), (1.0, 1.0, 1.0), 10.0),
