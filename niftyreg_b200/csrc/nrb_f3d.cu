@@ -1708,6 +1708,7 @@ extern "C" nrb_status nrb_f3d_register_host(const float *ref_host, const float *
 // ---------------------------------------------------------------------------------------------
 namespace nrb {
 
+int64_t velocity_field_stride(int64_t nvox);
 nrb_status velocity_to_deformation(const nrb_geometry *g, const float *vel, bool update, int *steps, float *def,
                                    float *fields, float *scratch, unsigned *minmax, cudaStream_t st);
 nrb_status exponentiate_gradient(const nrb_geometry *g, const float *vel_other, int steps, float *vgrad,
@@ -1819,7 +1820,7 @@ private:
     float *bw(DevBuf& b) { return b.p + 3 * nc_; }
 
     nrb_status Fields(int64_t nvox_max) {
-        const int64_t need = (int64_t)steps_ * 3 * nvox_max;
+        const int64_t need = (int64_t)steps_ * velocity_field_stride(nvox_max);
         if (need > fields_n_) {
             NRB_TRY(fields_.alloc(need, st_));
             fields_n_ = need;

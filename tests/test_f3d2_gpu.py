@@ -116,6 +116,62 @@ def test_exponentiated_gradient_matches_reference(R):
     assert np.array_equal(out, ref)
 
 
+def _rotated(xyz, angle=0.2):
+    c, s = np.cos(angle), np.sin(angle)
+    r = np.eye(4)
+    r[:2, :2] = [[c, -s], [s, c]]
+    return (r @ xyz.astype(np.float64)).astype(np.float32)
+
+
+# field dims, node spacing (mm) and amplitude: dims around the flow's 32 x 8 x 4 blocks, odd voxel
+# counts (fields and user buffers then start off the 8-byte boundary), nodes closer than the voxels,
+# many voxels per node, an even and an odd squaring number, a grid short of the field, flipped and
+# rotated images
+@pytest.mark.parametrize("fdim,spacing,amp,margin,orient", [
+    ((33, 9, 5), 5.0, 2.0, 1, "plain"), ((31, 7, 3), 4.0, 40.0, 1, "plain"), ((32, 8, 4), 0.7, 1.0, 1, "plain"),
+    ((45, 11, 13), 16.0, 2.0, 1, "plain"), ((21, 19, 17), 4.0, 2.0, -2, "plain"), ((21, 19, 17), 4.0, 2.0, 1, "flipped"),
+    ((21, 19, 17), 4.0, 2.0, 3, "rotated"), ((2, 2, 2), 3.0, 1.0, 1, "plain")])
+def test_velocity_operations_are_the_oracles(fdim, spacing, amp, margin, orient):
+    ensure_built()
+    O = oracle.Restated()
+    rng = np.random.default_rng(fdim[0])
+    fpix = (1.0, 1.1, 0.9)
+    fxyz = nrb.identity_header(fpix, (-3.0, 2.0, 1.5))
+    if orient == "flipped":
+        fxyz[0, 0], fxyz[0, 3] = -fxyz[0, 0], -3.0 + fpix[0] * (fdim[0] - 1)
+        fxyz[2, 2], fxyz[2, 3] = -fxyz[2, 2], 1.5 + fpix[2] * (fdim[2] - 1)
+    if orient == "rotated":
+        fxyz = _rotated(fxyz)
+    gdim = [int(np.ceil(n * p / spacing + 3)) + margin for n, p in zip(fdim, fpix)]
+    gxyz = nrb.identity_header((spacing,) * 3, [o - spacing - 0.5 for o in (-3.0, 2.0, 1.5)])
+    ident = identity_grid(gdim, gxyz)
+    vel = (ident + rng.normal(0, amp, ident.size)).astype(np.float32)
+    g = nrb.make_geometry(fdim, fpix, fxyz, fdim, fpix, fxyz, gdim, (spacing,) * 3, gxyz)
+    n = int(np.prod(fdim))
+    for update, steps_in in ((False, 6), (False, 5), (True, 6)):
+        want, want_steps = O.velocity_def_field(vel, gdim, gxyz, steps_in, update, fdim, fxyz)
+        for offset in (0, 1):  # an output that starts off the 8-byte boundary
+            buf = torch.full((3 * n + 2,), -9.0, device="cuda")
+            steps = nrb.get_def_field_from_velocity_grid(g, dev(vel), steps_in, buf[offset:], update=update)
+            out = host(buf)
+            assert steps == want_steps
+            assert np.array_equal(out[offset:offset + 3 * n], want)
+            assert np.all(out[:offset] == -9.0) and np.all(out[offset + 3 * n:] == -9.0)
+    for steps in (1, 2, 5, 6):
+        vg = rng.normal(0, 1.0, 3 * n).astype(np.float32)
+        want = O.exponentiate_gradient(fdim, fxyz, vel, gdim, gxyz, steps, vg)
+        for offset in (0, 1):
+            buf = torch.full((3 * n + 2,), -9.0, device="cuda")
+            buf[offset:offset + 3 * n] = dev(vg)
+            nrb.exponentiate_gradient(g, dev(vel), steps, buf[offset:])
+            out = host(buf)
+            if orient == "rotated":  # the orthogonal factor's last bits: as the oracle's own bar
+                assert np.abs(out[offset:offset + 3 * n] - want).max() <= 3e-7 * np.abs(want).max() * steps
+            else:
+                assert np.array_equal(out[offset:offset + 3 * n], want)
+            assert np.all(out[:offset] == -9.0) and np.all(out[offset + 3 * n:] == -9.0)
+
+
 def test_symmetrisation_is_bitwise(R):
     c = VelocityCase(55)
     rng = np.random.default_rng(55)
