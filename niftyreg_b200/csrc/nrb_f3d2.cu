@@ -295,7 +295,7 @@ __device__ __forceinline__ void flow_border(const VecField<false>& vel, int gx, 
 // Bound by the FP32 lanes: 464 products and sums per voxel, none fusable (92 us for 182x218x182 at
 // the lane rate). One voxel per thread took 362 us (1280 warp instructions per 32 voxels, 192 of
 // them loads).
-constexpr int kFlowVox = 4;
+constexpr int kFlowVox = 5;
 
 template <bool kExtrema>
 __global__ void __launch_bounds__(256, 2) k_velocity_flow_table(const float *__restrict__ vel, int gx, int gy, int gz,

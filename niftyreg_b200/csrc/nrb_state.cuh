@@ -36,6 +36,31 @@ void flo_texture_release(FloTexture& t);
 nrb_status flo_texture_upload(const FloTexture& t, const float *src, int width, int height, int layers,
                               cudaStream_t st);
 
+// How a walk reads the floating image: dims, row and slice strides with `margin` voxels on every
+// side, and the layered texture that holds it (0: none) with its coordinate limits.
+struct FloatingView {
+    int nx, ny, nz, sy, sz, margin;
+    unsigned long long tex;
+    float tex_off, tex_x, tex_y;  // margin + 1; largest gather coordinates
+    int tex_layer;                // largest lower layer
+};
+
+__host__ __device__ inline FloatingView floating_view(int nx, int ny, int nz, int margin, unsigned long long tex) {
+    FloatingView V;
+    V.nx = nx;
+    V.ny = ny;
+    V.nz = nz;
+    V.margin = margin;
+    V.sy = nx + 2 * margin;
+    V.sz = V.sy * (ny + 2 * margin);
+    V.tex = tex;
+    V.tex_off = (float)(margin + 1);
+    V.tex_x = (float)(nx + 2 * margin - 1);
+    V.tex_y = (float)(ny + 2 * margin - 1);
+    V.tex_layer = nz + 2 * margin - 2;
+    return V;
+}
+
 // Launch-time description of one voxel walk (a pair's reference volume, grid and floating image,
 // and the walk plan's item decomposition).
 struct WalkParams {
@@ -44,13 +69,12 @@ struct WalkParams {
     float gsx, gsy, gsz;     // grid spacing in reference voxels (grid pixdim / ref pixdim)
     int ty, tiles_x, tiles_y, zchunk, nitems;
     int sa, sb, sc;          // shared strides of the staged block (max spans)
-    int fnx, fny, fnz;       // floating dims
-    int fsy, fsz, fmargin;   // floating layout: row and slice strides, margin (sample_floating)
-    unsigned long long ftex; // the floating image with its margin as a layered texture (0: none)
+    FloatingView fv;         // the floating image
     Mat34 flo_ijk;           // mm -> floating voxel
     int flo_diag;            // flo_ijk has no off-diagonal terms
     float pad;               // padding value of out-of-volume taps
     int rb, fb;              // internal bin counts
+    float frb, ffb;          // the same as floats
     int cnv;                 // control points per component
     int log_in_smem;         // gradient: an FP32 copy of the log table is staged in shared memory
     int xs;                  // objective: x-contracted rows of the item staged in shared memory
@@ -183,7 +207,7 @@ struct BatchLaunch {
     int npairs = 0;
     BatchObjTable obj_table;
     BatchGradTable grad_table;
-    bool obj_xs = false, obj_diag = false, grad_f32 = false, grad_diag = false;
+    bool obj_xs = false, obj_diag = false, grad_f32 = false, grad_diag = false, tex = false;
     size_t obj_smem = 0, grad_smem = 0, fin_smem = 0;
     int obj_grid = 0, grad_grid = 0;
 };

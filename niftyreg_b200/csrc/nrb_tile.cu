@@ -224,9 +224,9 @@ __device__ __forceinline__ void column_plane_x(const WalkParams& P, const Column
 
 // World position (mm) of slice index zi (relative to the item) of the thread's column; zi must
 // not decrease between calls. X: the item's x-contracted rows, or null.
-__device__ __forceinline__ void column_position(const WalkParams& P, const Item& I, Column& C, const float *zb,
-                                                const int *zk, const float2 *zid, int zi, float pos[3],
-                                                const float *X = nullptr) {
+template <bool kXs = false>
+__device__ __forceinline__ void column_position(const WalkParams& P, Column& C, const float *zb, const int *zk,
+                                                const float2 *zid, int zi, float pos[3], const float *X = nullptr) {
     const int pz = zk[zi];
     if (pz != C.win) {
         if (pz == C.win + 1) {
@@ -234,12 +234,12 @@ __device__ __forceinline__ void column_position(const WalkParams& P, const Item&
             for (int t = 0; t < 3; ++t)
 #pragma unroll
                 for (int c = 0; c < 3; ++c) C.S[t][c] = C.S[t + 1][c];
-            if (X) column_plane_x(P, C, X, pz + 3, C.S[3]);
+            if (kXs) column_plane_x(P, C, X, pz + 3, C.S[3]);
             else column_plane(P, C, pz + 3, C.S[3]);
         } else {
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-                if (X) column_plane_x(P, C, X, pz + t, C.S[t]);
+                if (kXs) column_plane_x(P, C, X, pz + t, C.S[t]);
                 else column_plane(P, C, pz + t, C.S[t]);
             }
         }
@@ -283,11 +283,14 @@ __device__ __forceinline__ void to_floating_voxel(const Mat34& M, int diag, floa
 }
 
 // floor(v) as float and as int. v is clamped to +-2^21 first: every position that far out lies
-// outside any volume this library accepts, and the clamp keeps px + 1 from overflowing.
+// outside any volume this library accepts, and the clamp keeps px + 1 from overflowing. Adding
+// 1.5 * 2^23 rounded down leaves floor(v) in the sum's low bits (its ulp is 1 there): two additions
+// in place of a rounding and a conversion on the slower conversion pipe, and the same values.
 __device__ __forceinline__ int floor_split(float v, float& fl) {
     v = fminf(fmaxf(v, -2097152.0f), 2097152.0f);
-    fl = floorf(v);
-    return __float2int_rd(v);
+    const float t = __fadd_rd(v, 12582912.0f);
+    fl = __fsub_rn(t, 12582912.0f);
+    return __float_as_int(t) - __float_as_int(12582912.0f);
 }
 
 // (int)v for 0 <= v (truncation == floor there)
@@ -321,77 +324,90 @@ __device__ __forceinline__ void gather_footprint(unsigned long long tex, int lay
     v[0][0] = r3;
 }
 
-// tex (optional; needs margin >= 2): the same floating image with its margin as a 2D layered
-// float array (layer k = slice k - margin, texel (i, j) = voxel (i - margin, j - margin)); every
-// sample then fetches each slice's 2x2 footprint with one gather instead of four loads, with no
-// warp vote and no clamped path.
-template <bool kGrad, int kDiag = -1>
-__device__ __forceinline__ void sample_floating(const float *__restrict__ flo, unsigned long long tex, int fnx, int fny,
-                                                int fnz, int sy, int sz, int margin, const Mat34& M,
-                                                int diag, float pad, float x, float y, float z,
-                                                float& val, float g[3]) {
+// kTex (needs margin >= 2): the same floating image with its margin as a 2D layered float array
+// (layer k = slice k - margin, texel (i, j) = voxel (i - margin, j - margin)); every sample then
+// fetches each slice's 2x2 footprint with one gather instead of four loads, with no warp vote and
+// no clamped path.
+//
+// A sample is fetched in one step and evaluated in another, so that a walk can have the next
+// slice's fetch in flight while it works on this one.
+struct Footprint {
+    float v[2][2][2];  // z, y, x
+    float rx, ry, rz;  // position within the footprint
+};
+
+template <int kDiag, bool kTex>
+__device__ __forceinline__ void fetch_footprint(const float *__restrict__ flo, const FloatingView& V, const Mat34& M,
+                                                int diag, float pad, float x, float y, float z, Footprint& S) {
     float fx, fy, fz;
     to_floating_voxel<kDiag>(M, diag, x, y, z, fx, fy, fz);
     float flx, fly, flz;
     const int px = floor_split(fx, flx), py = floor_split(fy, fly), pz = floor_split(fz, flz);
-    const float rx = fx - flx, ry = fy - fly, rz = fz - flz;
-    const float bx0 = 1.f - rx, by0 = 1.f - ry, bz0 = 1.f - rz;
-    float v[2][2][2];
-    // -margin <= p and p + 1 <= n - 1 + margin on every axis (|p| <= 2^21: no overflow)
-    const bool plain = (unsigned)(px + margin) < (unsigned)(fnx + 2 * margin - 1) &&
-                       (unsigned)(py + margin) < (unsigned)(fny + 2 * margin - 1) &&
-                       (unsigned)(pz + margin) < (unsigned)(fnz + 2 * margin - 1);
-    if (tex) {
+    S.rx = fx - flx;
+    S.ry = fy - fly;
+    S.rz = fz - flz;
+    if (kTex) {
         // every sample, no vote: the footprint's first texel (p + margin on each axis) clamped to
         // [0, n + 2 margin - 2]. Unclamped, that is the plain path's footprint; clamped, both taps
         // on that axis lie outside the volume (p < -margin or p > n + margin - 2) and the clamped
         // footprint lies in the margin (margin >= 2), so they read the padding value, as the
         // clamped path substitutes it. Texels past the padded extent are never read.
-        const float off = (float)(margin + 1);
-        const float tx = fminf(fmaxf(flx + off, 1.f), (float)(fnx + 2 * margin - 1));
-        const float ty = fminf(fmaxf(fly + off, 1.f), (float)(fny + 2 * margin - 1));
-        const int layer = min(max(pz + margin, 0), fnz + 2 * margin - 2);
-        gather_footprint(tex, layer, tx, ty, v[0]);
-        gather_footprint(tex, layer + 1, tx, ty, v[1]);
-    } else if (__all_sync(__activemask(), plain)) {
-        const float *p = flo + (pz * sz + py * sy + px);
-        v[0][0][0] = __ldg(p);
-        v[0][0][1] = __ldg(p + 1);
-        v[0][1][0] = __ldg(p + sy);
-        v[0][1][1] = __ldg(p + sy + 1);
-        v[1][0][0] = __ldg(p + sz);
-        v[1][0][1] = __ldg(p + sz + 1);
-        v[1][1][0] = __ldg(p + sz + sy);
-        v[1][1][1] = __ldg(p + sz + sy + 1);
-    } else {
-        const bool inx[2] = { (unsigned)px < (unsigned)fnx, (unsigned)(px + 1) < (unsigned)fnx };
-        const bool iny[2] = { (unsigned)py < (unsigned)fny, (unsigned)(py + 1) < (unsigned)fny };
-        const bool inz[2] = { (unsigned)pz < (unsigned)fnz, (unsigned)(pz + 1) < (unsigned)fnz };
-        const int cx[2] = { min(max(px, 0), fnx - 1), min(max(px + 1, 0), fnx - 1) };
-        const int cy[2] = { min(max(py, 0), fny - 1), min(max(py + 1, 0), fny - 1) };
-        const int cz[2] = { min(max(pz, 0), fnz - 1), min(max(pz + 1, 0), fnz - 1) };
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const float *row = flo + cz[c] * sz + cy[b] * sy;
-#pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    const float t = __ldg(row + cx[a]);
-                    v[c][b][a] = (inx[a] && iny[b] && inz[c]) ? t : pad;
-                }
-            }
+        const float tx = fminf(fmaxf(flx + V.tex_off, 1.f), V.tex_x);
+        const float ty = fminf(fmaxf(fly + V.tex_off, 1.f), V.tex_y);
+        const int layer = min(max(pz + V.margin, 0), V.tex_layer);
+        gather_footprint(V.tex, layer, tx, ty, S.v[0]);
+        gather_footprint(V.tex, layer + 1, tx, ty, S.v[1]);
+        return;
     }
-    const float yv0 = fmaf(v[0][0][1], rx, v[0][0][0] * bx0);
-    const float yv1 = fmaf(v[0][1][1], rx, v[0][1][0] * bx0);
+    // -margin <= p and p + 1 <= n - 1 + margin on every axis (|p| <= 2^21: no overflow)
+    const bool plain = (unsigned)(px + V.margin) < (unsigned)(V.nx + 2 * V.margin - 1) &&
+                       (unsigned)(py + V.margin) < (unsigned)(V.ny + 2 * V.margin - 1) &&
+                       (unsigned)(pz + V.margin) < (unsigned)(V.nz + 2 * V.margin - 1);
+    if (__all_sync(__activemask(), plain)) {
+        const float *p = flo + (pz * V.sz + py * V.sy + px);
+        S.v[0][0][0] = __ldg(p);
+        S.v[0][0][1] = __ldg(p + 1);
+        S.v[0][1][0] = __ldg(p + V.sy);
+        S.v[0][1][1] = __ldg(p + V.sy + 1);
+        S.v[1][0][0] = __ldg(p + V.sz);
+        S.v[1][0][1] = __ldg(p + V.sz + 1);
+        S.v[1][1][0] = __ldg(p + V.sz + V.sy);
+        S.v[1][1][1] = __ldg(p + V.sz + V.sy + 1);
+        return;
+    }
+    const bool inx[2] = { (unsigned)px < (unsigned)V.nx, (unsigned)(px + 1) < (unsigned)V.nx };
+    const bool iny[2] = { (unsigned)py < (unsigned)V.ny, (unsigned)(py + 1) < (unsigned)V.ny };
+    const bool inz[2] = { (unsigned)pz < (unsigned)V.nz, (unsigned)(pz + 1) < (unsigned)V.nz };
+    const int cx[2] = { min(max(px, 0), V.nx - 1), min(max(px + 1, 0), V.nx - 1) };
+    const int cy[2] = { min(max(py, 0), V.ny - 1), min(max(py + 1, 0), V.ny - 1) };
+    const int cz[2] = { min(max(pz, 0), V.nz - 1), min(max(pz + 1, 0), V.nz - 1) };
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const float *row = flo + cz[c] * V.sz + cy[b] * V.sy;
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                const float t = __ldg(row + cx[a]);
+                S.v[c][b][a] = (inx[a] && iny[b] && inz[c]) ? t : pad;
+            }
+        }
+}
+
+template <bool kGrad>
+__device__ __forceinline__ void footprint_value(const Footprint& S, float& val, float g[3]) {
+    const float rx = S.rx, ry = S.ry, rz = S.rz;
+    const float bx0 = 1.f - rx, by0 = 1.f - ry, bz0 = 1.f - rz;
+    const float yv0 = fmaf(S.v[0][0][1], rx, S.v[0][0][0] * bx0);
+    const float yv1 = fmaf(S.v[0][1][1], rx, S.v[0][1][0] * bx0);
     const float zv0 = fmaf(yv1, ry, yv0 * by0);
-    const float yw0 = fmaf(v[1][0][1], rx, v[1][0][0] * bx0);
-    const float yw1 = fmaf(v[1][1][1], rx, v[1][1][0] * bx0);
+    const float yw0 = fmaf(S.v[1][0][1], rx, S.v[1][0][0] * bx0);
+    const float yw1 = fmaf(S.v[1][1][1], rx, S.v[1][1][0] * bx0);
     const float zv1 = fmaf(yw1, ry, yw0 * by0);
     val = fmaf(zv1, rz, zv0 * bz0);
     if (kGrad) {
-        const float dx00 = v[0][0][1] - v[0][0][0], dx01 = v[0][1][1] - v[0][1][0];
-        const float dx10 = v[1][0][1] - v[1][0][0], dx11 = v[1][1][1] - v[1][1][0];
+        const float dx00 = S.v[0][0][1] - S.v[0][0][0], dx01 = S.v[0][1][1] - S.v[0][1][0];
+        const float dx10 = S.v[1][0][1] - S.v[1][0][0], dx11 = S.v[1][1][1] - S.v[1][1][0];
         const float gx0 = fmaf(dx01, ry, dx00 * by0), gx1 = fmaf(dx11, ry, dx10 * by0);
         g[0] = fmaf(gx1, rz, gx0 * bz0);
         g[1] = fmaf(yw1 - yw0, rz, (yv1 - yv0) * bz0);
@@ -401,8 +417,6 @@ __device__ __forceinline__ void sample_floating(const float *__restrict__ flo, u
             if (g[d] != g[d]) g[d] = 0.f;
     }
 }
-
-constexpr int WALK_GROUP = 1;  // slices per step of the walk (two in flight measured 2% slower)
 
 // shared-memory layout of a walk block: cp block | z basis | z node index | kernel-specific
 struct WalkSmem {
@@ -458,53 +472,53 @@ __device__ __forceinline__ void flush_hist(const uint32_t *h, int nbins, uint32_
 // control points (the trial values best - len * grad when grad is given), walk its columns and
 // count every active voxel's (reference, warped) bin pair into the block's histogram h. Called
 // by every thread of the block.
-template <bool kXs, bool kDiag>
+//
+// The walk is one slice ahead of itself: the position of slice z + 1 is evaluated and its fetches
+// issued before slice z's are consumed, so a warp always has a slice's gathers in flight. Columns
+// outside the volume walk the nearest inside one and count nothing (no divergence).
+template <bool kXs, bool kDiag, bool kTex>
 __device__ __forceinline__ void objective_item(const WalkParams& P, const WalkSmem& S, uint32_t *h, float *X,
                                                int item, const float *__restrict__ ref,
                                                const float *__restrict__ flo, const int32_t *__restrict__ mask,
                                                const float *__restrict__ cpp, const float *__restrict__ grad,
                                                float scale) {
     const int lane = threadIdx.x & 31;
-    const float frb = (float)P.rb, ffb = (float)P.fb;
     Item I;
     stage_item<true>(P, cpp, item, S.cp, S.zb, S.zk, S.zid, I, grad, scale);
     Column C;
     column_init(P, I, S.cp, C);
     if (kXs) build_xrows(P, C, S.cp, X);
     const int nzi = I.z1 - I.z0;
-    int idx = (I.z0 * P.ny + C.y) * P.nx + C.x;
     const int zstride = P.nx * P.ny;
-    for (int zi = 0; zi < nzi; zi += WALK_GROUP) {
-        int bin[WALK_GROUP];
-#pragma unroll
-        for (int u = 0; u < WALK_GROUP; ++u) {
-            const int zu = min(zi + u, nzi - 1);
-            float pos[3];
-            column_position(P, I, C, S.zb, S.zk, S.zid, zu, pos, kXs ? X : nullptr);
-            bin[u] = -1;
-            if (C.inside && zi + u < nzi) {
-                const int vi = idx + u * zstride;
-                if (mask == nullptr || __ldg(&mask[vi]) > -1) {
-                    float w, g[3];
-                    sample_floating<false, kDiag ? 1 : 0>(flo, P.ftex, P.fnx, P.fny, P.fnz, P.fsy, P.fsz, P.fmargin,
-                                                          P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], w, g);
-                    const float rv = __ldg(&ref[vi]);
-                    if (0.f <= rv && rv < frb && 0.f <= w && w < ffb)  // false for NaN
-                        bin[u] = trunc_nonneg(rv) + trunc_nonneg(w) * P.rb;
-                }
-            }
+    int idx = (I.z0 * P.ny + min(C.y, P.ny - 1)) * P.nx + min(C.x, P.nx - 1);
+    const float rlim = C.inside ? P.frb : -1.f;  // no reference value counts in an outside column
+    auto issue = [&](int zi, Footprint& F, float& rv) {
+        float pos[3];
+        column_position<kXs>(P, C, S.zb, S.zk, S.zid, zi, pos, X);
+        fetch_footprint<kDiag ? 1 : 0, kTex>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
+        rv = __ldg(&ref[idx]);
+        if (mask != nullptr && __ldg(&mask[idx]) <= -1) rv = -1.f;
+        idx += zstride;
+    };
+    auto count = [&](const Footprint& F, float rv) {
+        float w, g[3];
+        footprint_value<false>(F, w, g);
+        int bin = -1;
+        if (0.f <= rv && rv < rlim && 0.f <= w && w < P.ffb)  // false for NaN
+            bin = trunc_nonneg(rv) + trunc_nonneg(w) * P.rb;
+        // a warp whose 32 voxels share one bin (background) adds 32 with one atomic
+        const int b0 = __shfl_sync(0xffffffffu, bin, 0);
+        if (__all_sync(0xffffffffu, bin == b0)) {
+            if (lane == 0 && b0 >= 0) atomicAdd(&h[b0], 32u);
+        } else if (bin >= 0) {
+            atomicAdd(&h[bin], 1u);
         }
-        idx += WALK_GROUP * zstride;
-#pragma unroll
-        for (int u = 0; u < WALK_GROUP; ++u) {
-            // a warp whose 32 voxels share one bin (background) adds 32 with one atomic
-            const int b0 = __shfl_sync(0xffffffffu, bin[u], 0);
-            if (__all_sync(0xffffffffu, bin[u] == b0)) {
-                if (lane == 0 && b0 >= 0) atomicAdd(&h[b0], 32u);
-            } else if (bin[u] >= 0) {
-                atomicAdd(&h[bin[u]], 1u);
-            }
-        }
+    };
+    for (int zi = 0; zi < nzi; ++zi) {
+        Footprint F;
+        float rv;
+        issue(zi, F, rv);
+        count(F, rv);
     }
 }
 
@@ -519,9 +533,9 @@ __device__ __forceinline__ void objective_smem(const WalkParams& P, void *base, 
 // fused objective: deformation + warp + joint histogram
 // ---------------------------------------------------------------------------------------------
 // kXs: the item's x-contracted node rows are staged in shared memory; kDiag: the floating
-// image's mm -> voxel matrix has no off-diagonal terms (launch-time choices made template
-// parameters, so the walk carries no test for them)
-template <bool kTrial, bool kXs, bool kDiag>
+// image's mm -> voxel matrix has no off-diagonal terms; kTex: the floating image is held as a
+// texture (launch-time choices made template parameters, so the walk carries no test for them)
+template <bool kTrial, bool kXs, bool kDiag, bool kTex>
 __global__ void __launch_bounds__(32 * TY_OBJECTIVE, 2)
 k_objective(WalkParams P, const float *__restrict__ ref, const float *__restrict__ flo,
             const int32_t *__restrict__ mask, const float *__restrict__ cpp,
@@ -537,7 +551,7 @@ k_objective(WalkParams P, const float *__restrict__ ref, const float *__restrict
     pdl_launch_dependents();  // the finalize may start its preamble (it waits for the counts)
     const float scale = kTrial ? -step->cur_len : 0.f;
     for (int item = blockIdx.x; item < P.nitems; item += gridDim.x)
-        objective_item<kXs, kDiag>(P, S, h, X, item, ref, flo, mask, cpp, kTrial ? grad : nullptr, scale);
+        objective_item<kXs, kDiag, kTex>(P, S, h, X, item, ref, flo, mask, cpp, kTrial ? grad : nullptr, scale);
     flush_hist(h, nbins, ghist);
 }
 
@@ -681,7 +695,7 @@ __device__ __forceinline__ void stage_log_table(const WalkParams& P, const doubl
 
 // One item of the fused gradient: stage the item's control points, walk its columns and write
 // every voxel's NMI gradient (zero where masked or NaN). Called by every thread of the block.
-template <bool kF32, bool kDiag>
+template <bool kF32, bool kDiag, bool kTex>
 __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSmem& S, const float *logf,
                                               const GradientTables& T, int item, const float *__restrict__ ref,
                                               const float *__restrict__ flo, const int32_t *__restrict__ mask,
@@ -696,14 +710,15 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
     int idx = (I.z0 * P.ny + C.y) * P.nx + C.x;
     for (int zi = 0; zi < nzi; ++zi, idx += zstride) {
         float pos[3];
-        column_position(P, I, C, S.zb, S.zk, S.zid, zi, pos);
+        column_position(P, C, S.zb, S.zk, S.zid, zi, pos);
         if (!C.inside) continue;
         float out[3] = { 0.f, 0.f, 0.f };
         if (mask == nullptr || __ldg(&mask[idx]) > -1) {
+            Footprint F;
             float w, g[3];
-            sample_floating<true, kDiag ? 1 : 0>(flo, P.ftex, P.fnx, P.fny, P.fnz, P.fsy, P.fsz, P.fmargin, P.flo_ijk,
-                                                 P.flo_diag, P.pad, pos[0], pos[1], pos[2], w, g);
+            fetch_footprint<kDiag ? 1 : 0, kTex>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
             const float rv = __ldg(&ref[idx]);
+            footprint_value<true>(F, w, g);
             if (rv == rv && w == w) {
                 if (kF32) {
                     const float s = nmi_window_f(rv, w, logf, P.rb, P.fb, T.nmi_f);
@@ -722,7 +737,7 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
     }
 }
 
-template <bool kF32, bool kDiag>
+template <bool kF32, bool kDiag, bool kTex>
 __global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 6 : 4)
 k_gradient(WalkParams P, const float *__restrict__ ref, const float *__restrict__ flo,
            const int32_t *__restrict__ mask, const float *__restrict__ cpp,
@@ -734,7 +749,7 @@ k_gradient(WalkParams P, const float *__restrict__ ref, const float *__restrict_
     float *logf = reinterpret_cast<float *>(S.tail);
     if (kF32) stage_log_table(P, T.logt, logf);
     for (int item = blockIdx.x; item < P.nitems; item += gridDim.x)
-        gradient_item<kF32, kDiag>(P, S, logf, T, item, ref, flo, mask, cpp, vgrad);
+        gradient_item<kF32, kDiag, kTex>(P, S, logf, T, item, ref, flo, mask, cpp, vgrad);
 }
 
 // standalone deformation field (Compute::GetDeformationField) with the same arithmetic
@@ -752,7 +767,7 @@ k_deformation(WalkParams P, const int32_t *__restrict__ mask, const float *__res
         const int nzi = I.z1 - I.z0;
         for (int zi = 0; zi < nzi; ++zi) {
             float pos[3];
-            column_position(P, I, C, S.zb, S.zk, S.zid, zi, pos);
+            column_position(P, C, S.zb, S.zk, S.zid, zi, pos);
             if (!C.inside) continue;
             const int idx = ((I.z0 + zi) * P.ny + C.y) * P.nx + C.x;
             if (mask != nullptr && __ldg(&mask[idx]) <= -1) pos[0] = pos[1] = pos[2] = 0.f;
@@ -1085,7 +1100,7 @@ k_nmi_finalize(FinArgs A, cudaGraphConditionalHandle line) {
 // standalone resampling / histogram / voxel gradient (materialised intermediates)
 // ---------------------------------------------------------------------------------------------
 template <bool kGrad>
-__global__ void k_resample(long long nv, int fnx, int fny, int fnz, Mat34 M, int diag, float pad,
+__global__ void k_resample(long long nv, FloatingView V, Mat34 M, int diag, float pad,
                            const float *__restrict__ flo, const float *__restrict__ def,
                            const int32_t *__restrict__ mask, float *__restrict__ out) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
@@ -1093,9 +1108,11 @@ __global__ void k_resample(long long nv, int fnx, int fny, int fnz, Mat34 M, int
         const bool active = mask == nullptr || mask[i] > -1;
         if (!kGrad && !active) continue;
         float w = 0.f, g[3] = { 0.f, 0.f, 0.f };
-        if (active)
-            sample_floating<kGrad>(flo, 0ull, fnx, fny, fnz, fnx, fnx * fny, 0, M, diag, pad, def[i], def[nv + i],
-                                   def[2 * nv + i], w, g);
+        if (active) {
+            Footprint F;
+            fetch_footprint<-1, false>(flo, V, M, diag, pad, def[i], def[nv + i], def[2 * nv + i], F);
+            footprint_value<kGrad>(F, w, g);
+        }
         if (kGrad) {
             out[i] = g[0];
             out[nv + i] = g[1];
@@ -1229,10 +1246,10 @@ k_warp_order(WalkParams P, const float *__restrict__ cpp, const float *__restric
         const int nzi = I.z1 - I.z0;
         for (int zi = 0; zi < nzi; ++zi) {
             float pos[3];
-            column_position(P, I, C, S.zb, S.zk, S.zid, zi, pos);
+            column_position(P, C, S.zb, S.zk, S.zid, zi, pos);
             if (!C.inside) continue;
             const int idx = ((I.z0 + zi) * P.ny + C.y) * P.nx + C.x;
-            warped[idx] = sample_order<kOrder>(flo, P.fnx, P.fny, P.fnz, P.flo_ijk, P.pad, pos[0], pos[1], pos[2]);
+            warped[idx] = sample_order<kOrder>(flo, P.fv.nx, P.fv.ny, P.fv.nz, P.flo_ijk, P.pad, pos[0], pos[1], pos[2]);
         }
     }
 }
@@ -1303,7 +1320,7 @@ __global__ void k_nmi_voxel_gradient(long long nv, int rb, int fb, const float *
 // The objective of every pair in INIT (at best) or LINE (at best - cur_len * grad): each block
 // walks its share of the pairs' items with the pair's own walk and histogram, exactly the
 // plain k_objective's work per item.
-template <bool kXs, bool kDiag>
+template <bool kXs, bool kDiag, bool kTex>
 __global__ void __launch_bounds__(32 * TY_OBJECTIVE, 2)
 k_b_objective(const __grid_constant__ BatchObjTable T, const OptState *__restrict__ states, int npairs) {
     extern __shared__ float4 sm4[];
@@ -1327,7 +1344,7 @@ k_b_objective(const __grid_constant__ BatchObjTable T, const OptState *__restric
         for (int j = G.j0[sg]; j < G.j1[sg]; ++j) {
             const int q = G.pair[sg];
             const bool line = states[q].phase == PH_LINE;
-            objective_item<kXs, kDiag>(T.e[q].P, S, h, X, j, T.e[q].ref, T.e[q].flo, nullptr, T.e[q].best,
+            objective_item<kXs, kDiag, kTex>(T.e[q].P, S, h, X, j, T.e[q].ref, T.e[q].flo, nullptr, T.e[q].best,
                                        line ? T.e[q].grad : nullptr, line ? -states[q].cur_len : 0.f);
         }
         flush_hist(h, nbins, T.e[G.pair[sg]].hist);
@@ -1336,7 +1353,7 @@ k_b_objective(const __grid_constant__ BatchObjTable T, const OptState *__restric
 
 // The fused voxel gradient of every pair in GRAD, at best, with the NMI tables of its best
 // position (the plain k_gradient's work per item).
-template <bool kF32, bool kDiag>
+template <bool kF32, bool kDiag, bool kTex>
 __global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 6 : 4)
 k_b_gradient(const __grid_constant__ BatchGradTable T, const OptState *__restrict__ states, int npairs) {
     extern __shared__ float4 sm4[];
@@ -1357,7 +1374,7 @@ k_b_gradient(const __grid_constant__ BatchGradTable T, const OptState *__restric
         __syncthreads();  // the previous pair's walk is done with the shared tables
         if (kF32) stage_log_table(E.P, N.logt, logf);  // visible after stage_item's first barrier
         for (int j = G.j0[sg]; j < G.j1[sg]; ++j)
-            gradient_item<kF32, kDiag>(E.P, S, logf, N, j, E.ref, E.flo, nullptr, E.best, E.vgrad);
+            gradient_item<kF32, kDiag, kTex>(E.P, S, logf, N, j, E.ref, E.flo, nullptr, E.best, E.vgrad);
     }
 }
 
@@ -1437,22 +1454,18 @@ static WalkParams make_params(const WalkPlan& W, const nrb_geometry *g, float pa
     P.sa = W.sa;
     P.sb = W.sb;
     P.sc = W.sc;
-    P.fnx = g->flo_dim[0];
-    P.fny = g->flo_dim[1];
-    P.fnz = g->flo_dim[2];
-    P.fsy = P.fnx;
-    P.fsz = P.fnx * P.fny;
-    P.fmargin = 0;
+    P.fv = floating_view(g->flo_dim[0], g->flo_dim[1], g->flo_dim[2], 0, 0ull);
     P.flo_ijk = to_mat34(g->flo_ijk);
     P.pad = pad;
     P.rb = rb;
     P.fb = fb;
+    P.frb = (float)rb;
+    P.ffb = (float)fb;
     P.cnv = P.cx * P.cy * P.cz;
     const float *m = g->flo_ijk;
     P.flo_diag = m[1] == 0.f && m[2] == 0.f && m[4] == 0.f && m[6] == 0.f && m[8] == 0.f && m[9] == 0.f;
     P.log_in_smem = 0;
     P.xs = 0;
-    P.ftex = 0;
     // identity split when the grid's voxel -> mm matrix has no off-diagonal terms
     const float *c = g->cpp_xyz;
     const bool cdiag = c[1] == 0.f && c[2] == 0.f && c[4] == 0.f && c[6] == 0.f && c[8] == 0.f && c[9] == 0.f;
@@ -1465,10 +1478,8 @@ static WalkParams make_params(const WalkPlan& W, const nrb_geometry *g, float pa
 
 // a floating image laid out by pad_volume with `margin` voxels on every side, passed as the
 // pointer to its voxel (0, 0, 0)
-static void set_floating_margin(WalkParams& P, int margin) {
-    P.fmargin = margin;
-    P.fsy = P.fnx + 2 * margin;
-    P.fsz = P.fsy * (P.fny + 2 * margin);
+static void set_floating_margin(WalkParams& P, int margin, unsigned long long tex) {
+    P.fv = floating_view(P.fv.nx, P.fv.ny, P.fv.nz, margin, margin >= 2 ? tex : 0ull);
 }
 
 template <typename K>
@@ -1498,8 +1509,30 @@ static long long blocks_resident(K kernel, int threads, size_t smem) {
     return (long long)per_sm * sm_count();
 }
 
-long long objective_slots(size_t smem) { return blocks_resident(k_objective<true, true, true>, 32 * TY_OBJECTIVE, smem); }
-long long gradient_slots(size_t smem) { return blocks_resident(k_gradient<true, true>, 32 * TY_GRADIENT, smem); }
+// launch-time choices -> the kernel compiled for them
+template <bool... kDone, typename F>
+static auto with_flags(F f) { return f.template operator()<kDone...>(); }
+template <bool... kDone, typename F, typename... Rest>
+static auto with_flags(F f, bool first, Rest... rest) {
+    return first ? with_flags<kDone..., true>(f, rest...) : with_flags<kDone..., false>(f, rest...);
+}
+struct ObjectiveKernel {
+    template <bool kTrial, bool kXs, bool kDiag, bool kTex> auto operator()() const { return k_objective<kTrial, kXs, kDiag, kTex>; }
+};
+struct GradientKernel {
+    template <bool kF32, bool kDiag, bool kTex> auto operator()() const { return k_gradient<kF32, kDiag, kTex>; }
+};
+struct BatchObjectiveKernel {
+    template <bool kXs, bool kDiag, bool kTex> auto operator()() const { return k_b_objective<kXs, kDiag, kTex>; }
+};
+struct BatchGradientKernel {
+    template <bool kF32, bool kDiag, bool kTex> auto operator()() const { return k_b_gradient<kF32, kDiag, kTex>; }
+};
+static auto pick_objective(bool trial, bool xs, bool diag, bool tex) { return with_flags<>(ObjectiveKernel{}, trial, xs, diag, tex); }
+static auto pick_gradient(bool f32, bool diag, bool tex) { return with_flags<>(GradientKernel{}, f32, diag, tex); }
+
+long long objective_slots(size_t smem) { return blocks_resident(k_objective<true, true, true, true>, 32 * TY_OBJECTIVE, smem); }
+long long gradient_slots(size_t smem) { return blocks_resident(k_gradient<true, true, true>, 32 * TY_GRADIENT, smem); }
 long long deformation_slots(size_t smem) { return blocks_resident(k_deformation, 32 * TY_DEFORMATION, smem); }
 
 template <int kOrder>
@@ -1510,8 +1543,7 @@ nrb_status launch_fused_objective(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geo
                                   const float *cpp, float padding, cudaStream_t st,
                                   const float *grad, const OptState *step, int flo_margin) {
     WalkParams P = make_params(ws->walk_obj, g, padding, nmi->rb, nmi->fb);
-    set_floating_margin(P, flo_margin);
-    P.ftex = flo_margin >= 2 ? ws->flo_tex : 0ull;
+    set_floating_margin(P, flo_margin, ws->flo_tex);
     const size_t base_smem = walk_smem_bytes(ws->walk_obj) + (size_t)((nmi->rb * nmi->fb + 3) & ~3) * 4;
     const size_t xs_bytes = (size_t)3 * P.sc * P.sb * 32 * 4;
     // the x-contracted rows when two blocks per SM still fit
@@ -1519,10 +1551,7 @@ nrb_status launch_fused_objective(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geo
     const size_t smem = base_smem + (P.xs ? xs_bytes : 0);
     const int threads = 32 * ws->walk_obj.ty;
     const bool trial = grad != nullptr;
-    auto kernel = P.flo_diag ? (trial ? (P.xs ? k_objective<true, true, true> : k_objective<true, false, true>)
-                                      : (P.xs ? k_objective<false, true, true> : k_objective<false, false, true>))
-                             : (trial ? (P.xs ? k_objective<true, true, false> : k_objective<true, false, false>)
-                                      : (P.xs ? k_objective<false, true, false> : k_objective<false, false, false>));
+    auto kernel = pick_objective(trial, P.xs, P.flo_diag, P.fv.tex != 0);
     int grid = 0;
     NRB_TRY(persistent_grid(kernel, threads, smem, P.nitems, grid, ws->walk_obj.resident));
     // algorithmic bytes: reference + floating (+ mask) per voxel, the grid once
@@ -1544,8 +1573,7 @@ nrb_status launch_fused_gradient(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geom
                                  const float *cpp, float padding, double weight, float *vgrad,
                                  cudaStream_t st, const OptState *sel, int flo_margin) {
     WalkParams P = make_params(ws->walk_grad, g, padding, nmi->rb, nmi->fb);
-    set_floating_margin(P, flo_margin);
-    P.ftex = flo_margin >= 2 ? ws->flo_tex : 0ull;
+    set_floating_margin(P, flo_margin, ws->flo_tex);
     // an FP32 copy of the log table rides in shared memory when it fits (64 bins: 19 KB,
     // 128 bins: 70 KB); larger tables use the FP64 window on the global table
     const size_t log_bytes = (size_t)nmi->total * sizeof(float);
@@ -1553,8 +1581,7 @@ nrb_status launch_fused_gradient(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geom
     const size_t smem = walk_smem_bytes(ws->walk_grad) + (P.log_in_smem ? log_bytes : 0);
     const int threads = 32 * ws->walk_grad.ty;
     int grid = 0;
-    auto kernel = P.flo_diag ? (P.log_in_smem ? k_gradient<true, true> : k_gradient<false, true>)
-                             : (P.log_in_smem ? k_gradient<true, false> : k_gradient<false, false>);
+    auto kernel = pick_gradient(P.log_in_smem, P.flo_diag, P.fv.tex != 0);
     NRB_TRY(persistent_grid(kernel, threads, smem, P.nitems, grid, ws->walk_grad.resident));
     // algorithmic bytes: reference + floating (+ mask) read, voxel gradient written, grid once
     const double nv = (double)P.nx * P.ny * P.nz;
@@ -1783,10 +1810,9 @@ nrb_status launch_nmi_finalize(nrb_nmi *nmi, const double *be_partials, int n_be
 nrb_status batch_walks(nrb_workspace *ws, const nrb_nmi *nmi, const nrb_geometry *g, float padding, int flo_margin,
                        WalkParams& wo, WalkParams& wg) {
     wo = make_params(ws->walk_obj, g, padding, nmi->rb, nmi->fb);
-    set_floating_margin(wo, flo_margin);
+    set_floating_margin(wo, flo_margin, ws->flo_tex);
     wg = make_params(ws->walk_grad, g, padding, nmi->rb, nmi->fb);
-    set_floating_margin(wg, flo_margin);
-    wo.ftex = wg.ftex = flo_margin >= 2 ? ws->flo_tex : 0ull;
+    set_floating_margin(wg, flo_margin, ws->flo_tex);
     wg.log_in_smem = (size_t)nmi->total * sizeof(float) <= 96 * 1024;
     return NRB_OK;
 }
@@ -1797,7 +1823,7 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
     if (L.npairs < 1 || L.npairs > BATCH_MAX_PAIRS)
         return fail(NRB_ERR_INVALID, "batched level: 1 to " + std::to_string(BATCH_MAX_PAIRS) + " pairs");
     size_t base = 0, xs = 0, gsm = 0;
-    bool diag = true, f32 = true;
+    bool diag = true, f32 = true, tex = true;  // tex: textures serve only if every pair has one
     int rb = pairs[0].rb, fb = pairs[0].fb;
     for (const BatchPair& b : pairs) {
         if (b.rb != rb || b.fb != fb) return fail(NRB_ERR_INVALID, "batched level: every pair needs the same bins");
@@ -1809,7 +1835,9 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
         gsm = std::max(gsm, (cp_g + 4 + (size_t)walk_table_floats(b.wg.zchunk)) * 4 + 16);
         diag = diag && b.wo.flo_diag;
         f32 = f32 && b.wg.log_in_smem;
+        tex = tex && b.wo.fv.tex != 0;
     }
+    L.tex = tex;
     L.obj_xs = base + xs <= 100 * 1024;
     L.obj_diag = diag;
     L.obj_smem = base + (L.obj_xs ? xs : 0);
@@ -1840,10 +1868,8 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
         g.last0 = b.last0;
         g.last1 = b.last1;
     }
-    auto ko = L.obj_diag ? (L.obj_xs ? k_b_objective<true, true> : k_b_objective<false, true>)
-                         : (L.obj_xs ? k_b_objective<true, false> : k_b_objective<false, false>);
-    auto kg = L.grad_diag ? (L.grad_f32 ? k_b_gradient<true, true> : k_b_gradient<false, true>)
-                          : (L.grad_f32 ? k_b_gradient<true, false> : k_b_gradient<false, false>);
+    auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.tex);
+    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.tex);
     int per = 0;
     NRB_CUDA(cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ko, 32 * TY_OBJECTIVE, L.obj_smem));
@@ -1858,8 +1884,7 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
 nrb_status launch_batch_objective(const BatchPair *d_pairs, const OptState *states, const BatchLaunch& L,
                                   cudaStream_t st, double bytes) {
     KernelTimer timer(TK_OBJECTIVE, bytes, st);
-    auto ko = L.obj_diag ? (L.obj_xs ? k_b_objective<true, true> : k_b_objective<false, true>)
-                         : (L.obj_xs ? k_b_objective<true, false> : k_b_objective<false, false>);
+    auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.tex);
     ko<<<L.obj_grid, 32 * TY_OBJECTIVE, L.obj_smem, st>>>(L.obj_table, states, L.npairs);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_objective");
@@ -1869,8 +1894,7 @@ nrb_status launch_batch_objective(const BatchPair *d_pairs, const OptState *stat
 nrb_status launch_batch_gradient(const BatchPair *d_pairs, const OptState *states, const BatchLaunch& L,
                                  cudaStream_t st, double bytes) {
     KernelTimer timer(TK_GRADIENT, bytes, st);
-    auto kg = L.grad_diag ? (L.grad_f32 ? k_b_gradient<true, true> : k_b_gradient<false, true>)
-                          : (L.grad_f32 ? k_b_gradient<true, false> : k_b_gradient<false, false>);
+    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.tex);
     kg<<<L.grad_grid, 32 * TY_GRADIENT, L.grad_smem, st>>>(L.grad_table, states, L.npairs);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_gradient");
@@ -2013,14 +2037,15 @@ static nrb_status resample_common(const nrb_geometry *g, const float *flo, const
     if (nv <= 0) return fail(NRB_ERR_INVALID, "resample: empty reference");
     const int threads = 256;
     const int grid = (int)std::min<long long>((nv + threads - 1) / threads, 64LL * sm_count());
+    const FloatingView V = floating_view(g->flo_dim[0], g->flo_dim[1], g->flo_dim[2], 0, 0ull);
     const Mat34 M = to_mat34(g->flo_ijk);
     const float *m = g->flo_ijk;
     const int diag = m[1] == 0.f && m[2] == 0.f && m[4] == 0.f && m[6] == 0.f && m[8] == 0.f && m[9] == 0.f;
     if (grad)
-        k_resample<true><<<grid, threads, 0, as_stream(stream)>>>(nv, g->flo_dim[0], g->flo_dim[1], g->flo_dim[2], M,
+        k_resample<true><<<grid, threads, 0, as_stream(stream)>>>(nv, V, M,
                                                                   diag, pad, flo, def, mask, out);
     else
-        k_resample<false><<<grid, threads, 0, as_stream(stream)>>>(nv, g->flo_dim[0], g->flo_dim[1], g->flo_dim[2], M,
+        k_resample<false><<<grid, threads, 0, as_stream(stream)>>>(nv, V, M,
                                                                    diag, pad, flo, def, mask, out);
     NRB_LAUNCHED("k_resample");
     return NRB_OK;
