@@ -10,6 +10,8 @@
 #include <mutex>
 #include <vector>
 
+#include <cuda_pipeline.h>
+
 #include "nrb_state.cuh"
 
 namespace nrb {
@@ -224,110 +226,236 @@ __device__ __forceinline__ float conv_at(int s, int n, int R, const float *__res
     return num / den;
 }
 
-// pass along x: a block stages CONV_X_ROWS consecutive (y, z) rows of each component in shared
-// memory (for a component those rows are one contiguous run of the volume, so the loads
-// coalesce and many are in flight per thread), then evaluates the sampled outputs of all of them
-constexpr int CONV_X_ROWS = 8, CONV_X_THREADS = 256;
-
-// rows [rb * CONV_X_ROWS, ...) of the x pass; `rows` is the block's shared memory
-// ([3][CONV_X_ROWS][nx] | kernel taps [2R + 1]); ends with every output of those rows written
-__device__ __forceinline__ void conv_x_rows(int nx, int ny, int nz, const float *__restrict__ vg,
-                                            const int *__restrict__ samples, int ns, const float *__restrict__ K,
-                                            int R, float *__restrict__ out, long long rb, float *rows) {
-    float *Ks = rows + 3 * CONV_X_ROWS * nx;
-    const long long nv = (long long)nx * ny * nz;
-    const long long nrow = (long long)ny * nz;
-    const long long r0 = rb * CONV_X_ROWS;
-    const int nr = (int)min((long long)CONV_X_ROWS, nrow - r0);
-    const int run = nr * nx;
-    int nan = 0;
+// Four consecutive sampled outputs of one line (samples ascend), the taps of each in ascending
+// order; where all four windows lie inside the line they share every weight. kPadded: ld reads 0
+// for the R positions beyond either end (a tap there adds weight * 0 and changes no sum), so every
+// window counts as inside. The sum assumes no NaN (its density is then dens[j], the in-line weights
+// summed in the same order); a NaN shows in it, and that output is taken again with conv_at.
+template <bool kPadded, typename Load>
+__device__ __forceinline__ void conv_outputs4(int n, int R, const float *w, const float *dens,
+                                              const int *__restrict__ samples, int ns, int j0, Load ld, float out[4]) {
+    const int last = min(4, ns - j0) - 1;
+    int s[4];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float *src = vg + c * nv + r0 * nx;
-        float *dst = rows + c * CONV_X_ROWS * nx;
-        for (int i = threadIdx.x; i < run; i += CONV_X_THREADS) {
-            const float v = __ldg(src + i);
-            nan |= v != v;
-            dst[i] = v;
+    for (int u = 0; u < 4; ++u) s[u] = __ldg(&samples[j0 + min(u, last)]);
+    float num[4] = { 0.f, 0.f, 0.f, 0.f };
+    if (kPadded || (s[0] >= R && s[3] + R < n)) {
+        const int taps = 2 * R + 1;
+        int t = 0;
+        for (; t + 4 <= taps; t += 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(w + t);
+            const float wt[4] = { q.x, q.y, q.z, q.w };
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) num[u] = fmaf(wt[e], ld(s[u] - R + t + e), num[u]);
         }
-    }
-    for (int i = threadIdx.x; i < 2 * R + 1; i += CONV_X_THREADS) Ks[i] = K[i];
-    // each sample's sum of in-row kernel weights (the same for every row without NaN), summed in
-    // the order of the check-free loop below
-    float *dens = Ks + 2 * R + 1;
-    for (int j = threadIdx.x; j < ns; j += CONV_X_THREADS) {
-        const int sj = samples[j];
-        const int k0 = max(0, sj - R), k1 = min(nx - 1, sj + R);
-        float den = 0.f;
-        for (int k = k0; k <= k1; ++k) den += K[k - sj + R];
-        dens[j] = den;
-    }
-    // rows without NaN (the fused gradient never writes one) take the check-free sum: the
-    // same operations in the same order as conv_at when every tap counts
-    const bool any_nan = __syncthreads_or(nan) != 0;
-    if (ns <= 0) return;  // no sample on this axis: nothing to write
-    // outputs (component c, row r < CONV_X_ROWS, sample j) in the order cr = c * CONV_X_ROWS + r,
-    // then j; a thread steps by CONV_X_THREADS outputs with carried counters (no division per
-    // output); rows beyond the block's last (r >= nr) are skipped
-    int j = threadIdx.x % ns, cr = threadIdx.x / ns;
-    const int dj = CONV_X_THREADS % ns, dcr = CONV_X_THREADS / ns;
-    for (; cr < 3 * CONV_X_ROWS; cr += dcr) {
-        const int c = cr / CONV_X_ROWS, r = cr % CONV_X_ROWS;
-        if (r < nr) {
-            const float *row = rows + cr * nx;
-            const int sj = samples[j];
-            float v;
-            if (any_nan) {
-                v = conv_at(sj, nx, R, Ks, [&](int k) { return row[k]; });
-            } else {
-                float num = 0.f;
-                const int k0 = max(0, sj - R), k1 = min(nx - 1, sj + R);
-                const float *w = Ks - sj + R;
+#pragma unroll 1
+        for (; t < taps; ++t) {
+            const float wt = w[t];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) num[u] = fmaf(wt, ld(s[u] - R + t), num[u]);
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k0 = max(0, s[u] - R), k1 = min(n - 1, s[u] + R);
 #pragma unroll 4
-                for (int k = k0; k <= k1; ++k) num = fmaf(w[k], row[k], num);
-                v = num / dens[j];
-            }
-            out[(c * nrow + r0 + r) * ns + j] = v;
+            for (int k = k0; k <= k1; ++k) num[u] = fmaf(w[k - s[u] + R], ld(k), num[u]);
         }
-        j += dj;
-        if (j >= ns) {
-            j -= ns;
-            ++cr;
-        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) out[u] = num[u] / dens[j0 + min(u, last)];
+#pragma unroll 1
+    for (int u = 0; u <= last; ++u) {
+        const float v = u < 2 ? (u == 0 ? num[0] : num[1]) : (u == 2 ? num[2] : num[3]);
+        if (v == v) continue;
+        const float r = conv_at(__ldg(&samples[j0 + u]), n, R, w, ld);
+        if (u == 0) out[0] = r;
+        else if (u == 1) out[1] = r;
+        else if (u == 2) out[2] = r;
+        else out[3] = r;
     }
 }
 
+// weights (16-byte aligned, padded to fours) and densities of one axis in a block's shared memory;
+// ends with a barrier
+__host__ __device__ inline int conv_weight_floats(int R, int ns) { return ((2 * R + 4) & ~3) + ((ns + 3) & ~3); }
+__device__ __forceinline__ void conv_weights(int n, int R, const float *__restrict__ K, const int *__restrict__ samples,
+                                             int ns, float *w, float *&dens) {
+    dens = w + ((2 * R + 4) & ~3);
+    for (int i = threadIdx.x; i < 2 * R + 1; i += blockDim.x) w[i] = K[i];
+    __syncthreads();
+    for (int j = threadIdx.x; j < ns; j += blockDim.x) {
+        const int sj = samples[j];
+        const int k0 = max(0, sj - R), k1 = min(n - 1, sj + R);
+        float den = 0.f;
+        for (int k = k0; k <= k1; ++k) den += w[k - sj + R];
+        dens[j] = den;
+    }
+    __syncthreads();
+}
+
+// Pass along x. A block takes kRows consecutive rows of one component, transposes them into shared
+// memory (column stride kRows + 1: no bank conflict either way; R columns of zeros on either side),
+// and each lane convolves one row; its warps share the outputs, four at a time. The outputs go out
+// through shared memory as one contiguous run. 32 rows while the tile stays small enough for
+// several blocks per SM; long rows take 16 or 8, the warp's other lanes then working on other
+// outputs of the same rows.
+//
+// One load and a quarter of a weight load per multiply-add, rows copied asynchronously: 182x218x182
+// with a 5-voxel grid (37 samples, 21 taps) takes 55 us (37.7 M warp instructions, issue-bound); it
+// took 64 us (47.6 M) when a thread stepped through the outputs of several rows with a weight, a
+// value and a bounds check per tap. The y pass went from 22 to 18 us.
+constexpr int CONV_X_THREADS = 128;
+__host__ __device__ inline size_t conv_x_bytes(int rows, int nx, int R, int ns) {
+    return 4 * ((size_t)conv_weight_floats(R, ns) + (size_t)(nx + 2 * R) * (rows + 1) + (size_t)rows * (ns | 1));
+}
+inline int conv_x_rows(int nx, int R, int ns) {
+    for (int rows : { 32, 16 })
+        if (conv_x_bytes(rows, nx, R, ns) <= 48 * 1024) return rows;
+    return 8;
+}
+__host__ __device__ inline long long conv_x_units(int rows, int ny, int nz) {
+    return 3 * (((long long)ny * nz + rows - 1) / rows);
+}
+
+// unit = (component, group of rows); conv_weights has filled w and dens
+template <int kRows>
+__device__ __forceinline__ void conv_x_unit(int nx, int ny, int nz, const float *__restrict__ vg,
+                                            const int *__restrict__ samples, int ns, int R, float *__restrict__ out,
+                                            long long unit, const float *w, const float *dens, float *tile) {
+    constexpr int kStride = kRows + 1, kSub = 32 / kRows, kWarps = CONV_X_THREADS / 32;
+    float *res = tile + (size_t)(nx + 2 * R) * kStride;
+    const int rstride = ns | 1;
+    const long long nrow = (long long)ny * nz, groups = (nrow + kRows - 1) / kRows;
+    const int c = (int)(unit / groups);
+    const long long r0 = (unit - c * groups) * kRows;
+    const int nr = (int)min((long long)kRows, nrow - r0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *body = tile + R * kStride;
+    for (int r = warp; r < nr; r += kWarps) {
+        const float *src = vg + (c * nrow + r0 + r) * nx;
+#pragma unroll 4
+        for (int x = lane; x < nx; x += 32) __pipeline_memcpy_async(body + x * kStride + r, src + x, 4);
+    }
+    __pipeline_commit();
+    for (int i = threadIdx.x; i < R * kStride; i += CONV_X_THREADS) tile[i] = body[nx * kStride + i] = 0.f;
+    __pipeline_wait_prior(0);
+    __syncthreads();
+    const int lrow = lane % kRows;
+    const float *col = body + lrow;
+    for (int q = warp * kSub + lane / kRows; 4 * q < ns; q += kWarps * kSub) {
+        if (lrow >= nr) continue;
+        float v[4];
+        conv_outputs4<true>(nx, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * kStride]; }, v);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (4 * q + u < ns) res[lrow * rstride + 4 * q + u] = v[u];
+    }
+    __syncthreads();
+    float *dst = out + (c * nrow + r0) * ns;
+    for (int r = warp; r < nr; r += kWarps)
+#pragma unroll 2
+        for (int j = lane; j < ns; j += 32) dst[r * ns + j] = res[r * rstride + j];
+}
+
+template <int kRows>
 __global__ void __launch_bounds__(CONV_X_THREADS)
 k_conv_x(int nx, int ny, int nz, const float *__restrict__ vg, const int *__restrict__ samples, int ns,
          const float *__restrict__ K, int R, float *__restrict__ out) {
-    extern __shared__ float rows[];
-    conv_x_rows(nx, ny, nz, vg, samples, ns, K, R, out, blockIdx.x, rows);
+    extern __shared__ __align__(16) float conv_sm[];
+    float *dens;
+    conv_weights(nx, R, K, samples, ns, conv_sm, dens);
+    conv_x_unit<kRows>(nx, ny, nz, vg, samples, ns, R, out, blockIdx.x, conv_sm, dens, conv_sm + conv_weight_floats(R, ns));
 }
 
-// pass along an outer axis of a [3][outer][len][inner] array at sampled positions of `len`:
-// out[3][outer][ns][inner]
-__device__ __forceinline__ void conv_strided_at(int outer, int len, int inner, const float *__restrict__ in,
-                                                const int *__restrict__ samples, int ns, const float *__restrict__ K,
-                                                int R, float *__restrict__ out, long long i) {
-    {
-        const int ii = (int)(i % inner);
-        long long rest = i / inner;
-        const int j = (int)(rest % ns);
-        rest /= ns;
-        const int o = (int)(rest % outer);
-        const int c = (int)(rest / outer);
-        const float *base = in + (((long long)c * outer + o) * len) * inner + ii;
-        out[i] = conv_at(samples[j], len, R, K, [&](int k) { return __ldg(&base[(long long)k * inner]); });
+// Pass along y of a [3][nz][ny][inner] array: a block takes `width` columns of one (component, z)
+// slice in shared memory (R rows of zeros above and below), a thread four outputs of a column.
+constexpr int CONV_Y_THREADS = 256;
+__host__ __device__ inline int conv_y_width(int ny, int inner, int R) {
+    const int most = 48 * 1024 / (4 * (ny + 2 * R));
+    return inner <= most ? inner : (most < 1 ? 1 : most);
+}
+__host__ __device__ inline long long conv_y_units(int ny, int nz, int inner, int R) {
+    const int width = conv_y_width(ny, inner, R);
+    return 3LL * nz * ((inner + width - 1) / width);
+}
+__host__ __device__ inline size_t conv_y_bytes(int ny, int inner, int R, int ns) {
+    return 4 * ((size_t)conv_weight_floats(R, ns) + (size_t)(ny + 2 * R) * conv_y_width(ny, inner, R));
+}
+
+__device__ __forceinline__ void conv_y_unit(int ny, int inner, const float *__restrict__ in,
+                                            const int *__restrict__ samples, int ns, int R, float *__restrict__ out,
+                                            long long unit, const float *w, const float *dens, float *tile) {
+    const int width = conv_y_width(ny, inner, R), chunks = (inner + width - 1) / width;
+    const long long slice = unit / chunks;  // component * nz + z
+    const int i0 = (int)(unit - slice * chunks) * width, wd = min(width, inner - i0);
+    const float *src = in + slice * ny * inner + i0;
+    float *body = tile + R * wd;
+    if (wd == inner) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < ny * inner; i += CONV_Y_THREADS) __pipeline_memcpy_async(body + i, src + i, 4);
+    } else {
+        for (int i = threadIdx.x; i < ny * wd; i += CONV_Y_THREADS) {
+            const int y = i / wd;
+            __pipeline_memcpy_async(body + i, src + (long long)y * inner + (i - y * wd), 4);
+        }
+    }
+    __pipeline_commit();
+    for (int i = threadIdx.x; i < R * wd; i += CONV_Y_THREADS) tile[i] = body[ny * wd + i] = 0.f;
+    __pipeline_wait_prior(0);
+    __syncthreads();
+    float *dst = out + slice * ns * inner + i0;
+    for (int e = threadIdx.x; e < (ns + 3) / 4 * wd; e += CONV_Y_THREADS) {
+        const int q = e / wd, ii = e - q * wd;
+        const float *col = body + ii;
+        float v[4];
+        conv_outputs4<true>(ny, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * wd]; }, v);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (4 * q + u < ns) dst[(long long)(4 * q + u) * inner + ii] = v[u];
     }
 }
 
-__global__ void k_conv_strided(int outer, int len, int inner, const float *__restrict__ in,
-                               const int *__restrict__ samples, int ns, const float *__restrict__ K,
-                               int R, float *__restrict__ out) {
-    const long long total = 3LL * outer * ns * inner;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x)
-        conv_strided_at(outer, len, inner, in, samples, ns, K, R, out, i);
+__global__ void __launch_bounds__(CONV_Y_THREADS)
+k_conv_y(int ny, int inner, const float *__restrict__ in, const int *__restrict__ samples, int ns,
+         const float *__restrict__ K, int R, float *__restrict__ out) {
+    extern __shared__ __align__(16) float conv_sm[];
+    float *dens;
+    conv_weights(ny, R, K, samples, ns, conv_sm, dens);
+    conv_y_unit(ny, inner, in, samples, ns, R, out, blockIdx.x, conv_sm, dens, conv_sm + conv_weight_floats(R, ns));
+}
+
+// Pass along z of a [3][nz][inner] array, four outputs of a column per thread, element = (component,
+// group of four, column): a column's reads are coalesced over the columns and shared by its groups
+// in L1. The array is small by now (y and x are sampled).
+__host__ __device__ inline long long conv_z_elements(int ns, int inner) { return 3LL * ((ns + 3) / 4) * inner; }
+
+__device__ __forceinline__ void conv_z_element(int nz, int inner, const float *__restrict__ in,
+                                               const int *__restrict__ samples, int ns, int R, float *__restrict__ out,
+                                               long long e, const float *w, const float *dens) {
+    const int groups = (ns + 3) / 4;
+    const int ii = (int)(e % inner);
+    const long long rest = e / inner;
+    const int q = (int)(rest % groups), c = (int)(rest / groups);
+    const float *col = in + (long long)c * nz * inner + ii;
+    float v[4];
+    conv_outputs4<false>(nz, R, w, dens, samples, ns, 4 * q, [&](int k) { return __ldg(col + (long long)k * inner); }, v);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (4 * q + u < ns) out[((long long)c * ns + 4 * q + u) * inner + ii] = v[u];
+}
+
+__global__ void __launch_bounds__(128)
+k_conv_z(int nz, int inner, const float *__restrict__ in, const int *__restrict__ samples, int ns,
+         const float *__restrict__ K, int R, float *__restrict__ out) {
+    extern __shared__ __align__(16) float conv_sm[];
+    float *dens;
+    conv_weights(nz, R, K, samples, ns, conv_sm, dens);
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < conv_z_elements(ns, inner);
+         e += (long long)gridDim.x * blockDim.x)
+        conv_z_element(nz, inner, in, samples, ns, R, out, e, conv_sm, dens);
 }
 
 // reg_voxelCentricToNodeCentric (reg-lib/cpu/_reg_localTrans.cpp:1616-1683): trilinear sample
@@ -475,57 +603,84 @@ __global__ void k_b_be_accumulate(const BatchPair *__restrict__ pairs, const Opt
     });
 }
 
-// x pass of the node convolution: work unit = one block of the plain k_conv_x
+// x, y and z passes of the node convolution: work unit = one block of the plain k_conv_x and
+// k_conv_y, one element of k_conv_z. A block fills its weights when it comes to a pair's first unit.
+template <int kRows>
 __global__ void __launch_bounds__(CONV_X_THREADS)
 k_b_conv_x(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
-    extern __shared__ float rows[];
+    extern __shared__ __align__(16) float conv_sm[];
     __shared__ BatchList L;
     batch_list_build(states, npairs, 1u << PH_GRAD,
                      [&](int q, int& u, int& w) {
                          const BatchPair& b = pairs[q];
-                         u = b.xblocks;
+                         u = (int)conv_x_units(kRows, b.rdim[1], b.rdim[2]);
                          w = 1;
                      }, L);
-    int k = 0;
+    int k = 0, have = -1;
+    float *dens = nullptr;
     for (long long u = blockIdx.x; u < L.total; u += gridDim.x) {
         while (L.pref[k + 1] <= u) ++k;
         const BatchPair& P = pairs[L.pair[k]];
-        conv_x_rows(P.rdim[0], P.rdim[1], P.rdim[2], P.vgrad, P.samples[0], P.ns[0], P.kernel[0], P.radius[0], P.conv1,
-                    u - L.pref[k], rows);
-        __syncthreads();  // rows are reused by the next unit
+        if (have != k) {
+            conv_weights(P.rdim[0], P.radius[0], P.kernel[0], P.samples[0], P.ns[0], conv_sm, dens);
+            have = k;
+        }
+        conv_x_unit<kRows>(P.rdim[0], P.rdim[1], P.rdim[2], P.vgrad, P.samples[0], P.ns[0], P.radius[0], P.conv1,
+                           u - L.pref[k], conv_sm, dens, conv_sm + conv_weight_floats(P.radius[0], P.ns[0]));
+        __syncthreads();  // the tile is reused by the next unit
     }
 }
 
-// y pass ([3][nz][ny][nsx] -> [3][nz][nsy][nsx]) and z pass ([3][nz][nsy * nsx] ->
-// [3][nsz][nsy * nsx]) of the node convolution, element-wise
-__global__ void k_b_conv_y(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
+__global__ void __launch_bounds__(CONV_Y_THREADS)
+k_b_conv_y(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
+    extern __shared__ __align__(16) float conv_sm[];
     __shared__ BatchList L;
     batch_list_build(states, npairs, 1u << PH_GRAD,
                      [&](int q, int& u, int& w) {
                          const BatchPair& b = pairs[q];
-                         u = 3 * b.rdim[2] * b.ns[1] * b.ns[0];
+                         u = (int)conv_y_units(b.rdim[1], b.rdim[2], b.ns[0], b.radius[1]);
                          w = 1;
                      }, L);
-    batch_elements(L, [&](int p, long long i) {
-        const BatchPair& P = pairs[p];
-        conv_strided_at(P.rdim[2], P.rdim[1], P.ns[0], P.conv1, P.samples[1], P.ns[1], P.kernel[1], P.radius[1],
-                        P.conv2, i);
-    });
+    int k = 0, have = -1;
+    float *dens = nullptr;
+    for (long long u = blockIdx.x; u < L.total; u += gridDim.x) {
+        while (L.pref[k + 1] <= u) ++k;
+        const BatchPair& P = pairs[L.pair[k]];
+        if (have != k) {
+            conv_weights(P.rdim[1], P.radius[1], P.kernel[1], P.samples[1], P.ns[1], conv_sm, dens);
+            have = k;
+        }
+        conv_y_unit(P.rdim[1], P.ns[0], P.conv1, P.samples[1], P.ns[1], P.radius[1], P.conv2, u - L.pref[k], conv_sm, dens,
+                    conv_sm + conv_weight_floats(P.radius[1], P.ns[1]));
+        __syncthreads();
+    }
 }
 
-__global__ void k_b_conv_z(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
+__global__ void __launch_bounds__(128)
+k_b_conv_z(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
+    extern __shared__ __align__(16) float conv_sm[];
     __shared__ BatchList L;
     batch_list_build(states, npairs, 1u << PH_GRAD,
                      [&](int q, int& u, int& w) {
                          const BatchPair& b = pairs[q];
-                         u = 3 * b.ns[2] * b.ns[1] * b.ns[0];
+                         u = (int)((conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]) + 127) / 128);
                          w = 1;
                      }, L);
-    batch_elements(L, [&](int p, long long i) {
-        const BatchPair& P = pairs[p];
-        conv_strided_at(1, P.rdim[2], P.ns[1] * P.ns[0], P.conv2, P.samples[2], P.ns[2], P.kernel[2], P.radius[2],
-                        P.conv1, i);
-    });
+    int k = 0, have = -1;
+    float *dens = nullptr;
+    for (long long u = blockIdx.x; u < L.total; u += gridDim.x) {
+        while (L.pref[k + 1] <= u) ++k;
+        const BatchPair& P = pairs[L.pair[k]];
+        const int inner = P.ns[1] * P.ns[0];
+        if (have != k) {
+            __syncthreads();  // the previous pair's weights are done with
+            conv_weights(P.rdim[2], P.radius[2], P.kernel[2], P.samples[2], P.ns[2], conv_sm, dens);
+            have = k;
+        }
+        const long long e = (u - L.pref[k]) * 128 + threadIdx.x;
+        if (e < conv_z_elements(P.ns[2], inner))
+            conv_z_element(P.rdim[2], inner, P.conv2, P.samples[2], P.ns[2], P.radius[2], P.conv1, e, conv_sm, dens);
+    }
 }
 
 // node sampling, reorientation and weighting (overwrites the node gradient)
@@ -1445,6 +1600,27 @@ int be_partial_count(const nrb_geometry *g) { return be_grid(g); }
 nrb_status voxel_to_node_general(const float *vox, const nrb_geometry *g, float weight, float *node,
                                  cudaStream_t st);
 
+// The node convolution serves rows and kernels up to the extent it has always served (24 rows of
+// the volume, the taps and one float per sample in 227 KB)
+static nrb_status conv_supported(int nx, int R, int ns) {
+    if (((size_t)24 * nx + 2 * R + 1 + ns) * 4 > 227 * 1024)
+        return fail(NRB_ERR_UNSUPPORTED, "convolution: rows and kernel exceed shared memory");
+    return NRB_OK;
+}
+// radii and taps of the axes: taps further out than a line is long meet no voxel and are left out,
+// which bounds what a block stages
+static void conv_kernels(const nrb_workspace *ws, const nrb_geometry *g, int R[3], const float *K[3]) {
+    for (int i = 0; i < 3; ++i) {
+        R[i] = std::min(ws->ax[i].radius, g->ref_dim[i] - 1);
+        K[i] = ws->d_kernel[i] + (ws->ax[i].radius - R[i]);
+    }
+}
+template <typename K>
+static nrb_status conv_smem(K kernel, size_t bytes) {
+    if (bytes > 48 * 1024) NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return NRB_OK;
+}
+
 nrb_status launch_convolve_to_nodes(nrb_workspace *ws, const nrb_geometry *g, const float *vgrad,
                                     float weight, float *node, cudaStream_t st) {
     if (ws->general) {
@@ -1463,25 +1639,29 @@ nrb_status launch_convolve_to_nodes(nrb_workspace *ws, const nrb_geometry *g, co
     const int nsx = ws->ax[0].nsamples, nsy = ws->ax[1].nsamples, nsz = ws->ax[2].nsamples;
     // compulsory traffic of the whole voxel->node step: the voxel gradient once, the nodes once
     KernelTimer timer(TK_CONV, 12.0 * (double)nx * ny * nz + 12.0 * (double)nvox(g->cpp_dim), st);
-    // x pass: one block per row
-    // rows | kernel taps | per-sample weight sums (nx <= 2048: <= 205 KB)
-    const size_t smem = ((size_t)3 * CONV_X_ROWS * nx + 2 * ws->ax[0].radius + 1 + nsx) * 4;
-    if (smem > 227 * 1024) return fail(NRB_ERR_UNSUPPORTED, "convolution: rows and kernel exceed shared memory");
-    if (smem > 48 * 1024) NRB_CUDA(cudaFuncSetAttribute(k_conv_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int xblocks = (int)(((long long)ny * nz + CONV_X_ROWS - 1) / CONV_X_ROWS);
-    k_conv_x<<<xblocks, CONV_X_THREADS, smem, st>>>(nx, ny, nz, vgrad, ws->d_samples[0], nsx, ws->d_kernel[0],
-                                         ws->ax[0].radius, ws->conv1);
+    NRB_TRY(conv_supported(nx, ws->ax[0].radius, nsx));
+    int R[3];
+    const float *K[3];
+    conv_kernels(ws, g, R, K);
+    // x pass: [3][nz][ny][nx] -> [3][nz][ny][nsx]
+    const int rows = conv_x_rows(nx, R[0], nsx);
+    const size_t xsm = conv_x_bytes(rows, nx, R[0], nsx), ysm = conv_y_bytes(ny, nsx, R[1], nsy);
+    auto kx = rows == 32 ? k_conv_x<32> : rows == 16 ? k_conv_x<16> : k_conv_x<8>;
+    NRB_TRY(conv_smem(kx, xsm));
+    kx<<<(unsigned)conv_x_units(rows, ny, nz), CONV_X_THREADS, xsm, st>>>(nx, ny, nz, vgrad, ws->d_samples[0], nsx,
+                                                                         K[0], R[0], ws->conv1);
     NRB_LAUNCHED("k_conv_x");
     // y pass: [3][nz][ny][nsx] -> [3][nz][nsy][nsx]
-    long long t2 = 3LL * nz * nsy * nsx;
-    k_conv_strided<<<grid_for(t2, 256), 256, 0, st>>>(nz, ny, nsx, ws->conv1, ws->d_samples[1], nsy,
-                                                      ws->d_kernel[1], ws->ax[1].radius, ws->conv2);
-    NRB_LAUNCHED("k_conv_strided(y)");
-    // z pass: [3][1][nz][nsy*nsx] -> [3][nsz][nsy*nsx] (reuses conv1)
-    long long t3 = 3LL * nsz * nsy * nsx;
-    k_conv_strided<<<grid_for(t3, 256), 256, 0, st>>>(1, nz, nsy * nsx, ws->conv2, ws->d_samples[2], nsz,
-                                                      ws->d_kernel[2], ws->ax[2].radius, ws->conv1);
-    NRB_LAUNCHED("k_conv_strided(z)");
+    NRB_TRY(conv_smem(k_conv_y, ysm));
+    k_conv_y<<<(unsigned)conv_y_units(ny, nz, nsx, R[1]), CONV_Y_THREADS, ysm, st>>>(ny, nsx, ws->conv1, ws->d_samples[1], nsy,
+                                                                              K[1], R[1], ws->conv2);
+    NRB_LAUNCHED("k_conv_y");
+    // z pass: [3][nz][nsy * nsx] -> [3][nsz][nsy * nsx] (reuses conv1)
+    const size_t zsm = 4 * (size_t)conv_weight_floats(R[2], nsz);
+    NRB_TRY(conv_smem(k_conv_z, zsm));
+    k_conv_z<<<grid_for(conv_z_elements(nsz, nsy * nsx), 128), 128, zsm, st>>>(nz, nsy * nsx, ws->conv2, ws->d_samples[2],
+                                                                              nsz, K[2], R[2], ws->conv1);
+    NRB_LAUNCHED("k_conv_z");
     // node sampling, reorientation (floating ijk) and weighting
     float w = weight;
     for (int i = 0; i < 3; ++i) w *= g->cpp_pixdim[i] / g->ref_pixdim[i];
@@ -1724,12 +1904,12 @@ nrb_status batch_node_stage(const nrb_workspace *ws, const nrb_geometry *g, floa
         b.rdim[i] = g->ref_dim[i];
         b.cdim[i] = g->cpp_dim[i];
         b.ns[i] = ws->ax[i].nsamples;
-        b.radius[i] = ws->ax[i].radius;
         b.samples[i] = ws->d_samples[i];
         b.tap_slot[i] = ws->d_tap_slot[i];
         b.tap_weight[i] = ws->d_tap_weight[i];
-        b.kernel[i] = ws->d_kernel[i];
     }
+    NRB_TRY(conv_supported(b.rdim[0], ws->ax[0].radius, b.ns[0]));
+    conv_kernels(ws, g, b.radius, b.kernel);
     b.nnode = nvox(g->cpp_dim);
     b.conv1 = ws->conv1;
     b.conv2 = ws->conv2;
@@ -1744,7 +1924,6 @@ nrb_status batch_node_stage(const nrb_workspace *ws, const nrb_geometry *g, floa
     b.be_der = ws->be_deriv;
     b.be_ratio = be_weight / (float)b.nnode;
     b.red = ws->red;
-    b.xblocks = (int)(((long long)g->ref_dim[1] * g->ref_dim[2] + CONV_X_ROWS - 1) / CONV_X_ROWS);
     return NRB_OK;
 }
 
@@ -1784,33 +1963,35 @@ nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const Batch
         NRB_LAUNCHED("k_b_be_derivatives");
     }
     NRB_TRY(gradient(d, states, st, gradient_arg));
-    // x pass: shared rows for the widest reference
-    int nx = 0, R = 0, nsx = 0;
-    long long xb = 0;
+    // shared memory and rows per block for the largest pair
+    size_t xsm = 0, ysm = 0, zsm = 0;
+    long long xb = 0, yb = 0, zb = 0;
+    int rows = 32;
+    for (const BatchPair& b : hp) rows = std::min(rows, conv_x_rows(b.rdim[0], b.radius[0], b.ns[0]));
     for (const BatchPair& b : hp) {
-        nx = std::max(nx, b.rdim[0]);
-        R = std::max(R, b.radius[0]);
-        nsx = std::max(nsx, b.ns[0]);
-        xb += b.xblocks;
+        xsm = std::max(xsm, conv_x_bytes(rows, b.rdim[0], b.radius[0], b.ns[0]));
+        ysm = std::max(ysm, conv_y_bytes(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]));
+        zsm = std::max(zsm, 4 * (size_t)conv_weight_floats(b.radius[2], b.ns[2]));
+        xb += conv_x_units(rows, b.rdim[1], b.rdim[2]);
+        yb += conv_y_units(b.rdim[1], b.rdim[2], b.ns[0], b.radius[1]);
+        zb += (conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]) + 127) / 128;
     }
-    const size_t smem = ((size_t)3 * CONV_X_ROWS * nx + 2 * R + 1 + nsx) * 4;
-    if (smem > 227 * 1024) return fail(NRB_ERR_UNSUPPORTED, "convolution: rows and kernel exceed shared memory");
-    NRB_CUDA(cudaFuncSetAttribute(k_b_conv_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per = 0;
-    NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_b_conv_x, CONV_X_THREADS, smem));
-    const int xg = (int)std::max(1LL, std::min(xb, (long long)std::max(1, per) * sm_count()));
+    auto launch = [&](auto kernel, long long units, int threads, size_t smem) -> nrb_status {
+        int per = 0;
+        NRB_TRY(conv_smem(kernel, smem));
+        NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
+        const int grid = (int)std::max(1LL, std::min(units, (long long)std::max(1, per) * sm_count()));
+        kernel<<<grid, threads, smem, st>>>(d, states, np);
+        NRB_CUDA(cudaGetLastError());
+        return NRB_OK;
+    };
     {
     KernelTimer timer(TK_CONV, 0.0, st);
-    k_b_conv_x<<<xg, CONV_X_THREADS, smem, st>>>(d, states, np);
-    NRB_CUDA(cudaGetLastError());
+    NRB_TRY(launch(rows == 32 ? k_b_conv_x<32> : rows == 16 ? k_b_conv_x<16> : k_b_conv_x<8>, xb, CONV_X_THREADS, xsm));
     NRB_LAUNCHED("k_b_conv_x");
-    const int gy = batch_grid(hp, [](const BatchPair& b) { return 3LL * b.rdim[2] * b.ns[1] * b.ns[0]; }, 256, 16);
-    k_b_conv_y<<<gy, 256, 0, st>>>(d, states, np);
-    NRB_CUDA(cudaGetLastError());
+    NRB_TRY(launch(k_b_conv_y, yb, CONV_Y_THREADS, ysm));
     NRB_LAUNCHED("k_b_conv_y");
-    const int gz = batch_grid(hp, [](const BatchPair& b) { return 3LL * b.ns[2] * b.ns[1] * b.ns[0]; }, 256, 16);
-    k_b_conv_z<<<gz, 256, 0, st>>>(d, states, np);
-    NRB_CUDA(cudaGetLastError());
+    NRB_TRY(launch(k_b_conv_z, zb, 128, zsm));
     NRB_LAUNCHED("k_b_conv_z");
     const int gn = batch_grid(hp, [](const BatchPair& b) { return b.nnode; }, 256, 16);
     k_b_nodes<<<gn, 256, 0, st>>>(d, states, np);

@@ -174,7 +174,7 @@ struct BatchPair {
     Mat34 flo_ijk;                   // reorientation of the node gradient
     double sim_w, be_w;
     OptState *st;
-    int obj_items, grad_items, xblocks;
+    int obj_items, grad_items;
 };
 
 constexpr int BATCH_MAX_PAIRS = 64;

@@ -192,6 +192,64 @@ def test_convolve_to_nodes(O, case):
     assert np.abs(host(node) - ref).max() <= 1e-5 * scale
 
 
+def convolve_then_sample(O, v, dim, pix, cdim, cpix, weight):
+    """The node gradient of an identity-oriented image whose grid starts one spacing before it: the
+    oracle's convolution along each axis, then the trilinear sample at every node over the taps of
+    non-zero weight inside the volume (a tap of zero weight is not read, so a NaN there does not
+    count; the oracle's own node sampling multiplies it)."""
+    nx, ny, nz = dim
+    for axis in range(3):
+        v = O.kernel_convolution_cubic(v, 3, dim, pix, cpix[axis], axis)
+    vol = np.asarray(v, np.float64).reshape(3, nz, ny, nx)
+    out = vol
+    with np.errstate(invalid="ignore"):
+        for axis, (n, nodes, step, d) in enumerate(zip(dim, cdim, cpix, pix)):
+            step = float(np.float32(step))  # as the geometry holds it
+            at = (np.arange(nodes) * (step / d) - step / d).astype(np.float32).astype(np.float64)
+            pre = np.floor(at).astype(int)
+            parts = []
+            for p, w1 in zip(pre, at - pre):
+                acc = np.zeros(np.delete(out.shape, 3 - axis))
+                for q, w in ((p, 1.0 - w1), (p + 1, w1)):
+                    if 0 <= q < n and w != 0.0:
+                        acc = acc + w * np.take(out, q, axis=3 - axis)
+                parts.append(acc)
+            out = np.stack(parts, axis=3 - axis)
+        # reorientation by the identity: an infinite component meets the other rows' zeros
+        out = np.stack([sum(np.eye(3)[c, d] * out[c] for c in range(3)) for d in range(3)])
+        return (out * weight * np.prod([c / p for c, p in zip(cpix, pix)])).ravel()
+
+
+@pytest.mark.parametrize("shape,spacing", [((3, 11, 200), 5.0), ((2, 5, 401), 5.0), ((2, 3, 900), 7.3), ((3, 301, 222), 3.0),
+                                           ((33, 6, 7), 2.5), ((9, 10, 12), 30.0)])
+def test_convolve_to_nodes_at_tile_edges(O, shape, spacing):
+    """Rows staged 32, 16 and 8 at a time with a remainder, a y pass in column chunks, outputs not a
+    multiple of four, two samples per node (a spacing that is no whole number of voxels), windows
+    longer than the lines; finite gradients, then NaN and infinite ones. The bar of the op above."""
+    rng = np.random.default_rng(shape[2])
+    nz, ny, nx = shape
+    dim, pix = (nx, ny, nz), (1.0, 1.0, 1.0)
+    xyz = nrb.identity_header(pix)
+    cdim, cpix, cxyz = nrb.control_grid_header(dim, pix, (spacing,) * 3)
+    g = nrb.make_geometry(dim, pix, xyz, dim, pix, xyz, cdim, cpix, cxyz)
+    ws = nrb.Workspace(g)
+    n, nc = nx * ny * nz, int(np.prod(cdim))
+    vgrad = rng.normal(0, 1e-3, 3 * n).astype(np.float32)
+    spoiled = vgrad.copy()
+    spoiled[rng.integers(0, 3 * n, 5)] = np.nan
+    spoiled[rng.integers(0, 3 * n, 2)] = np.inf
+    for v in (vgrad, spoiled):
+        node = torch.full((3 * nc,), 123.0, dtype=torch.float32, device="cuda")
+        nrb.convolve_voxel_based_gradient(ws, dev(v), node, 0.995)
+        ref = convolve_then_sample(O, v, dim, pix, cdim, cpix, 0.995)
+        out = host(node)
+        ok = np.isfinite(ref)
+        assert np.array_equal(np.isfinite(out), ok)
+        assert np.array_equal(np.isnan(out), np.isnan(ref))
+        if ok.any():
+            assert np.abs(out[ok] - ref[ok]).max() <= 1e-5 * np.abs(ref[ok]).max()
+
+
 def test_convolve_to_nodes_nan_free_path_is_exact():
     """The x pass sums NaN-free rows with a check-free loop and takes the per-tap path (conv_at)
     for rows holding a NaN; both must give the same bits. A NaN at voxel (0, 3, 0) sends the
