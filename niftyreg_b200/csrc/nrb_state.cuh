@@ -19,7 +19,7 @@ namespace nrb {
 // 16 warps leaves most of the SM's L1 to the floating-image gathers); the gradient pass, whose
 // threads carry more registers, uses 4 warps.
 constexpr int COL_X = 32;
-constexpr int TY_OBJECTIVE = 16, TY_GRADIENT = 4, TY_DEFORMATION = 4;
+constexpr int TY_OBJECTIVE = 16, TY_GRADIENT = 4, TY_FIELD = 16, TY_DEFORMATION = 4;
 
 // A floating image (with its margin) held as a 2D layered float array, one layer per z slice,
 // and its texture object. Arrays are pooled per process and reused across registrations:
@@ -475,7 +475,7 @@ size_t walk_smem_bytes(const WalkPlan& W);
 // co-resident blocks of the persistent voxel passes for a given dynamic shared-memory size
 long long objective_slots(size_t smem);
 long long gradient_slots(size_t smem);
-long long deformation_slots(size_t smem);
+long long field_slots(size_t smem);
 
 }  // namespace nrb
 

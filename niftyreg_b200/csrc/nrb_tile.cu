@@ -752,24 +752,31 @@ k_gradient(WalkParams P, const float *__restrict__ ref, const float *__restrict_
         gradient_item<kF32, kDiag, kTex>(P, S, logf, T, item, ref, flo, mask, cpp, vgrad);
 }
 
-// standalone deformation field (Compute::GetDeformationField) with the same arithmetic
-__global__ void __launch_bounds__(32 * TY_DEFORMATION)
+// standalone deformation field (Compute::GetDeformationField) with the same arithmetic, in the
+// objective's block shape: 16 rows share the staged nodes and their x contractions (kXs; when two
+// blocks per SM still fit), which leaves a thread 4 loads per component and node plane instead of
+// 16. Bound by the latency of an item's set-up and the stores; blocks of 4 rows without the x rows
+// took 75 us for 181x217x181 (96 registers, 27% of the warps).
+template <bool kXs>
+__global__ void __launch_bounds__(32 * TY_FIELD, 2)
 k_deformation(WalkParams P, const int32_t *__restrict__ mask, const float *__restrict__ cpp,
               float *__restrict__ def) {
     extern __shared__ float4 sm4[];
     const WalkSmem S = walk_smem(P, sm4);
-    const int nv = P.nx * P.ny * P.nz;
+    float *X = reinterpret_cast<float *>(S.tail);
+    const int nv = P.nx * P.ny * P.nz, zstride = P.nx * P.ny;
     for (int item = blockIdx.x; item < P.nitems; item += gridDim.x) {
         Item I;
         stage_item(P, cpp, item, S.cp, S.zb, S.zk, S.zid, I);
         Column C;
         column_init(P, I, S.cp, C);
+        if (kXs) build_xrows(P, C, S.cp, X);
         const int nzi = I.z1 - I.z0;
-        for (int zi = 0; zi < nzi; ++zi) {
+        int idx = (I.z0 * P.ny + C.y) * P.nx + C.x;
+        if (!C.inside) continue;
+        for (int zi = 0; zi < nzi; ++zi, idx += zstride) {
             float pos[3];
-            column_position(P, C, S.zb, S.zk, S.zid, zi, pos);
-            if (!C.inside) continue;
-            const int idx = ((I.z0 + zi) * P.ny + C.y) * P.nx + C.x;
+            column_position<kXs>(P, C, S.zb, S.zk, S.zid, zi, pos, X);
             if (mask != nullptr && __ldg(&mask[idx]) <= -1) pos[0] = pos[1] = pos[2] = 0.f;
             def[idx] = pos[0];
             def[nv + idx] = pos[1];
@@ -1099,27 +1106,30 @@ k_nmi_finalize(FinArgs A, cudaGraphConditionalHandle line) {
 // ---------------------------------------------------------------------------------------------
 // standalone resampling / histogram / voxel gradient (materialised intermediates)
 // ---------------------------------------------------------------------------------------------
-template <bool kGrad>
-__global__ void k_resample(long long nv, FloatingView V, Mat34 M, int diag, float pad,
-                           const float *__restrict__ flo, const float *__restrict__ def,
-                           const int32_t *__restrict__ mask, float *__restrict__ out) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
-         i += (long long)gridDim.x * blockDim.x) {
-        const bool active = mask == nullptr || mask[i] > -1;
-        if (!kGrad && !active) continue;
-        float w = 0.f, g[3] = { 0.f, 0.f, 0.f };
-        if (active) {
-            Footprint F;
-            fetch_footprint<-1, false>(flo, V, M, diag, pad, def[i], def[nv + i], def[2 * nv + i], F);
-            footprint_value<kGrad>(F, w, g);
-        }
-        if (kGrad) {
-            out[i] = g[0];
-            out[nv + i] = g[1];
-            out[2 * nv + i] = g[2];
-        } else {
-            out[i] = w;
-        }
+// One voxel per thread and few registers: the kernel waits on its position loads, then on the
+// gather, and the warps of six blocks per SM cover both (a grid-stride loop at
+// 48 registers took 56 us for the warp and 62 us for the gradient of 181x217x181).
+template <bool kGrad, int kDiag>
+__global__ void __launch_bounds__(256, 6)
+k_resample(long long nv, FloatingView V, Mat34 M, float pad, const float *__restrict__ flo, const float *__restrict__ def,
+           const int32_t *__restrict__ mask, float *__restrict__ out) {
+    const long long i = blockIdx.x * 256ll + threadIdx.x;
+    if (i >= nv) return;
+    const float x = __ldg(def + i), y = __ldg(def + nv + i), z = __ldg(def + 2 * nv + i);
+    const bool active = mask == nullptr || __ldg(mask + i) > -1;
+    if (!kGrad && !active) return;
+    float w = 0.f, g[3] = { 0.f, 0.f, 0.f };
+    if (active) {
+        Footprint F;
+        fetch_footprint<kDiag, false>(flo, V, M, 0, pad, x, y, z, F);
+        footprint_value<kGrad>(F, w, g);
+    }
+    if (kGrad) {
+        out[i] = g[0];
+        out[nv + i] = g[1];
+        out[2 * nv + i] = g[2];
+    } else {
+        out[i] = w;
     }
 }
 
@@ -1254,22 +1264,44 @@ k_warp_order(WalkParams P, const float *__restrict__ cpp, const float *__restric
     }
 }
 
-__global__ void k_histogram(long long nv, int rb, int fb, const float *__restrict__ ref,
-                            const float *__restrict__ war, const int32_t *__restrict__ mask,
-                            uint32_t *__restrict__ ghist) {
+// Joint histogram of two images in a block's shared memory, four voxels per thread in flight (all
+// loads before the first count), two blocks of 1024 threads per SM. A warp whose 32 voxels share one
+// bin (background) counts them with one atomic, as the fused pass does. Two blocks of 512 threads,
+// one voxel at a time: 30 us for 181x217x181 (latency).
+constexpr int HIST_THREADS = 1024, HIST_VOX = 4;
+__global__ void __launch_bounds__(HIST_THREADS, 2)
+k_histogram(long long nv, int rb, int fb, const float *__restrict__ ref, const float *__restrict__ war,
+            const int32_t *__restrict__ mask, uint32_t *__restrict__ ghist) {
     extern __shared__ uint32_t hs[];
     const int nbins = rb * fb;
-    for (int i = threadIdx.x; i < nbins; i += blockDim.x) hs[i] = 0u;
+    for (int i = threadIdx.x; i < nbins; i += HIST_THREADS) hs[i] = 0u;
     __syncthreads();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
-         i += (long long)gridDim.x * blockDim.x) {
-        if (mask != nullptr && mask[i] <= -1) continue;
-        const float r = ref[i], w = war[i];
-        if (r == r && w == w && 0.f <= r && r < (float)rb && 0.f <= w && w < (float)fb)
-            atomicAdd(&hs[(int)r + (int)w * rb], 1u);
+    const float frb = (float)rb, ffb = (float)fb;
+    for (long long base = blockIdx.x * (long long)(HIST_THREADS * HIST_VOX); base < nv;
+         base += (long long)gridDim.x * (HIST_THREADS * HIST_VOX)) {
+        float r[HIST_VOX], w[HIST_VOX];
+#pragma unroll
+        for (int u = 0; u < HIST_VOX; ++u) {
+            const long long i = base + u * HIST_THREADS + threadIdx.x;
+            r[u] = i < nv ? __ldg(ref + i) : -1.f;
+            w[u] = i < nv ? __ldg(war + i) : -1.f;
+            if (mask != nullptr && i < nv && __ldg(mask + i) <= -1) r[u] = -1.f;
+        }
+#pragma unroll
+        for (int u = 0; u < HIST_VOX; ++u) {
+            int bin = -1;
+            if (0.f <= r[u] && r[u] < frb && 0.f <= w[u] && w[u] < ffb)  // false for NaN
+                bin = (int)r[u] + (int)w[u] * rb;
+            const int b0 = __shfl_sync(0xffffffffu, bin, 0);
+            if (__all_sync(0xffffffffu, bin == b0)) {
+                if ((threadIdx.x & 31) == 0 && b0 >= 0) atomicAdd(&hs[b0], 32u);
+            } else if (bin >= 0) {
+                atomicAdd(&hs[bin], 1u);
+            }
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nbins; i += blockDim.x) {
+    for (int i = threadIdx.x; i < nbins; i += HIST_THREADS) {
         const uint32_t v = hs[i];
         if (v) atomicAdd(&ghist[i], v);
     }
@@ -1278,38 +1310,48 @@ __global__ void k_histogram(long long nv, int rb, int fb, const float *__restric
 // kF32: the Parzen window in FP32 on an FP32 copy of the log table in shared memory, as the fused
 // gradient runs it (the normalisation constant formed in FP64); otherwise the FP64 window on the
 // global table (tables too large for shared memory).
+//
+// Persistent blocks (the table is converted once per block), and a voxel's eight loads all issued
+// before the window: the kernel waits on memory, then on the window's shared-memory reads. With the
+// gradients loaded after the window, and 16 blocks per SM each converting the table, it took 117 us
+// for 181x217x181 with a mask.
 template <bool kF32>
-__global__ void k_nmi_voxel_gradient(long long nv, int rb, int fb, const float *__restrict__ ref,
-                                     const float *__restrict__ war, const float *__restrict__ wgrad,
-                                     const int32_t *__restrict__ mask, const double *__restrict__ logt,
-                                     const nrb_objective *__restrict__ last, double weight,
-                                     float *__restrict__ vgrad) {
+__global__ void __launch_bounds__(256, kF32 ? 4 : 2)
+k_nmi_voxel_gradient(long long nv, int rb, int fb, const float *__restrict__ ref, const float *__restrict__ war,
+                     const float *__restrict__ wgrad, const int32_t *__restrict__ mask,
+                     const double *__restrict__ logt, const nrb_objective *__restrict__ last, double weight,
+                     float *__restrict__ vgrad) {
     extern __shared__ float logf_sm[];
     const double nmi = last->nmi;
     const double scale = weight / (last->entropy[2] * last->entropy[3]);
     const float nmi_f = (float)nmi, scale_f = (float)scale;
     if (kF32) {
         const int total = rb * fb + rb + fb;
+#pragma unroll 4
         for (int i = threadIdx.x; i < total; i += blockDim.x) logf_sm[i] = (float)logt[i];
         __syncthreads();
     }
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
          i += (long long)gridDim.x * blockDim.x) {
-        if (mask != nullptr && mask[i] <= -1) continue;
-        const float r = ref[i], w = war[i];
+        if (mask != nullptr && __ldg(mask + i) <= -1) continue;
+        const float r = __ldg(ref + i), w = __ldg(war + i);
+        float g[3], v[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            g[d] = __ldg(wgrad + d * nv + i);
+            v[d] = vgrad[d * nv + i];
+        }
         if (!(r == r && w == w)) continue;
         if (kF32) {
             const float s = nmi_window_f(r, w, logf_sm, rb, fb, nmi_f);
-            for (int d = 0; d < 3; ++d) {
-                const float g = wgrad[d * nv + i];
-                if (g == g) vgrad[d * nv + i] += scale_f * (g * s);
-            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (g[d] == g[d]) vgrad[d * nv + i] = v[d] + scale_f * (g[d] * s);
         } else {
             const double s = nmi_window(r, w, logt, rb, fb, nmi);
-            for (int d = 0; d < 3; ++d) {
-                const float g = wgrad[d * nv + i];
-                if (g == g) vgrad[d * nv + i] += (float)(scale * ((double)g * s));
-            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (g[d] == g[d]) vgrad[d * nv + i] = v[d] + (float)(scale * ((double)g[d] * s));
         }
     }
 }
@@ -1533,7 +1575,7 @@ static auto pick_gradient(bool f32, bool diag, bool tex) { return with_flags<>(G
 
 long long objective_slots(size_t smem) { return blocks_resident(k_objective<true, true, true, true>, 32 * TY_OBJECTIVE, smem); }
 long long gradient_slots(size_t smem) { return blocks_resident(k_gradient<true, true, true>, 32 * TY_GRADIENT, smem); }
-long long deformation_slots(size_t smem) { return blocks_resident(k_deformation, 32 * TY_DEFORMATION, smem); }
+long long field_slots(size_t smem) { return blocks_resident(k_deformation<true>, 32 * TY_FIELD, smem); }
 
 template <int kOrder>
 static long long warp_slots(size_t smem) { return blocks_resident(k_warp_order<kOrder>, 32 * TY_DEFORMATION, smem); }
@@ -2019,12 +2061,15 @@ extern "C" nrb_status nrb_get_deformation_field(const nrb_geometry *g, const flo
                                                 const int32_t *mask, float *def, void *stream) {
     if (!g || !cpp || !def) return fail(NRB_ERR_INVALID, "nrb_get_deformation_field: null pointer");
     NRB_TRY(validate_geometry(g));
-    const WalkPlan W = plan_walk(g, TY_DEFORMATION, deformation_slots, 0);
+    const WalkPlan W = plan_walk(g, TY_FIELD, field_slots, 24 * 1024, 4, 6);
     const WalkParams P = make_params(W, g, 0.f, 0, 0);
-    const size_t smem = walk_smem_bytes(W);
+    const size_t rows = (size_t)3 * P.sc * P.sb * 32 * 4;
+    const bool xs = walk_smem_bytes(W) + rows <= 100 * 1024;
+    const size_t smem = walk_smem_bytes(W) + (xs ? rows : 0);
+    auto kernel = xs ? k_deformation<true> : k_deformation<false>;
     int grid = 0;
-    NRB_TRY(persistent_grid(k_deformation, 32 * W.ty, smem, P.nitems, grid));
-    k_deformation<<<grid, 32 * W.ty, smem, as_stream(stream)>>>(P, mask, cpp, def);
+    NRB_TRY(persistent_grid(kernel, 32 * W.ty, smem, P.nitems, grid));
+    kernel<<<grid, 32 * W.ty, smem, as_stream(stream)>>>(P, mask, cpp, def);
     NRB_LAUNCHED("k_deformation");
     return NRB_OK;
 }
@@ -2035,18 +2080,12 @@ static nrb_status resample_common(const nrb_geometry *g, const float *flo, const
     if (!g || !flo || !def || !out) return fail(NRB_ERR_INVALID, "resample: null pointer");
     const long long nv = nvox(g->ref_dim);
     if (nv <= 0) return fail(NRB_ERR_INVALID, "resample: empty reference");
-    const int threads = 256;
-    const int grid = (int)std::min<long long>((nv + threads - 1) / threads, 64LL * sm_count());
     const FloatingView V = floating_view(g->flo_dim[0], g->flo_dim[1], g->flo_dim[2], 0, 0ull);
     const Mat34 M = to_mat34(g->flo_ijk);
     const float *m = g->flo_ijk;
-    const int diag = m[1] == 0.f && m[2] == 0.f && m[4] == 0.f && m[6] == 0.f && m[8] == 0.f && m[9] == 0.f;
-    if (grad)
-        k_resample<true><<<grid, threads, 0, as_stream(stream)>>>(nv, V, M,
-                                                                  diag, pad, flo, def, mask, out);
-    else
-        k_resample<false><<<grid, threads, 0, as_stream(stream)>>>(nv, V, M,
-                                                                   diag, pad, flo, def, mask, out);
+    const bool diag = m[1] == 0.f && m[2] == 0.f && m[4] == 0.f && m[6] == 0.f && m[8] == 0.f && m[9] == 0.f;
+    auto kernel = grad ? (diag ? k_resample<true, 1> : k_resample<true, 0>) : (diag ? k_resample<false, 1> : k_resample<false, 0>);
+    kernel<<<(unsigned)((nv + 255) / 256), 256, 0, as_stream(stream)>>>(nv, V, M, pad, flo, def, mask, out);
     NRB_LAUNCHED("k_resample");
     return NRB_OK;
 }
@@ -2118,8 +2157,8 @@ extern "C" nrb_status nrb_nmi_value(nrb_nmi *nmi, const nrb_geometry *g, const f
     if (!nmi || !g || !ref || !warped) return fail(NRB_ERR_INVALID, "nrb_nmi_value: null pointer");
     const long long nv = nvox(g->ref_dim);
     cudaStream_t st = as_stream(stream);
-    const int threads = 512;
-    const int grid = (int)std::min<long long>((nv + threads - 1) / threads, 2LL * sm_count());
+    const int threads = HIST_THREADS;
+    const int grid = (int)std::min<long long>((nv + threads * HIST_VOX - 1) / (threads * HIST_VOX), 2LL * sm_count());
     const size_t smem = (size_t)nmi->rb * nmi->fb * 4;
     NRB_CUDA(cudaFuncSetAttribute(k_histogram, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     k_histogram<<<grid, threads, smem, st>>>(nv, nmi->rb, nmi->fb, ref, warped, mask, nmi->hist);
@@ -2142,18 +2181,17 @@ nrb_status nmi_voxel_gradient(nrb_nmi *nmi, const nrb_geometry *g, const float *
                               cudaStream_t st, bool fp64) {
     const long long nv = nvox(g->ref_dim);
     const int threads = 256;
-    const int grid = (int)std::min<long long>((nv + threads - 1) / threads, 16LL * sm_count());
     // the FP32 window when the log table fits in shared memory (64 bins: 19 KB, 128 bins: 70 KB)
     const size_t log_bytes = (size_t)nmi->total * sizeof(float);
-    if (!fp64 && log_bytes <= 96 * 1024) {
-        NRB_CUDA(cudaFuncSetAttribute(k_nmi_voxel_gradient<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)log_bytes));
-        k_nmi_voxel_gradient<true><<<grid, threads, log_bytes, st>>>(nv, nmi->rb, nmi->fb, ref, warped, warped_grad,
-                                                                     mask, nmi->logt, nmi->last, weight, vgrad);
-    } else {
-        k_nmi_voxel_gradient<false><<<grid, threads, 0, st>>>(nv, nmi->rb, nmi->fb, ref, warped, warped_grad, mask,
-                                                              nmi->logt, nmi->last, weight, vgrad);
-    }
+    const bool f32 = !fp64 && log_bytes <= 96 * 1024;
+    auto kernel = f32 ? k_nmi_voxel_gradient<true> : k_nmi_voxel_gradient<false>;
+    const size_t smem = f32 ? log_bytes : 0;
+    if (f32) NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)log_bytes));
+    int per = 0;
+    NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
+    const int grid = (int)std::min<long long>((nv + threads - 1) / threads, (long long)std::max(1, per) * sm_count());
+    kernel<<<grid, threads, smem, st>>>(nv, nmi->rb, nmi->fb, ref, warped, warped_grad, mask, nmi->logt, nmi->last, weight,
+                                        vgrad);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_nmi_voxel_gradient");
     return NRB_OK;
