@@ -207,7 +207,8 @@ struct BatchLaunch {
     int npairs = 0;
     BatchObjTable obj_table;
     BatchGradTable grad_table;
-    bool obj_xs = false, obj_diag = false, grad_f32 = false, grad_diag = false, tex = false;
+    bool obj_xs = false, obj_diag = false, grad_f32 = false, grad_diag = false;
+    int fetch = 0;  // how the floating images are read (Fetch)
     size_t obj_smem = 0, grad_smem = 0, fin_smem = 0;
     int obj_grid = 0, grad_grid = 0;
 };

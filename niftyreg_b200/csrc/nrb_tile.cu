@@ -324,7 +324,7 @@ __device__ __forceinline__ void gather_footprint(unsigned long long tex, int lay
     v[0][0] = r3;
 }
 
-// kTex (needs margin >= 2): the same floating image with its margin as a 2D layered float array
+// FETCH_TEX (needs margin >= 2): the same floating image with its margin as a 2D layered float array
 // (layer k = slice k - margin, texel (i, j) = voxel (i - margin, j - margin)); every sample then
 // fetches each slice's 2x2 footprint with one gather instead of four loads, with no warp vote and
 // no clamped path.
@@ -336,7 +336,14 @@ struct Footprint {
     float rx, ry, rz;  // position within the footprint
 };
 
-template <int kDiag, bool kTex>
+// kFetch: how the floating image is read. FETCH_TEX as above; FETCH_NAN for a NaN padding value and
+// at least two voxels per axis: any tap outside makes the value NaN and the gradient 0 whatever the
+// others hold, so the footprint is moved inside and one of its values replaced by NaN, with no vote
+// and no second path (in FETCH_ANY a warp with an outside tap, a quarter of them at 182x218x182,
+// runs the clamped path: eight addresses, eight tests). k_objective at 182x218x182: 91 -> 81 us.
+enum Fetch : int { FETCH_ANY = 0, FETCH_NAN = 1, FETCH_TEX = 2 };
+
+template <int kDiag, int kFetch>
 __device__ __forceinline__ void fetch_footprint(const float *__restrict__ flo, const FloatingView& V, const Mat34& M,
                                                 int diag, float pad, float x, float y, float z, Footprint& S) {
     float fx, fy, fz;
@@ -346,7 +353,7 @@ __device__ __forceinline__ void fetch_footprint(const float *__restrict__ flo, c
     S.rx = fx - flx;
     S.ry = fy - fly;
     S.rz = fz - flz;
-    if (kTex) {
+    if (kFetch == FETCH_TEX) {
         // every sample, no vote: the footprint's first texel (p + margin on each axis) clamped to
         // [0, n + 2 margin - 2]. Unclamped, that is the plain path's footprint; clamped, both taps
         // on that axis lie outside the volume (p < -margin or p > n + margin - 2) and the clamped
@@ -363,8 +370,14 @@ __device__ __forceinline__ void fetch_footprint(const float *__restrict__ flo, c
     const bool plain = (unsigned)(px + V.margin) < (unsigned)(V.nx + 2 * V.margin - 1) &&
                        (unsigned)(py + V.margin) < (unsigned)(V.ny + 2 * V.margin - 1) &&
                        (unsigned)(pz + V.margin) < (unsigned)(V.nz + 2 * V.margin - 1);
-    if (__all_sync(__activemask(), plain)) {
-        const float *p = flo + (pz * V.sz + py * V.sy + px);
+    if (kFetch == FETCH_NAN || __all_sync(__activemask(), plain)) {
+        int qx = px, qy = py, qz = pz;
+        if (kFetch == FETCH_NAN) {
+            qx = min(max(px, -V.margin), V.nx + V.margin - 2);
+            qy = min(max(py, -V.margin), V.ny + V.margin - 2);
+            qz = min(max(pz, -V.margin), V.nz + V.margin - 2);
+        }
+        const float *p = flo + (qz * V.sz + qy * V.sy + qx);
         S.v[0][0][0] = __ldg(p);
         S.v[0][0][1] = __ldg(p + 1);
         S.v[0][1][0] = __ldg(p + V.sy);
@@ -373,6 +386,7 @@ __device__ __forceinline__ void fetch_footprint(const float *__restrict__ flo, c
         S.v[1][0][1] = __ldg(p + V.sz + 1);
         S.v[1][1][0] = __ldg(p + V.sz + V.sy);
         S.v[1][1][1] = __ldg(p + V.sz + V.sy + 1);
+        if (kFetch == FETCH_NAN && !plain) S.v[0][0][0] = __int_as_float(0x7fffffff);
         return;
     }
     const bool inx[2] = { (unsigned)px < (unsigned)V.nx, (unsigned)(px + 1) < (unsigned)V.nx };
@@ -476,7 +490,7 @@ __device__ __forceinline__ void flush_hist(const uint32_t *h, int nbins, uint32_
 // The walk is one slice ahead of itself: the position of slice z + 1 is evaluated and its fetches
 // issued before slice z's are consumed, so a warp always has a slice's gathers in flight. Columns
 // outside the volume walk the nearest inside one and count nothing (no divergence).
-template <bool kXs, bool kDiag, bool kTex>
+template <bool kXs, bool kDiag, int kFetch>
 __device__ __forceinline__ void objective_item(const WalkParams& P, const WalkSmem& S, uint32_t *h, float *X,
                                                int item, const float *__restrict__ ref,
                                                const float *__restrict__ flo, const int32_t *__restrict__ mask,
@@ -495,7 +509,7 @@ __device__ __forceinline__ void objective_item(const WalkParams& P, const WalkSm
     auto issue = [&](int zi, Footprint& F, float& rv) {
         float pos[3];
         column_position<kXs>(P, C, S.zb, S.zk, S.zid, zi, pos, X);
-        fetch_footprint<kDiag ? 1 : 0, kTex>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
+        fetch_footprint<kDiag ? 1 : 0, kFetch>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
         rv = __ldg(&ref[idx]);
         if (mask != nullptr && __ldg(&mask[idx]) <= -1) rv = -1.f;
         idx += zstride;
@@ -533,9 +547,9 @@ __device__ __forceinline__ void objective_smem(const WalkParams& P, void *base, 
 // fused objective: deformation + warp + joint histogram
 // ---------------------------------------------------------------------------------------------
 // kXs: the item's x-contracted node rows are staged in shared memory; kDiag: the floating
-// image's mm -> voxel matrix has no off-diagonal terms; kTex: the floating image is held as a
-// texture (launch-time choices made template parameters, so the walk carries no test for them)
-template <bool kTrial, bool kXs, bool kDiag, bool kTex>
+// image's mm -> voxel matrix has no off-diagonal terms; kFetch: how the floating image is
+// read (launch-time choices made template parameters, so the walk carries no test for them)
+template <bool kTrial, bool kXs, bool kDiag, int kFetch>
 __global__ void __launch_bounds__(32 * TY_OBJECTIVE, 2)
 k_objective(WalkParams P, const float *__restrict__ ref, const float *__restrict__ flo,
             const int32_t *__restrict__ mask, const float *__restrict__ cpp,
@@ -551,7 +565,7 @@ k_objective(WalkParams P, const float *__restrict__ ref, const float *__restrict
     pdl_launch_dependents();  // the finalize may start its preamble (it waits for the counts)
     const float scale = kTrial ? -step->cur_len : 0.f;
     for (int item = blockIdx.x; item < P.nitems; item += gridDim.x)
-        objective_item<kXs, kDiag, kTex>(P, S, h, X, item, ref, flo, mask, cpp, kTrial ? grad : nullptr, scale);
+        objective_item<kXs, kDiag, kFetch>(P, S, h, X, item, ref, flo, mask, cpp, kTrial ? grad : nullptr, scale);
     flush_hist(h, nbins, ghist);
 }
 
@@ -594,6 +608,9 @@ __device__ __forceinline__ double nmi_window(float rv, float wv, const double *l
     return sr + sw - nmi * sj;
 }
 
+// k_gradient at 182x218x182 went from 179 to 152 us with this window and the fetch modes (115 M ->
+// 101 M warp instructions, no spills at 80 registers).
+//
 // The same window in FP32 on an FP32 copy of the log table (the fused gradient pass): the
 // per-voxel terms are a 16-tap weighted sum whose FP32 rounding (~1e-6 relative) stays far
 // below the voxel-face jumps of the trilinear spatial gradient, while the FP64 normalisation
@@ -601,51 +618,62 @@ __device__ __forceinline__ double nmi_window(float rv, float wv, const double *l
 __device__ __forceinline__ float nmi_window_f(float rv, float wv, const float *logt, int rb, int fb, float nmi) {
     const float *rlog = logt + rb * fb;
     const float *wlog = rlog + rb;
-    const int r0 = (int)(rv - 1.f), r1 = (int)(rv + 3.f);
-    const int w0 = (int)(wv - 1.f), w1 = (int)(wv + 3.f);
-    // taps outside the window or the table get weight 0 and a clamped (valid) table index, so
-    // the sums need no branches; the marginal terms factor out of the double sum:
+    // the marginal terms factor out of the double sum:
     //   sum_tu br_t dw_u rlog_t = (sum_t br_t rlog_t)(sum_u dw_u), and likewise for wlog
-    float br[4], dw[4], rl[4], wl[4];
-    int ri[4], wi[4];
+    float br[4], dw[4];
     if (rv >= 1.f && wv >= 1.f && rv < (float)(rb - 2) && wv < (float)(fb - 2)) {
-        // r0 + 1 = floor(rv): the four taps sit at rv - r = f + 1, f, f - 1, f - 2 (all exact)
-        // with f the fractional part, each inside one known piece of the kernel. The pieces
-        // parzenf / parzen_derivf would select are written out with their operations in their
-        // order (sign changes are exact), so every value is the same float; only |x| = 1 at
-        // f = 0 falls in the other piece and is given its value (1/6) explicitly.
-        const float f = rv - (float)(r0 + 1), mf = 1.f - f;
+        // the four taps sit at rv - r = f + 1, f, f - 1, f - 2 (all exact) with f the fractional
+        // part, each inside one known piece of the kernel. The pieces parzenf / parzen_derivf would
+        // select are written out with their operations in their order (sign changes are exact), so
+        // every value is the same float; only |x| = 1 at f = 0 falls in the other piece and is given
+        // its value (1/6) explicitly. The taps floor(v) - 1 .. floor(v) + 2 all lie in the table, so
+        // none is masked or clamped, and the 16 table reads are constant offsets from one pointer per
+        // row (a clamped index per tap cost an addition and a shift each).
+        float flr, flw;
+        const int r0 = floor_split(rv, flr) - 1, w0 = floor_split(wv, flw) - 1;
+        const float f = rv - flr, mf = 1.f - f;
         br[0] = mf * mf * mf * (1.f / 6.f);
         br[1] = (2.0f / 3.0f) + (0.5f * f - 1.f) * f * f;
         br[2] = mf < 1.f ? (2.0f / 3.0f) + (0.5f * mf - 1.f) * mf * mf : (1.f / 6.f);
         br[3] = f * f * f * (1.f / 6.f);
-        const float g = wv - (float)(w0 + 1), mg = 1.f - g;
+        const float g = wv - flw, mg = 1.f - g;
         dw[0] = -0.5f * mg * mg;
         dw[1] = (1.5f * g - 2.f) * g;
         dw[2] = (1.5f * mg - 2.f) * -mg;
         dw[3] = 0.5f * g * g;
-        // 1 <= rv < rb - 2: the taps r0 .. r0 + 3 = floor(rv) - 1 .. floor(rv) + 2 all lie in the
-        // table (and likewise for wv), so none is masked or clamped
+        const float *p0 = logt + w0 * rb + r0, *p1 = p0 + rb, *p2 = p1 + rb, *p3 = p2 + rb;
+        const float *pr = rlog + r0, *pw = wlog + w0;
+        float sbr = 0.f, sdw = 0.f, sr = 0.f, sw = 0.f, sj = 0.f;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            ri[t] = r0 + t;
-            wi[t] = (w0 + t) * rb;
-            rl[t] = rlog[r0 + t];
-            wl[t] = wlog[w0 + t];
+            sbr += br[t];
+            sdw += dw[t];
+            sr = fmaf(br[t], pr[t], sr);
+            sw = fmaf(dw[t], pw[t], sw);
+            float row = fmaf(dw[0], p0[t], 0.f);
+            row = fmaf(dw[1], p1[t], row);
+            row = fmaf(dw[2], p2[t], row);
+            row = fmaf(dw[3], p3[t], row);
+            sj = fmaf(br[t], row, sj);
         }
-    } else {
+        return fmaf(sr, sdw, sbr * sw) - nmi * sj;
+    }
+    // taps outside the window or the table get weight 0 and a clamped (valid) table index
+    const int r0 = (int)(rv - 1.f), r1 = (int)(rv + 3.f);
+    const int w0 = (int)(wv - 1.f), w1 = (int)(wv + 3.f);
+    float rl[4], wl[4];
+    int ri[4], wi[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int r = r0 + t, w = w0 + t;
-            const bool rok = r < r1 && -1 < r && r < rb;
-            const bool wok = w < w1 && -1 < w && w < fb;
-            ri[t] = min(max(r, 0), rb - 1);
-            wi[t] = min(max(w, 0), fb - 1) * rb;
-            br[t] = rok ? parzenf(rv - (float)r) : 0.f;
-            dw[t] = wok ? parzen_derivf(wv - (float)w) : 0.f;
-            rl[t] = rlog[ri[t]];
-            wl[t] = wlog[min(max(w, 0), fb - 1)];
-        }
+    for (int t = 0; t < 4; ++t) {
+        const int r = r0 + t, w = w0 + t;
+        const bool rok = r < r1 && -1 < r && r < rb;
+        const bool wok = w < w1 && -1 < w && w < fb;
+        ri[t] = min(max(r, 0), rb - 1);
+        wi[t] = min(max(w, 0), fb - 1) * rb;
+        br[t] = rok ? parzenf(rv - (float)r) : 0.f;
+        dw[t] = wok ? parzen_derivf(wv - (float)w) : 0.f;
+        rl[t] = rlog[ri[t]];
+        wl[t] = wlog[min(max(w, 0), fb - 1)];
     }
     float sbr = 0.f, sdw = 0.f, sr = 0.f, sw = 0.f, sj = 0.f;
 #pragma unroll
@@ -695,7 +723,7 @@ __device__ __forceinline__ void stage_log_table(const WalkParams& P, const doubl
 
 // One item of the fused gradient: stage the item's control points, walk its columns and write
 // every voxel's NMI gradient (zero where masked or NaN). Called by every thread of the block.
-template <bool kF32, bool kDiag, bool kTex>
+template <bool kF32, bool kDiag, int kFetch>
 __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSmem& S, const float *logf,
                                               const GradientTables& T, int item, const float *__restrict__ ref,
                                               const float *__restrict__ flo, const int32_t *__restrict__ mask,
@@ -716,7 +744,7 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
         if (mask == nullptr || __ldg(&mask[idx]) > -1) {
             Footprint F;
             float w, g[3];
-            fetch_footprint<kDiag ? 1 : 0, kTex>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
+            fetch_footprint<kDiag ? 1 : 0, kFetch>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
             const float rv = __ldg(&ref[idx]);
             footprint_value<true>(F, w, g);
             if (rv == rv && w == w) {
@@ -737,7 +765,7 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
     }
 }
 
-template <bool kF32, bool kDiag, bool kTex>
+template <bool kF32, bool kDiag, int kFetch>
 __global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 6 : 4)
 k_gradient(WalkParams P, const float *__restrict__ ref, const float *__restrict__ flo,
            const int32_t *__restrict__ mask, const float *__restrict__ cpp,
@@ -749,7 +777,7 @@ k_gradient(WalkParams P, const float *__restrict__ ref, const float *__restrict_
     float *logf = reinterpret_cast<float *>(S.tail);
     if (kF32) stage_log_table(P, T.logt, logf);
     for (int item = blockIdx.x; item < P.nitems; item += gridDim.x)
-        gradient_item<kF32, kDiag, kTex>(P, S, logf, T, item, ref, flo, mask, cpp, vgrad);
+        gradient_item<kF32, kDiag, kFetch>(P, S, logf, T, item, ref, flo, mask, cpp, vgrad);
 }
 
 // standalone deformation field (Compute::GetDeformationField) with the same arithmetic, in the
@@ -1109,7 +1137,7 @@ k_nmi_finalize(FinArgs A, cudaGraphConditionalHandle line) {
 // One voxel per thread and few registers: the kernel waits on its position loads, then on the
 // gather, and the warps of six blocks per SM cover both (a grid-stride loop at
 // 48 registers took 56 us for the warp and 62 us for the gradient of 181x217x181).
-template <bool kGrad, int kDiag>
+template <bool kGrad, int kDiag, int kFetch>
 __global__ void __launch_bounds__(256, 6)
 k_resample(long long nv, FloatingView V, Mat34 M, float pad, const float *__restrict__ flo, const float *__restrict__ def,
            const int32_t *__restrict__ mask, float *__restrict__ out) {
@@ -1121,7 +1149,7 @@ k_resample(long long nv, FloatingView V, Mat34 M, float pad, const float *__rest
     float w = 0.f, g[3] = { 0.f, 0.f, 0.f };
     if (active) {
         Footprint F;
-        fetch_footprint<kDiag, false>(flo, V, M, 0, pad, x, y, z, F);
+        fetch_footprint<kDiag, kFetch>(flo, V, M, 0, pad, x, y, z, F);
         footprint_value<kGrad>(F, w, g);
     }
     if (kGrad) {
@@ -1362,7 +1390,7 @@ k_nmi_voxel_gradient(long long nv, int rb, int fb, const float *__restrict__ ref
 // The objective of every pair in INIT (at best) or LINE (at best - cur_len * grad): each block
 // walks its share of the pairs' items with the pair's own walk and histogram, exactly the
 // plain k_objective's work per item.
-template <bool kXs, bool kDiag, bool kTex>
+template <bool kXs, bool kDiag, int kFetch>
 __global__ void __launch_bounds__(32 * TY_OBJECTIVE, 2)
 k_b_objective(const __grid_constant__ BatchObjTable T, const OptState *__restrict__ states, int npairs) {
     extern __shared__ float4 sm4[];
@@ -1386,7 +1414,7 @@ k_b_objective(const __grid_constant__ BatchObjTable T, const OptState *__restric
         for (int j = G.j0[sg]; j < G.j1[sg]; ++j) {
             const int q = G.pair[sg];
             const bool line = states[q].phase == PH_LINE;
-            objective_item<kXs, kDiag, kTex>(T.e[q].P, S, h, X, j, T.e[q].ref, T.e[q].flo, nullptr, T.e[q].best,
+            objective_item<kXs, kDiag, kFetch>(T.e[q].P, S, h, X, j, T.e[q].ref, T.e[q].flo, nullptr, T.e[q].best,
                                        line ? T.e[q].grad : nullptr, line ? -states[q].cur_len : 0.f);
         }
         flush_hist(h, nbins, T.e[G.pair[sg]].hist);
@@ -1395,7 +1423,7 @@ k_b_objective(const __grid_constant__ BatchObjTable T, const OptState *__restric
 
 // The fused voxel gradient of every pair in GRAD, at best, with the NMI tables of its best
 // position (the plain k_gradient's work per item).
-template <bool kF32, bool kDiag, bool kTex>
+template <bool kF32, bool kDiag, int kFetch>
 __global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 6 : 4)
 k_b_gradient(const __grid_constant__ BatchGradTable T, const OptState *__restrict__ states, int npairs) {
     extern __shared__ float4 sm4[];
@@ -1416,7 +1444,7 @@ k_b_gradient(const __grid_constant__ BatchGradTable T, const OptState *__restric
         __syncthreads();  // the previous pair's walk is done with the shared tables
         if (kF32) stage_log_table(E.P, N.logt, logf);  // visible after stage_item's first barrier
         for (int j = G.j0[sg]; j < G.j1[sg]; ++j)
-            gradient_item<kF32, kDiag, kTex>(E.P, S, logf, N, j, E.ref, E.flo, nullptr, E.best, E.vgrad);
+            gradient_item<kF32, kDiag, kFetch>(E.P, S, logf, N, j, E.ref, E.flo, nullptr, E.best, E.vgrad);
     }
 }
 
@@ -1558,23 +1586,48 @@ template <bool... kDone, typename F, typename... Rest>
 static auto with_flags(F f, bool first, Rest... rest) {
     return first ? with_flags<kDone..., true>(f, rest...) : with_flags<kDone..., false>(f, rest...);
 }
+// NaN padding and a floating image of at least two voxels per axis take FETCH_NAN; a texture comes
+// before both. Batches share one mode: a pair that needs another sends all to the one they allow.
+static int fetch_mode(const FloatingView& V, float pad) {
+    if (V.tex) return FETCH_TEX;
+    return pad != pad && V.nx >= 2 && V.ny >= 2 && V.nz >= 2 ? FETCH_NAN : FETCH_ANY;
+}
+template <bool kTexOrNan, bool kTexture>
+constexpr int fetch_of() { return kTexture ? FETCH_TEX : kTexOrNan ? FETCH_NAN : FETCH_ANY; }
 struct ObjectiveKernel {
-    template <bool kTrial, bool kXs, bool kDiag, bool kTex> auto operator()() const { return k_objective<kTrial, kXs, kDiag, kTex>; }
+    template <bool kTrial, bool kXs, bool kDiag, bool kNan, bool kTex> auto operator()() const {
+        return k_objective<kTrial, kXs, kDiag, fetch_of<kNan, kTex>()>;
+    }
 };
 struct GradientKernel {
-    template <bool kF32, bool kDiag, bool kTex> auto operator()() const { return k_gradient<kF32, kDiag, kTex>; }
+    template <bool kF32, bool kDiag, bool kNan, bool kTex> auto operator()() const {
+        return k_gradient<kF32, kDiag, fetch_of<kNan, kTex>()>;
+    }
 };
 struct BatchObjectiveKernel {
-    template <bool kXs, bool kDiag, bool kTex> auto operator()() const { return k_b_objective<kXs, kDiag, kTex>; }
+    template <bool kXs, bool kDiag, bool kNan, bool kTex> auto operator()() const {
+        return k_b_objective<kXs, kDiag, fetch_of<kNan, kTex>()>;
+    }
 };
 struct BatchGradientKernel {
-    template <bool kF32, bool kDiag, bool kTex> auto operator()() const { return k_b_gradient<kF32, kDiag, kTex>; }
+    template <bool kF32, bool kDiag, bool kNan, bool kTex> auto operator()() const {
+        return k_b_gradient<kF32, kDiag, fetch_of<kNan, kTex>()>;
+    }
 };
-static auto pick_objective(bool trial, bool xs, bool diag, bool tex) { return with_flags<>(ObjectiveKernel{}, trial, xs, diag, tex); }
-static auto pick_gradient(bool f32, bool diag, bool tex) { return with_flags<>(GradientKernel{}, f32, diag, tex); }
+struct ResampleKernel {
+    template <bool kGrad, bool kDiag, bool kNan> auto operator()() const {
+        return k_resample<kGrad, kDiag ? 1 : 0, kNan ? FETCH_NAN : FETCH_ANY>;
+    }
+};
+static auto pick_objective(bool trial, bool xs, bool diag, int fetch) {
+    return with_flags<>(ObjectiveKernel{}, trial, xs, diag, fetch == FETCH_NAN, fetch == FETCH_TEX);
+}
+static auto pick_gradient(bool f32, bool diag, int fetch) {
+    return with_flags<>(GradientKernel{}, f32, diag, fetch == FETCH_NAN, fetch == FETCH_TEX);
+}
 
-long long objective_slots(size_t smem) { return blocks_resident(k_objective<true, true, true, true>, 32 * TY_OBJECTIVE, smem); }
-long long gradient_slots(size_t smem) { return blocks_resident(k_gradient<true, true, true>, 32 * TY_GRADIENT, smem); }
+long long objective_slots(size_t smem) { return blocks_resident(k_objective<true, true, true, FETCH_TEX>, 32 * TY_OBJECTIVE, smem); }
+long long gradient_slots(size_t smem) { return blocks_resident(k_gradient<true, true, FETCH_TEX>, 32 * TY_GRADIENT, smem); }
 long long field_slots(size_t smem) { return blocks_resident(k_deformation<true>, 32 * TY_FIELD, smem); }
 
 template <int kOrder>
@@ -1593,7 +1646,7 @@ nrb_status launch_fused_objective(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geo
     const size_t smem = base_smem + (P.xs ? xs_bytes : 0);
     const int threads = 32 * ws->walk_obj.ty;
     const bool trial = grad != nullptr;
-    auto kernel = pick_objective(trial, P.xs, P.flo_diag, P.fv.tex != 0);
+    auto kernel = pick_objective(trial, P.xs, P.flo_diag, fetch_mode(P.fv, P.pad));
     int grid = 0;
     NRB_TRY(persistent_grid(kernel, threads, smem, P.nitems, grid, ws->walk_obj.resident));
     // algorithmic bytes: reference + floating (+ mask) per voxel, the grid once
@@ -1623,7 +1676,7 @@ nrb_status launch_fused_gradient(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geom
     const size_t smem = walk_smem_bytes(ws->walk_grad) + (P.log_in_smem ? log_bytes : 0);
     const int threads = 32 * ws->walk_grad.ty;
     int grid = 0;
-    auto kernel = pick_gradient(P.log_in_smem, P.flo_diag, P.fv.tex != 0);
+    auto kernel = pick_gradient(P.log_in_smem, P.flo_diag, fetch_mode(P.fv, P.pad));
     NRB_TRY(persistent_grid(kernel, threads, smem, P.nitems, grid, ws->walk_grad.resident));
     // algorithmic bytes: reference + floating (+ mask) read, voxel gradient written, grid once
     const double nv = (double)P.nx * P.ny * P.nz;
@@ -1865,7 +1918,7 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
     if (L.npairs < 1 || L.npairs > BATCH_MAX_PAIRS)
         return fail(NRB_ERR_INVALID, "batched level: 1 to " + std::to_string(BATCH_MAX_PAIRS) + " pairs");
     size_t base = 0, xs = 0, gsm = 0;
-    bool diag = true, f32 = true, tex = true;  // tex: textures serve only if every pair has one
+    bool diag = true, f32 = true, tex = true, nan = true;
     int rb = pairs[0].rb, fb = pairs[0].fb;
     for (const BatchPair& b : pairs) {
         if (b.rb != rb || b.fb != fb) return fail(NRB_ERR_INVALID, "batched level: every pair needs the same bins");
@@ -1878,8 +1931,11 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
         diag = diag && b.wo.flo_diag;
         f32 = f32 && b.wg.log_in_smem;
         tex = tex && b.wo.fv.tex != 0;
+        FloatingView plain = b.wo.fv;
+        plain.tex = 0;
+        nan = nan && fetch_mode(plain, b.wo.pad) == FETCH_NAN;
     }
-    L.tex = tex;
+    L.fetch = tex ? FETCH_TEX : nan ? FETCH_NAN : FETCH_ANY;
     L.obj_xs = base + xs <= 100 * 1024;
     L.obj_diag = diag;
     L.obj_smem = base + (L.obj_xs ? xs : 0);
@@ -1910,8 +1966,8 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
         g.last0 = b.last0;
         g.last1 = b.last1;
     }
-    auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.tex);
-    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.tex);
+    auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
+    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
     int per = 0;
     NRB_CUDA(cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ko, 32 * TY_OBJECTIVE, L.obj_smem));
@@ -1926,7 +1982,7 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
 nrb_status launch_batch_objective(const BatchPair *d_pairs, const OptState *states, const BatchLaunch& L,
                                   cudaStream_t st, double bytes) {
     KernelTimer timer(TK_OBJECTIVE, bytes, st);
-    auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.tex);
+    auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
     ko<<<L.obj_grid, 32 * TY_OBJECTIVE, L.obj_smem, st>>>(L.obj_table, states, L.npairs);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_objective");
@@ -1936,7 +1992,7 @@ nrb_status launch_batch_objective(const BatchPair *d_pairs, const OptState *stat
 nrb_status launch_batch_gradient(const BatchPair *d_pairs, const OptState *states, const BatchLaunch& L,
                                  cudaStream_t st, double bytes) {
     KernelTimer timer(TK_GRADIENT, bytes, st);
-    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.tex);
+    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
     kg<<<L.grad_grid, 32 * TY_GRADIENT, L.grad_smem, st>>>(L.grad_table, states, L.npairs);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_gradient");
@@ -2084,7 +2140,7 @@ static nrb_status resample_common(const nrb_geometry *g, const float *flo, const
     const Mat34 M = to_mat34(g->flo_ijk);
     const float *m = g->flo_ijk;
     const bool diag = m[1] == 0.f && m[2] == 0.f && m[4] == 0.f && m[6] == 0.f && m[8] == 0.f && m[9] == 0.f;
-    auto kernel = grad ? (diag ? k_resample<true, 1> : k_resample<true, 0>) : (diag ? k_resample<false, 1> : k_resample<false, 0>);
+    auto kernel = with_flags<>(ResampleKernel{}, grad, diag, fetch_mode(V, pad) == FETCH_NAN);
     kernel<<<(unsigned)((nv + 255) / 256), 256, 0, as_stream(stream)>>>(nv, V, M, pad, flo, def, mask, out);
     NRB_LAUNCHED("k_resample");
     return NRB_OK;
