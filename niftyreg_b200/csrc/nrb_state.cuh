@@ -17,9 +17,9 @@ namespace nrb {
 // `zchunk` slices; a block of ty warps stages the item's control points once and each thread
 // walks its voxel column along z. The objective pass uses tall blocks (one shared histogram for
 // 16 warps leaves most of the SM's L1 to the floating-image gathers); the gradient pass, whose
-// threads carry more registers, uses 4 warps.
+// threads carry more registers, uses 8 warps.
 constexpr int COL_X = 32;
-constexpr int TY_OBJECTIVE = 16, TY_GRADIENT = 4, TY_FIELD = 16, TY_DEFORMATION = 4;
+constexpr int TY_OBJECTIVE = 16, TY_GRADIENT = 8, TY_FIELD = 16, TY_DEFORMATION = 4;
 
 // A floating image (with its margin) held as a 2D layered float array, one layer per z slice,
 // and its texture object. Arrays are pooled per process and reused across registrations:
@@ -77,7 +77,7 @@ struct WalkParams {
     float frb, ffb;          // the same as floats
     int cnv;                 // control points per component
     int log_in_smem;         // gradient: an FP32 copy of the log table is staged in shared memory
-    int xs;                  // objective: x-contracted rows of the item staged in shared memory
+    int xs;                  // x-contracted rows of the item staged in shared memory
     // identity split of the positions (grid matrix without off-diagonal terms; zero otherwise):
     // node k of axis c sits at io[c] + is[c] * k mm when the transformation is the identity
     float io[3], is[3];
@@ -207,7 +207,7 @@ struct BatchLaunch {
     int npairs = 0;
     BatchObjTable obj_table;
     BatchGradTable grad_table;
-    bool obj_xs = false, obj_diag = false, grad_f32 = false, grad_diag = false;
+    bool obj_xs = false, obj_diag = false, grad_f32 = false, grad_diag = false, grad_xs = false;
     int fetch = 0;  // how the floating images are read (Fetch)
     size_t obj_smem = 0, grad_smem = 0, fin_smem = 0;
     int obj_grid = 0, grad_grid = 0;

@@ -16,6 +16,7 @@
 #include <cooperative_groups.h>
 #include <cuda_pipeline.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -721,10 +722,16 @@ __device__ __forceinline__ void stage_log_table(const WalkParams& P, const doubl
     for (int i = threadIdx.x; i < total; i += blockDim.x) logf[i] = (float)logt[i];
 }
 
+// shared layout of a gradient block: walk | log table (FP32 window) | x-contracted rows (kXs)
+__host__ __device__ inline int gradient_log_floats(int rb, int fb) { return (rb * fb + rb + fb + 3) & ~3; }
+__device__ __forceinline__ float *gradient_xrows(const WalkParams& P, float *logf, bool f32) {
+    return logf + (f32 ? gradient_log_floats(P.rb, P.fb) : 0);
+}
+
 // One item of the fused gradient: stage the item's control points, walk its columns and write
 // every voxel's NMI gradient (zero where masked or NaN). Called by every thread of the block.
-template <bool kF32, bool kDiag, int kFetch>
-__device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSmem& S, const float *logf,
+template <bool kF32, bool kXs, bool kDiag, int kFetch>
+__device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSmem& S, const float *logf, float *X,
                                               const GradientTables& T, int item, const float *__restrict__ ref,
                                               const float *__restrict__ flo, const int32_t *__restrict__ mask,
                                               const float *__restrict__ cpp, float *__restrict__ vgrad) {
@@ -733,12 +740,13 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
     stage_item(P, cpp, item, S.cp, S.zb, S.zk, S.zid, I);
     Column C;
     column_init(P, I, S.cp, C);
+    if (kXs) build_xrows(P, C, S.cp, X);
     const int nzi = I.z1 - I.z0;
     const int zstride = P.nx * P.ny;
     int idx = (I.z0 * P.ny + C.y) * P.nx + C.x;
     for (int zi = 0; zi < nzi; ++zi, idx += zstride) {
         float pos[3];
-        column_position(P, C, S.zb, S.zk, S.zid, zi, pos);
+        column_position<kXs>(P, C, S.zb, S.zk, S.zid, zi, pos, X);
         if (!C.inside) continue;
         float out[3] = { 0.f, 0.f, 0.f };
         if (mask == nullptr || __ldg(&mask[idx]) > -1) {
@@ -765,8 +773,11 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
     }
 }
 
-template <bool kF32, bool kDiag, int kFetch>
-__global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 6 : 4)
+// kXs: the x-contracted node rows as in the objective (a node plane then costs a thread 12 shared
+// loads instead of 48). Eight rows share them and the log table: three blocks of 8 warps per SM
+// (two with the FP64 window or a 128-bin table).
+template <bool kF32, bool kXs, bool kDiag, int kFetch>
+__global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 3 : 2)
 k_gradient(WalkParams P, const float *__restrict__ ref, const float *__restrict__ flo,
            const int32_t *__restrict__ mask, const float *__restrict__ cpp,
            const double *logt0, const nrb_objective *last0, const double *logt1, const nrb_objective *last1,
@@ -776,8 +787,9 @@ k_gradient(WalkParams P, const float *__restrict__ ref, const float *__restrict_
     const GradientTables T = gradient_tables(logt0, last0, logt1, last1, sel && sel->best_buf == 1, weight);
     float *logf = reinterpret_cast<float *>(S.tail);
     if (kF32) stage_log_table(P, T.logt, logf);
+    float *X = gradient_xrows(P, logf, kF32);
     for (int item = blockIdx.x; item < P.nitems; item += gridDim.x)
-        gradient_item<kF32, kDiag, kFetch>(P, S, logf, T, item, ref, flo, mask, cpp, vgrad);
+        gradient_item<kF32, kXs, kDiag, kFetch>(P, S, logf, X, T, item, ref, flo, mask, cpp, vgrad);
 }
 
 // standalone deformation field (Compute::GetDeformationField) with the same arithmetic, in the
@@ -1423,8 +1435,8 @@ k_b_objective(const __grid_constant__ BatchObjTable T, const OptState *__restric
 
 // The fused voxel gradient of every pair in GRAD, at best, with the NMI tables of its best
 // position (the plain k_gradient's work per item).
-template <bool kF32, bool kDiag, int kFetch>
-__global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 6 : 4)
+template <bool kF32, bool kXs, bool kDiag, int kFetch>
+__global__ void __launch_bounds__(32 * TY_GRADIENT, kF32 ? 3 : 2)
 k_b_gradient(const __grid_constant__ BatchGradTable T, const OptState *__restrict__ states, int npairs) {
     extern __shared__ float4 sm4[];
     __shared__ BatchList L;
@@ -1444,7 +1456,7 @@ k_b_gradient(const __grid_constant__ BatchGradTable T, const OptState *__restric
         __syncthreads();  // the previous pair's walk is done with the shared tables
         if (kF32) stage_log_table(E.P, N.logt, logf);  // visible after stage_item's first barrier
         for (int j = G.j0[sg]; j < G.j1[sg]; ++j)
-            gradient_item<kF32, kDiag, kFetch>(E.P, S, logf, N, j, E.ref, E.flo, nullptr, E.best, E.vgrad);
+            gradient_item<kF32, kXs, kDiag, kFetch>(E.P, S, logf, gradient_xrows(E.P, logf, kF32), N, j, E.ref, E.flo, nullptr, E.best, E.vgrad);
     }
 }
 
@@ -1600,8 +1612,8 @@ struct ObjectiveKernel {
     }
 };
 struct GradientKernel {
-    template <bool kF32, bool kDiag, bool kNan, bool kTex> auto operator()() const {
-        return k_gradient<kF32, kDiag, fetch_of<kNan, kTex>()>;
+    template <bool kF32, bool kXs, bool kDiag, bool kNan, bool kTex> auto operator()() const {
+        return k_gradient<kF32, kXs, kDiag, fetch_of<kNan, kTex>()>;
     }
 };
 struct BatchObjectiveKernel {
@@ -1610,8 +1622,8 @@ struct BatchObjectiveKernel {
     }
 };
 struct BatchGradientKernel {
-    template <bool kF32, bool kDiag, bool kNan, bool kTex> auto operator()() const {
-        return k_b_gradient<kF32, kDiag, fetch_of<kNan, kTex>()>;
+    template <bool kF32, bool kXs, bool kDiag, bool kNan, bool kTex> auto operator()() const {
+        return k_b_gradient<kF32, kXs, kDiag, fetch_of<kNan, kTex>()>;
     }
 };
 struct ResampleKernel {
@@ -1622,12 +1634,19 @@ struct ResampleKernel {
 static auto pick_objective(bool trial, bool xs, bool diag, int fetch) {
     return with_flags<>(ObjectiveKernel{}, trial, xs, diag, fetch == FETCH_NAN, fetch == FETCH_TEX);
 }
-static auto pick_gradient(bool f32, bool diag, int fetch) {
-    return with_flags<>(GradientKernel{}, f32, diag, fetch == FETCH_NAN, fetch == FETCH_TEX);
+static auto pick_gradient(bool f32, bool xs, bool diag, int fetch) {
+    return with_flags<>(GradientKernel{}, f32, xs, diag, fetch == FETCH_NAN, fetch == FETCH_TEX);
+}
+
+// x-contracted rows for the gradient when they leave as many blocks per SM as there were
+static bool gradient_rows_fit(size_t base, size_t rows, bool f32, int threads) {
+    const size_t sm = 227 * 1024, fixed = 1024, most = (size_t)(f32 ? 3 : 2) * 32 * TY_GRADIENT / threads;
+    auto blocks = [&](size_t b) { return std::min(most, sm / (b + fixed)); };
+    return base + rows <= 200 * 1024 && blocks(base + rows) == blocks(base);
 }
 
 long long objective_slots(size_t smem) { return blocks_resident(k_objective<true, true, true, FETCH_TEX>, 32 * TY_OBJECTIVE, smem); }
-long long gradient_slots(size_t smem) { return blocks_resident(k_gradient<true, true, FETCH_TEX>, 32 * TY_GRADIENT, smem); }
+long long gradient_slots(size_t smem) { return blocks_resident(k_gradient<true, true, true, FETCH_TEX>, 32 * TY_GRADIENT, smem); }
 long long field_slots(size_t smem) { return blocks_resident(k_deformation<true>, 32 * TY_FIELD, smem); }
 
 template <int kOrder>
@@ -1673,10 +1692,13 @@ nrb_status launch_fused_gradient(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geom
     // 128 bins: 70 KB); larger tables use the FP64 window on the global table
     const size_t log_bytes = (size_t)nmi->total * sizeof(float);
     P.log_in_smem = log_bytes <= 96 * 1024;
-    const size_t smem = walk_smem_bytes(ws->walk_grad) + (P.log_in_smem ? log_bytes : 0);
     const int threads = 32 * ws->walk_grad.ty;
+    const size_t base = walk_smem_bytes(ws->walk_grad) + (P.log_in_smem ? (size_t)gradient_log_floats(nmi->rb, nmi->fb) * 4 : 0);
+    const size_t rows = (size_t)3 * P.sc * P.sb * 32 * 4;
+    P.xs = gradient_rows_fit(base, rows, P.log_in_smem, threads);
+    const size_t smem = base + (P.xs ? rows : 0);
     int grid = 0;
-    auto kernel = pick_gradient(P.log_in_smem, P.flo_diag, fetch_mode(P.fv, P.pad));
+    auto kernel = pick_gradient(P.log_in_smem, P.xs, P.flo_diag, fetch_mode(P.fv, P.pad));
     NRB_TRY(persistent_grid(kernel, threads, smem, P.nitems, grid, ws->walk_grad.resident));
     // algorithmic bytes: reference + floating (+ mask) read, voxel gradient written, grid once
     const double nv = (double)P.nx * P.ny * P.nz;
@@ -1917,7 +1939,7 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
     L.npairs = (int)pairs.size();
     if (L.npairs < 1 || L.npairs > BATCH_MAX_PAIRS)
         return fail(NRB_ERR_INVALID, "batched level: 1 to " + std::to_string(BATCH_MAX_PAIRS) + " pairs");
-    size_t base = 0, xs = 0, gsm = 0;
+    size_t base = 0, xs = 0, gsm = 0, gxs = 0;
     bool diag = true, f32 = true, tex = true, nan = true;
     int rb = pairs[0].rb, fb = pairs[0].fb;
     for (const BatchPair& b : pairs) {
@@ -1928,6 +1950,7 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
         xs = std::max(xs, (size_t)3 * b.wo.sc * b.wo.sb * 32 * 4);
         const size_t cp_g = (size_t)3 * b.wg.sa * b.wg.sb * b.wg.sc;
         gsm = std::max(gsm, (cp_g + 4 + (size_t)walk_table_floats(b.wg.zchunk)) * 4 + 16);
+        gxs = std::max(gxs, (size_t)3 * b.wg.sc * b.wg.sb * 32 * 4);
         diag = diag && b.wo.flo_diag;
         f32 = f32 && b.wg.log_in_smem;
         tex = tex && b.wo.fv.tex != 0;
@@ -1941,7 +1964,9 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
     L.obj_smem = base + (L.obj_xs ? xs : 0);
     L.grad_f32 = f32;
     L.grad_diag = diag;
-    L.grad_smem = gsm + (f32 ? (size_t)(rb * fb + rb + fb) * sizeof(float) : 0);
+    L.grad_smem = gsm + (f32 ? (size_t)gradient_log_floats(rb, fb) * sizeof(float) : 0);
+    L.grad_xs = gradient_rows_fit(L.grad_smem, gxs, f32, 32 * TY_GRADIENT);
+    if (L.grad_xs) L.grad_smem += gxs;
     const int rpc = (fb + FIN_CLUSTER - 1) / FIN_CLUSTER;
     L.fin_smem = (size_t)(2 * rpc + 2) * rb * sizeof(double);
     for (size_t i = 0; i < pairs.size(); ++i) {
@@ -1967,7 +1992,7 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
         g.last1 = b.last1;
     }
     auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
-    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
+    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_xs, L.grad_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
     int per = 0;
     NRB_CUDA(cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ko, 32 * TY_OBJECTIVE, L.obj_smem));
@@ -1992,7 +2017,7 @@ nrb_status launch_batch_objective(const BatchPair *d_pairs, const OptState *stat
 nrb_status launch_batch_gradient(const BatchPair *d_pairs, const OptState *states, const BatchLaunch& L,
                                  cudaStream_t st, double bytes) {
     KernelTimer timer(TK_GRADIENT, bytes, st);
-    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
+    auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_xs, L.grad_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
     kg<<<L.grad_grid, 32 * TY_GRADIENT, L.grad_smem, st>>>(L.grad_table, states, L.npairs);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_gradient");
