@@ -155,13 +155,20 @@ __device__ __forceinline__ double node_tail_cluster(cg::cluster_group& cluster, 
             __syncthreads();
         }
         cluster.sync();  // every partial written
-        if (rank == 0 && tid == 0) {
-            double gg = 0, dgg = 0;
-            for (int i = 0; i < np; ++i) {
-                gg += partials[2 * i];
-                dgg += partials[2 * i + 1];
+        if (rank == 0) {
+            // the partials into shared memory at once, then summed in index order (a thread's chain
+            // of global loads waited on each)
+            static_assert(2 * NRB_RED_BLOCKS <= TAIL_THREADS, "one partial per thread");
+            if (tid < 2 * np) red[tid] = __ldcg(&partials[tid]);
+            __syncthreads();
+            if (tid == 0) {
+                double gg = 0, dgg = 0;
+                for (int i = 0; i < np; ++i) {
+                    gg += red[2 * i];
+                    dgg += red[2 * i + 1];
+                }
+                gam_s = dgg / gg;
             }
-            gam_s = dgg / gg;
         }
         cluster.sync();
         const double gm = *cluster.map_shared_rank(&gam_s, 0);

@@ -121,14 +121,23 @@ __device__ __forceinline__ float identity_pos(const Mat34& M, int k, int x, int 
 
 // reg_spline_approxBendingEnergyGradient3D (reg-lib/cpu/_reg_localTrans_regul.cpp:286-451),
 // first half: the 6 derivative values of component k of node n from zero-padded stencils of the
-// displacements, cross terms doubled. Layout der[(3 * t + k) * nc + node].
+// displacements, cross terms doubled. Layout der[(3 * t + k) * BePad::size + BePad node]: every derivative
+// plane has a ring of zeros around the grid (cleared when the workspace is made and never written),
+// so that the second half reads all 27 neighbours of any node without a test; a zero adds nothing.
+struct BePad {
+    int sy, sz;
+    long long size;
+    __host__ __device__ __forceinline__ BePad(int cx, int cy, int cz)
+        : sy(cx + 2), sz((cx + 2) * (cy + 2)), size((long long)(cx + 2) * (cy + 2) * (cz + 2)) {}
+    __device__ __forceinline__ long long node(int x, int y, int z) const { return (long long)(z + 1) * sz + (y + 1) * sy + x + 1; }
+};
+
 __device__ __forceinline__ void be_node_derivatives_k(int cx, int cy, int cz, const Mat34& M,
                                                       const float *__restrict__ cpp, const BeBasis& B,
                                                       float *__restrict__ der, long long n, int k) {
     const long long nc = (long long)cx * cy * cz;
-    const int x = (int)(n % cx);
-    const int y = (int)((n / cx) % cy);
-    const int z = (int)(n / ((long long)cx * cy));
+    // node indices fit 32 bits (a grid has fewer than 2^31 / 3 nodes)
+    const int i32 = (int)n, row = i32 / cx, x = i32 - row * cx, z = row / cy, y = row - z * cy;
     // row k of the grid matrix picked by selects (a runtime index into the parameter would copy
     // the matrix to local memory)
     float m[4];
@@ -153,10 +162,12 @@ __device__ __forceinline__ void be_node_derivatives_k(int cx, int cy, int cz, co
 #pragma unroll
                 for (int t = 0; t < 6; ++t) d[t] = __fadd_rn(d[t], __fmul_rn(B.v[t][i], v));
             }
+    const BePad pad(cx, cy, cz);
+    float *q = der + k * pad.size + pad.node(x, y, z);
 #pragma unroll
-    for (int t = 0; t < 3; ++t) der[(3 * t + k) * nc + n] = d[t];
+    for (int t = 0; t < 3; ++t) q[3 * t * pad.size] = d[t];
 #pragma unroll
-    for (int t = 3; t < 6; ++t) der[(3 * t + k) * nc + n] = (float)(2.0 * (double)d[t]);
+    for (int t = 3; t < 6; ++t) q[3 * t * pad.size] = (float)(2.0 * (double)d[t]);
 }
 
 // one thread per (node, component): component k = blockIdx.y
@@ -175,23 +186,23 @@ __device__ __forceinline__ void be_node_accumulate_k(int cx, int cy, int cz, con
                                                      const BeBasis& B, float ratio, float *__restrict__ grad,
                                                      long long n, int k) {
     const long long nc = (long long)cx * cy * cz;
-    const int x = (int)(n % cx);
-    const int y = (int)((n / cx) % cy);
-    const int z = (int)(n / ((long long)cx * cy));
+    // node indices fit 32 bits (a grid has fewer than 2^31 / 3 nodes)
+    const int i32 = (int)n, row = i32 / cx, x = i32 - row * cx, z = row / cy, y = row - z * cy;
+    const BePad pad(cx, cy, cz);
+    const float *p = der + k * pad.size + pad.node(x, y, z);
     float g = 0.f;
 #pragma unroll
     for (int c = -1; c < 2; ++c)
 #pragma unroll
-        for (int b = -1; b < 2; ++b)
+        for (int b = -1; b < 2; ++b) {
+            const float *r = p + (c * pad.sz + b * pad.sy);
 #pragma unroll
             for (int e = -1; e < 2; ++e) {
                 const int a = 9 * (c + 1) + 3 * (b + 1) + (e + 1);
-                const int X = x + e, Y = y + b, Z = z + c;
-                if (X < 0 || Y < 0 || Z < 0 || X >= cx || Y >= cy || Z >= cz) continue;
-                const long long j = ((long long)Z * cy + Y) * cx + X;
 #pragma unroll
-                for (int t = 0; t < 6; ++t) g = __fadd_rn(g, __fmul_rn(__ldg(&der[(3 * t + k) * nc + j]), B.v[t][a]));
+                for (int t = 0; t < 6; ++t) g = __fadd_rn(g, __fmul_rn(__ldg(r + 3 * t * pad.size + e), B.v[t][a]));
             }
+        }
     grad[k * nc + n] = __fadd_rn(grad[k * nc + n], __fmul_rn(ratio, g));
 }
 
@@ -226,12 +237,11 @@ __device__ __forceinline__ float conv_at(int s, int n, int R, const float *__res
     return num / den;
 }
 
-// Four consecutive sampled outputs of one line (samples ascend), the taps of each in ascending
-// order; where all four windows lie inside the line they share every weight. kPadded: ld reads 0
-// for the R positions beyond either end (a tap there adds weight * 0 and changes no sum), so every
-// window counts as inside. The sum assumes no NaN (its density is then dens[j], the in-line weights
+// Four consecutive sampled outputs of one line, the taps of each in ascending order and every weight
+// read once for the four. ld reads 0 for the R positions beyond either end (a tap there adds
+// weight * 0 and changes no sum). The sum assumes no NaN (its density is then dens[j], the in-line weights
 // summed in the same order); a NaN shows in it, and that output is taken again with conv_at.
-template <bool kPadded, typename Load>
+template <typename Load>
 __device__ __forceinline__ void conv_outputs4(int n, int R, const float *w, const float *dens,
                                               const int *__restrict__ samples, int ns, int j0, Load ld, float out[4]) {
     const int last = min(4, ns - j0) - 1;
@@ -239,30 +249,21 @@ __device__ __forceinline__ void conv_outputs4(int n, int R, const float *w, cons
 #pragma unroll
     for (int u = 0; u < 4; ++u) s[u] = __ldg(&samples[j0 + min(u, last)]);
     float num[4] = { 0.f, 0.f, 0.f, 0.f };
-    if (kPadded || (s[0] >= R && s[3] + R < n)) {
-        const int taps = 2 * R + 1;
-        int t = 0;
-        for (; t + 4 <= taps; t += 4) {
-            const float4 q = *reinterpret_cast<const float4 *>(w + t);
-            const float wt[4] = { q.x, q.y, q.z, q.w };
+    const int taps = 2 * R + 1;
+    int t = 0;
+    for (; t + 4 <= taps; t += 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(w + t);
+        const float wt[4] = { q.x, q.y, q.z, q.w };
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < 4; ++e)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) num[u] = fmaf(wt[e], ld(s[u] - R + t + e), num[u]);
-        }
+            for (int u = 0; u < 4; ++u) num[u] = fmaf(wt[e], ld(s[u] - R + t + e), num[u]);
+    }
 #pragma unroll 1
-        for (; t < taps; ++t) {
-            const float wt = w[t];
+    for (; t < taps; ++t) {
+        const float wt = w[t];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) num[u] = fmaf(wt, ld(s[u] - R + t), num[u]);
-        }
-    } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k0 = max(0, s[u] - R), k1 = min(n - 1, s[u] + R);
-#pragma unroll 4
-            for (int k = k0; k <= k1; ++k) num[u] = fmaf(w[k - s[u] + R], ld(k), num[u]);
-        }
+        for (int u = 0; u < 4; ++u) num[u] = fmaf(wt, ld(s[u] - R + t), num[u]);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) out[u] = num[u] / dens[j0 + min(u, last)];
@@ -348,7 +349,7 @@ __device__ __forceinline__ void conv_x_unit(int nx, int ny, int nz, const float 
     for (int q = warp * kSub + lane / kRows; 4 * q < ns; q += kWarps * kSub) {
         if (lrow >= nr) continue;
         float v[4];
-        conv_outputs4<true>(nx, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * kStride]; }, v);
+        conv_outputs4(nx, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * kStride]; }, v);
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (4 * q + u < ns) res[lrow * rstride + 4 * q + u] = v[u];
@@ -411,7 +412,7 @@ __device__ __forceinline__ void conv_y_unit(int ny, int inner, const float *__re
         const int q = e / wd, ii = e - q * wd;
         const float *col = body + ii;
         float v[4];
-        conv_outputs4<true>(ny, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * wd]; }, v);
+        conv_outputs4(ny, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * wd]; }, v);
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (4 * q + u < ns) dst[(long long)(4 * q + u) * inner + ii] = v[u];
@@ -427,35 +428,37 @@ k_conv_y(int ny, int inner, const float *__restrict__ in, const int *__restrict_
     conv_y_unit(ny, inner, in, samples, ns, R, out, blockIdx.x, conv_sm, dens, conv_sm + conv_weight_floats(R, ns));
 }
 
-// Pass along z of a [3][nz][inner] array, four outputs of a column per thread, element = (component,
-// group of four, column): a column's reads are coalesced over the columns and shared by its groups
-// in L1. The array is small by now (y and x are sampled).
-__host__ __device__ inline long long conv_z_elements(int ns, int inner) { return 3LL * ((ns + 3) / 4) * inner; }
+// Pass along z of a [3][nz][inner] array, one output per thread, element = (component, sample,
+// column): reads are coalesced over the columns and shared by a column's samples in L1. The array is
+// small by now (y and x are sampled): four outputs per thread left too few warps and staged weights
+// cost more than they saved (14 and 12 us against 9).
+__host__ __device__ inline long long conv_z_elements(int ns, int inner) { return 3LL * ns * inner; }
 
 __device__ __forceinline__ void conv_z_element(int nz, int inner, const float *__restrict__ in,
-                                               const int *__restrict__ samples, int ns, int R, float *__restrict__ out,
-                                               long long e, const float *w, const float *dens) {
-    const int groups = (ns + 3) / 4;
-    const int ii = (int)(e % inner);
-    const long long rest = e / inner;
-    const int q = (int)(rest % groups), c = (int)(rest / groups);
+                                               const int *__restrict__ samples, int ns, const float *__restrict__ K, int R,
+                                               float *__restrict__ out, long long e) {
+    const int i32 = (int)e, rest = i32 / inner, ii = i32 - rest * inner;  // < 3 x voxels, below 2^31
+    const int c = rest / ns, s = __ldg(&samples[rest - c * ns]);
     const float *col = in + (long long)c * nz * inner + ii;
-    float v[4];
-    conv_outputs4<false>(nz, R, w, dens, samples, ns, 4 * q, [&](int k) { return __ldg(col + (long long)k * inner); }, v);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-        if (4 * q + u < ns) out[((long long)c * ns + 4 * q + u) * inner + ii] = v[u];
+    const int k0 = max(0, s - R), k1 = min(nz - 1, s + R);
+    const float *p = col + (long long)k0 * inner, *q = K + (k0 - s + R);
+    float num = 0.f, den = 0.f;
+#pragma unroll 8
+    for (int k = k0; k <= k1; ++k, p += inner, ++q) {
+        const float w = __ldg(q);
+        num = fmaf(w, __ldg(p), num);
+        den += w;
+    }
+    float v = num / den;
+    if (num != num) v = conv_at(s, nz, R, K, [&](int k) { return __ldg(col + (long long)k * inner); });
+    out[e] = v;
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 k_conv_z(int nz, int inner, const float *__restrict__ in, const int *__restrict__ samples, int ns,
          const float *__restrict__ K, int R, float *__restrict__ out) {
-    extern __shared__ __align__(16) float conv_sm[];
-    float *dens;
-    conv_weights(nz, R, K, samples, ns, conv_sm, dens);
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < conv_z_elements(ns, inner);
-         e += (long long)gridDim.x * blockDim.x)
-        conv_z_element(nz, inner, in, samples, ns, R, out, e, conv_sm, dens);
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e < conv_z_elements(ns, inner)) conv_z_element(nz, inner, in, samples, ns, K, R, out, e);
 }
 
 // reg_voxelCentricToNodeCentric (reg-lib/cpu/_reg_localTrans.cpp:1616-1683): trilinear sample
@@ -604,7 +607,7 @@ __global__ void k_b_be_accumulate(const BatchPair *__restrict__ pairs, const Opt
 }
 
 // x, y and z passes of the node convolution: work unit = one block of the plain k_conv_x and
-// k_conv_y, one element of k_conv_z. A block fills its weights when it comes to a pair's first unit.
+// k_conv_y; element-wise along z. A block fills its weights when it comes to a pair's first unit.
 template <int kRows>
 __global__ void __launch_bounds__(CONV_X_THREADS)
 k_b_conv_x(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
@@ -656,31 +659,18 @@ k_b_conv_y(const BatchPair *__restrict__ pairs, const OptState *__restrict__ sta
     }
 }
 
-__global__ void __launch_bounds__(128)
-k_b_conv_z(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
-    extern __shared__ __align__(16) float conv_sm[];
+__global__ void k_b_conv_z(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
     __shared__ BatchList L;
     batch_list_build(states, npairs, 1u << PH_GRAD,
                      [&](int q, int& u, int& w) {
                          const BatchPair& b = pairs[q];
-                         u = (int)((conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]) + 127) / 128);
+                         u = (int)conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]);
                          w = 1;
                      }, L);
-    int k = 0, have = -1;
-    float *dens = nullptr;
-    for (long long u = blockIdx.x; u < L.total; u += gridDim.x) {
-        while (L.pref[k + 1] <= u) ++k;
-        const BatchPair& P = pairs[L.pair[k]];
-        const int inner = P.ns[1] * P.ns[0];
-        if (have != k) {
-            __syncthreads();  // the previous pair's weights are done with
-            conv_weights(P.rdim[2], P.radius[2], P.kernel[2], P.samples[2], P.ns[2], conv_sm, dens);
-            have = k;
-        }
-        const long long e = (u - L.pref[k]) * 128 + threadIdx.x;
-        if (e < conv_z_elements(P.ns[2], inner))
-            conv_z_element(P.rdim[2], inner, P.conv2, P.samples[2], P.ns[2], P.radius[2], P.conv1, e, conv_sm, dens);
-    }
+    batch_elements(L, [&](int p, long long e) {
+        const BatchPair& P = pairs[p];
+        conv_z_element(P.rdim[2], P.ns[1] * P.ns[0], P.conv2, P.samples[2], P.ns[2], P.kernel[2], P.radius[2], P.conv1, e);
+    });
 }
 
 // node sampling, reorientation and weighting (overwrites the node gradient)
@@ -1100,11 +1090,18 @@ k_maxlen(long long nnode, const float *__restrict__ g, float *__restrict__ pmax)
     if (threadIdx.x == 0) pmax[blockIdx.x] = s[0];
 }
 
-__global__ void k_maxlen_finish(const float *__restrict__ pmax, int np, nrb_objective *__restrict__ obj,
-                                double *__restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        float mx = 0.f;
-        for (int i = 0; i < np; ++i) mx = fmaxf(mx, pmax[i]);
+// one thread per partial (a max is exact in any order; a single thread's chain of loads took 9 us)
+__global__ void __launch_bounds__(NRB_RED_BLOCKS)
+k_maxlen_finish(const float *__restrict__ pmax, int np, nrb_objective *__restrict__ obj, double *__restrict__ out) {
+    __shared__ float s[NRB_RED_BLOCKS / 32];
+    float mx = threadIdx.x < np ? pmax[threadIdx.x] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 0; w < NRB_RED_BLOCKS / 32; ++w) mx = fmaxf(mx, s[w]);
         if (obj) obj->max_grad_len = (double)mx;
         if (out) *out = (double)mx;
     }
@@ -1527,18 +1524,21 @@ static nrb_status workspace_alloc(nrb_workspace *ws) {
     const long long c2 = 3LL * nz * ws->ax[1].nsamples * ws->ax[0].nsamples;
     const long long c3 = 3LL * ws->ax[2].nsamples * ws->ax[1].nsamples * ws->ax[0].nsamples;
     (void)nx;
-    const long long nc = nvox(g->cpp_dim);
     const size_t sz1 = (size_t)std::max(c1, c3) * 4, sz2 = (size_t)c2 * 4;
+    const size_t be_bytes = (size_t)18 * BePad(g->cpp_dim[0], g->cpp_dim[1], g->cpp_dim[2]).size * 4;
     cudaStream_t st = ws->st;
     if (dev_alloc(&ws->conv1, sz1, st) != cudaSuccess || dev_alloc(&ws->conv2, sz2, st) != cudaSuccess ||
-        dev_alloc(&ws->be_deriv, (size_t)18 * nc * 4, st) != cudaSuccess ||
+        dev_alloc(&ws->be_deriv, be_bytes, st) != cudaSuccess ||
         dev_alloc(&ws->red, 2 * NRB_RED_BLOCKS * sizeof(double), st) != cudaSuccess ||
         dev_alloc(&ws->be_partials, NRB_RED_BLOCKS * sizeof(double), st) != cudaSuccess ||
         dev_alloc(&ws->fred, 2 * NRB_RED_BLOCKS * sizeof(float), st) != cudaSuccess) {
         cudaGetLastError();
         return fail(NRB_ERR_OOM, "workspace allocation failed");
     }
-    bytes += sz1 + sz2 + (size_t)18 * nc * 4 + 3 * NRB_RED_BLOCKS * sizeof(double) + 2 * NRB_RED_BLOCKS * 4;
+    // the ring of zeros around every derivative plane
+    NRB_CUDA(cudaMemsetAsync(ws->be_deriv, 0, be_bytes, st));
+    if (!st) NRB_CUDA(cudaStreamSynchronize(st));  // the workspace may be used on any stream at once
+    bytes += sz1 + sz2 + be_bytes + 3 * NRB_RED_BLOCKS * sizeof(double) + 2 * NRB_RED_BLOCKS * 4;
     ws->bytes = bytes;
     NRB_CUDA(cudaStreamCreateWithFlags(&ws->side, cudaStreamNonBlocking));
     NRB_CUDA(cudaEventCreateWithFlags(&ws->ev_fork, cudaEventDisableTiming));
@@ -1657,10 +1657,8 @@ nrb_status launch_convolve_to_nodes(nrb_workspace *ws, const nrb_geometry *g, co
                                                                               K[1], R[1], ws->conv2);
     NRB_LAUNCHED("k_conv_y");
     // z pass: [3][nz][nsy * nsx] -> [3][nsz][nsy * nsx] (reuses conv1)
-    const size_t zsm = 4 * (size_t)conv_weight_floats(R[2], nsz);
-    NRB_TRY(conv_smem(k_conv_z, zsm));
-    k_conv_z<<<grid_for(conv_z_elements(nsz, nsy * nsx), 128), 128, zsm, st>>>(nz, nsy * nsx, ws->conv2, ws->d_samples[2],
-                                                                              nsz, K[2], R[2], ws->conv1);
+    k_conv_z<<<(unsigned)((conv_z_elements(nsz, nsy * nsx) + 255) / 256), 256, 0, st>>>(
+        nz, nsy * nsx, ws->conv2, ws->d_samples[2], nsz, K[2], R[2], ws->conv1);
     NRB_LAUNCHED("k_conv_z");
     // node sampling, reorientation (floating ijk) and weighting
     float w = weight;
@@ -1964,17 +1962,16 @@ nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const Batch
     }
     NRB_TRY(gradient(d, states, st, gradient_arg));
     // shared memory and rows per block for the largest pair
-    size_t xsm = 0, ysm = 0, zsm = 0;
+    size_t xsm = 0, ysm = 0;
     long long xb = 0, yb = 0, zb = 0;
     int rows = 32;
     for (const BatchPair& b : hp) rows = std::min(rows, conv_x_rows(b.rdim[0], b.radius[0], b.ns[0]));
     for (const BatchPair& b : hp) {
         xsm = std::max(xsm, conv_x_bytes(rows, b.rdim[0], b.radius[0], b.ns[0]));
         ysm = std::max(ysm, conv_y_bytes(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]));
-        zsm = std::max(zsm, 4 * (size_t)conv_weight_floats(b.radius[2], b.ns[2]));
         xb += conv_x_units(rows, b.rdim[1], b.rdim[2]);
         yb += conv_y_units(b.rdim[1], b.rdim[2], b.ns[0], b.radius[1]);
-        zb += (conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]) + 127) / 128;
+        zb += conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]);
     }
     auto launch = [&](auto kernel, long long units, int threads, size_t smem) -> nrb_status {
         int per = 0;
@@ -1991,7 +1988,8 @@ nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const Batch
     NRB_LAUNCHED("k_b_conv_x");
     NRB_TRY(launch(k_b_conv_y, yb, CONV_Y_THREADS, ysm));
     NRB_LAUNCHED("k_b_conv_y");
-    NRB_TRY(launch(k_b_conv_z, zb, 128, zsm));
+    k_b_conv_z<<<grid_for(std::max(1LL, zb), 256), 256, 0, st>>>(d, states, np);
+    NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_conv_z");
     const int gn = batch_grid(hp, [](const BatchPair& b) { return b.nnode; }, 256, 16);
     k_b_nodes<<<gn, 256, 0, st>>>(d, states, np);
@@ -2057,7 +2055,7 @@ extern "C" nrb_status nrb_get_maximal_length(const float *node_grad, int64_t nno
     NRB_CUDA(tmp_alloc(&dm, sizeof(double), st));
     k_maxlen<<<np, NRB_RED_THREADS, 0, st>>>(nnode, node_grad, pm);
     NRB_LAUNCHED("k_maxlen");
-    k_maxlen_finish<<<1, 32, 0, st>>>(pm, np, obj, dm);
+    k_maxlen_finish<<<1, NRB_RED_BLOCKS, 0, st>>>(pm, np, obj, dm);
     NRB_LAUNCHED("k_maxlen_finish");
     if (max_host) {
         NRB_CUDA(cudaMemcpyAsync(max_host, dm, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -2085,7 +2083,7 @@ nrb_status max_and_normalise(nrb_workspace *ws, float *grad, int64_t nnode, nrb_
     const int np = (int)std::max<long long>(1, std::min<long long>((nnode + NRB_RED_THREADS - 1) / NRB_RED_THREADS, NRB_RED_BLOCKS));
     k_maxlen<<<np, NRB_RED_THREADS, 0, st>>>(nnode, grad, ws->fred);
     NRB_LAUNCHED("k_maxlen");
-    k_maxlen_finish<<<1, 32, 0, st>>>(ws->fred, np, obj, nullptr);
+    k_maxlen_finish<<<1, NRB_RED_BLOCKS, 0, st>>>(ws->fred, np, obj, nullptr);
     NRB_LAUNCHED("k_maxlen_finish");
     k_normalise<<<grid_for(3 * nnode, 256), 256, 0, st>>>(3 * nnode, grad, obj, -1.0);
     NRB_LAUNCHED("k_normalise");
