@@ -1826,44 +1826,63 @@ private:
     float *fw(DevBuf& b) { return b.p; }
     float *bw(DevBuf& b) { return b.p + 3 * nc_; }
 
-    nrb_status Fields(int64_t nvox_max) {
-        const int64_t need = (int64_t)steps_ * velocity_field_stride(nvox_max);
-        if (need > fields_n_) {
-            NRB_TRY(fields_.alloc(need, st_));
-            fields_n_ = need;
-        }
+    // The two directions share nothing but the grids and the squaring number, and at most sizes a
+    // kernel of one leaves most of the device idle: the backward direction runs on a stream of its
+    // own between a fork and a join, in the order and with the arithmetic of one stream.
+    nrb_status Fork() {
+        NRB_CUDA(cudaEventRecord(ev_fork_, st_));
+        NRB_CUDA(cudaStreamWaitEvent(side_, ev_fork_, 0));
+        return NRB_OK;
+    }
+    nrb_status Join() {
+        NRB_CUDA(cudaEventRecord(ev_join_, side_));
+        NRB_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));
+        return NRB_OK;
+    }
+    // intermediate fields of both gradient exponentiations
+    nrb_status Fields(int64_t nref, int64_t nflo) {
+        const int64_t need[2] = { (int64_t)steps_ * velocity_field_stride(nref), (int64_t)steps_ * velocity_field_stride(nflo) };
+        DevBuf *const buf[2] = { &fields_, &fields_b_ };
+        for (int i = 0; i < 2; ++i)
+            if (need[i] > fields_n_[i]) {
+                NRB_TRY(buf[i]->alloc(need[i], st_));
+                fields_n_[i] = need[i];
+            }
         return NRB_OK;
     }
     // reg_f3d2::GetDeformationField + WarpFloatingImage (_reg_f3d2.cpp:144-181): the forward
     // field (squaring number updated when the optimiser runs), the backward one with the same
-    // number, both images warped (trilinear)
+    // number, both images warped (trilinear). Forked: the backward half is on the side stream.
     nrb_status Warp(bool update) {
         NRB_TRY(velocity_to_deformation(&gfw_, fw(cur_), update, &steps_, def_fw_.p, nullptr, scr_r_.p, mm_, st_));
-        NRB_TRY(velocity_to_deformation(&gbw_, bw(cur_), false, &steps_, def_bw_.p, nullptr, scr_f_.p, mm_, st_));
+        NRB_TRY(velocity_to_deformation(&gbw_, bw(cur_), false, &steps_, def_bw_.p, nullptr, scr_f_.p, mm_, side_));
         KernelTimer kt(TK_F2_WARP, 0.0, st_);
         NRB_TRY(nrb_resample_image(&gfw_, flo_.p, def_fw_.p, nullptr, pad_, war_fw_.p, st_));
-        NRB_TRY(nrb_resample_image(&gbw_, ref_.p, def_bw_.p, nullptr, pad_, war_bw_.p, st_));
+        NRB_TRY(nrb_resample_image(&gbw_, ref_.p, def_bw_.p, nullptr, pad_, war_bw_.p, side_));
         return NRB_OK;
     }
-    // both NMI values into the device scalars (obj_[2], obj_[3]); no host read
+    // both NMI values into the device scalars (obj_[2], obj_[3]); no host read. Forked.
     nrb_status Similarity() {
         KernelTimer kt(TK_F2_NMI, 0.0, st_);
         NRB_TRY(nrb_nmi_value(nmi_fw_.h, &gfw_, ref_.p, war_fw_.p, nullptr, obj_ + 2, nullptr, st_));
-        NRB_TRY(nrb_nmi_value(nmi_bw_.h, &gbw_, flo_.p, war_bw_.p, nullptr, obj_ + 3, nullptr, st_));
+        NRB_TRY(nrb_nmi_value(nmi_bw_.h, &gbw_, flo_.p, war_bw_.p, nullptr, obj_ + 3, nullptr, side_));
         return NRB_OK;
     }
     // reg_f3d2::GetObjectiveFunctionValue (_reg_f3d2.cpp:465-485): both energies and both NMI
     // values land in device scalars and come back in one read
     nrb_status GetObjectiveFunctionValue(bool update, double& value) {
+        NRB_TRY(Fork());
         if (be_w_ > 0) {
-            KernelTimer kt(TK_F2_BE, 0.0, st_);
-            NRB_TRY(nrb_approx_bending_energy(ws_fw_.h, &gfw_, fw(cur_), obj_, nullptr, st_));
-            NRB_TRY(nrb_approx_bending_energy(ws_bw_.h, &gbw_, bw(cur_), obj_ + 1, nullptr, st_));
+            // both energies on the side stream, beside the forward flow whose extrema the host waits for
+            KernelTimer kt(TK_F2_BE, 0.0, side_);
+            NRB_TRY(nrb_approx_bending_energy(ws_fw_.h, &gfw_, fw(cur_), obj_, nullptr, side_));
+            NRB_TRY(nrb_approx_bending_energy(ws_bw_.h, &gbw_, bw(cur_), obj_ + 1, nullptr, side_));
         }
         if (sim_w_ > 0) {
             NRB_TRY(Warp(update));
             NRB_TRY(Similarity());
         }
+        NRB_TRY(Join());
         NRB_CUDA(cudaMemcpyAsync(obj_h_, obj_, 4 * sizeof(nrb_objective), cudaMemcpyDeviceToHost, st_));
         NRB_CUDA(cudaStreamSynchronize(st_));
         const double be_f = be_w_ > 0 ? obj_h_[0].be : 0.0, be_b = be_w_ > 0 ? obj_h_[1].be : 0.0;
@@ -1880,6 +1899,8 @@ private:
     // (:244-305), ExponentiateGradient (:637-650) and NormaliseGradient (:369-391)
     nrb_status GetObjectiveFunctionGradient() {
         const int64_t nr = nvox(gfw_.ref_dim), nf = nvox(gbw_.ref_dim);
+        if (sim_w_ > 0) NRB_TRY(Fields(nr, nf));
+        NRB_TRY(Fork());
         if (sim_w_ > 0) {
             // the fields and warped images at the best position: those of the accepted trial when
             // it recomputed the squaring number (the same flow gives the same number, so they are
@@ -1898,17 +1919,16 @@ private:
             {
                 KernelTimer kt(TK_F2_VOXEL_GRADIENT, 0.0, st_);
                 NRB_CUDA(cudaMemsetAsync(vg_fw_.p, 0, 3 * nr * sizeof(float), st_));
-                NRB_CUDA(cudaMemsetAsync(vg_bw_.p, 0, 3 * nf * sizeof(float), st_));
+                NRB_CUDA(cudaMemsetAsync(vg_bw_.p, 0, 3 * nf * sizeof(float), side_));
                 NRB_TRY(nrb_get_image_gradient(&gfw_, flo_.p, def_fw_.p, nullptr, pad_, wg_fw_.p, st_));
-                NRB_TRY(nrb_get_image_gradient(&gbw_, ref_.p, def_bw_.p, nullptr, pad_, wg_bw_.p, st_));
+                NRB_TRY(nrb_get_image_gradient(&gbw_, ref_.p, def_bw_.p, nullptr, pad_, wg_bw_.p, side_));
                 // the FP64 window: the trajectory follows reg_f3d2's
                 NRB_TRY(nmi_voxel_gradient(nmi_fw_.h, &gfw_, ref_.p, war_fw_.p, wg_fw_.p, nullptr, 1.0, vg_fw_.p, st_,
                                            true));
-                NRB_TRY(nmi_voxel_gradient(nmi_bw_.h, &gbw_, flo_.p, war_bw_.p, wg_bw_.p, nullptr, 1.0, vg_bw_.p, st_,
+                NRB_TRY(nmi_voxel_gradient(nmi_bw_.h, &gbw_, flo_.p, war_bw_.p, wg_bw_.p, nullptr, 1.0, vg_bw_.p, side_,
                                            true));
             }
             // forward gradient along the backward transformation on the reference grid, and back
-            NRB_TRY(Fields(std::max(nr, nf)));
             nrb_geometry gx = gfw_;
             for (int i = 0; i < 3; ++i) gx.cpp_dim[i] = gbw_.cpp_dim[i], gx.cpp_pixdim[i] = gbw_.cpp_pixdim[i];
             memcpy(gx.cpp_xyz, gbw_.cpp_xyz, sizeof(gx.cpp_xyz));
@@ -1918,19 +1938,21 @@ private:
             for (int i = 0; i < 3; ++i) gx.cpp_dim[i] = gfw_.cpp_dim[i], gx.cpp_pixdim[i] = gfw_.cpp_pixdim[i];
             memcpy(gx.cpp_xyz, gfw_.cpp_xyz, sizeof(gx.cpp_xyz));
             memcpy(gx.cpp_ijk, gfw_.cpp_ijk, sizeof(gx.cpp_ijk));
-            NRB_TRY(exponentiate_gradient(&gx, fw(cur_), steps_, vg_bw_.p, fields_.p, scr_f_.p, mm_, st_));
+            NRB_TRY(exponentiate_gradient(&gx, fw(cur_), steps_, vg_bw_.p, fields_b_.p, scr_f_.p, mm_, side_));
             KernelTimer kt(TK_F2_NODES, 0.0, st_);
             NRB_TRY(nrb_convolve_voxel_based_gradient(ws_fw_.h, &gfw_, vg_fw_.p, sim_w_, fw(grad_), st_));
-            NRB_TRY(nrb_convolve_voxel_based_gradient(ws_bw_.h, &gbw_, vg_bw_.p, sim_w_, bw(grad_), st_));
+            NRB_TRY(nrb_convolve_voxel_based_gradient(ws_bw_.h, &gbw_, vg_bw_.p, sim_w_, bw(grad_), side_));
         } else {
-            NRB_CUDA(cudaMemsetAsync(grad_.p, 0, 6 * nc_ * sizeof(float), st_));
+            NRB_CUDA(cudaMemsetAsync(fw(grad_), 0, 3 * nc_ * sizeof(float), st_));
+            NRB_CUDA(cudaMemsetAsync(bw(grad_), 0, 3 * nc_ * sizeof(float), side_));
         }
         ++it_;
         ++n_grad_;
         if (be_w_ > 0) {
             NRB_TRY(nrb_approx_bending_energy_gradient(ws_fw_.h, &gfw_, fw(cur_), be_w_, fw(grad_), st_));
-            NRB_TRY(nrb_approx_bending_energy_gradient(ws_bw_.h, &gbw_, bw(cur_), be_w_, bw(grad_), st_));
+            NRB_TRY(nrb_approx_bending_energy_gradient(ws_bw_.h, &gbw_, bw(cur_), be_w_, bw(grad_), side_));
         }
+        NRB_TRY(Join());
         double mf = 0, mb = 0;
         NRB_TRY(nrb_get_maximal_length(fw(grad_), nc_, nullptr, &mf, st_));
         NRB_TRY(nrb_get_maximal_length(bw(grad_), nc_, nullptr, &mb, st_));
@@ -2010,12 +2032,15 @@ private:
     int64_t nc_ = 0;
     int steps_ = 6;               // squaring number (the grids' intent_p2)
     DevBuf ref_, flo_, cur_, best_, grad_, g1_, g2_;  // dof arrays: [forward | backward]
-    DevBuf def_fw_, def_bw_, war_fw_, war_bw_, wg_fw_, wg_bw_, vg_fw_, vg_bw_, scr_r_, scr_f_, fields_;
+    DevBuf def_fw_, def_bw_, war_fw_, war_bw_, wg_fw_, wg_bw_, vg_fw_, vg_bw_, scr_r_, scr_f_, fields_,
+        fields_b_;
     // the deformation fields and warped images of the best position, when best_fields_
     DevBuf bdef_fw_, bdef_bw_, bwar_fw_, bwar_bw_;
     bool best_fields_ = false;
     int best_steps_ = 6;
-    int64_t fields_n_ = 0;
+    int64_t fields_n_[2] = { 0, 0 };
+    cudaStream_t side_ = nullptr;  // the backward direction's stream
+    cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
     unsigned *mm_ = nullptr;
     nrb_objective *obj_ = nullptr;    // device: BE forward, BE backward, NMI forward, NMI backward
     nrb_objective *obj_h_ = nullptr;  // pinned host copy
@@ -2032,6 +2057,11 @@ private:
 
 public:
     ~F3d2Registration() {
+        // buffers go back on st_: an evaluation that failed between fork and join may still be running
+        if (side_) cudaStreamSynchronize(side_);
+        if (ev_fork_) cudaEventDestroy(ev_fork_);
+        if (ev_join_) cudaEventDestroy(ev_join_);
+        if (side_) cudaStreamDestroy(side_);
         dev_free(mm_, st_);
         dev_free(obj_, st_);
         if (obj_h_) cudaFreeHost(obj_h_);
@@ -2083,7 +2113,7 @@ nrb_status F3d2Registration::InitLevel(int level, float& max_step) {
     NRB_TRY(wg_bw_.alloc(3 * nfv, st_));
     NRB_TRY(vg_bw_.alloc(3 * nfv, st_));
     NRB_TRY(scr_f_.alloc(3 * nfv, st_));
-    fields_n_ = 0;
+    fields_n_[0] = fields_n_[1] = 0;
     for (WsHandle *w : { &ws_fw_, &ws_bw_ }) {
         nrb_workspace_destroy(w->h);
         w->h = nullptr;
@@ -2123,6 +2153,9 @@ nrb_status F3d2Registration::Run(const float *ref, const float *flo, const Image
     } else {
         sim_w_ = 1 - penalty;
     }
+    NRB_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
+    NRB_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
+    NRB_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
     NRB_CUDA(dev_alloc(&mm_, 2 * sizeof(unsigned), st_));
     NRB_CUDA(dev_alloc(&obj_, 4 * sizeof(nrb_objective), st_));
     NRB_CUDA(cudaMemsetAsync(obj_, 0, 4 * sizeof(nrb_objective), st_));
@@ -2424,10 +2457,11 @@ extern "C" nrb_status nrb_f3d2_register_images(const nrb_image *ref, const nrb_i
     // the buffers a level or an evaluation frees stay in the pool for the next. Per voxel of
     // the larger image at the finest level, both directions: deformation, warped, image and voxel
     // gradients, scratch (52 B), the best position's deformation and warped image (16 B), the
-    // intermediate fields (12 B per squaring, up to 16 kept here), the pyramids, and slack.
+    // intermediate fields of each direction (12 B per squaring, up to 16 kept here), the pyramids,
+    // and slack.
     {
         const int64_t big = std::max(nref, nflo);
-        keep_pool(big * (2 * 52 + 2 * 16 + 16 * 12 + 2 * 8 * 2) + (256LL << 20));
+        keep_pool(big * (2 * 52 + 2 * 16 + 2 * 16 * 12 + 2 * 8 * 2) + (256LL << 20));
     }
     nrb_status s = NRB_OK;
     float *fw = nullptr, *bw = nullptr, *wf = nullptr, *wb = nullptr;
