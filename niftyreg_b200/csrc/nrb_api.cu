@@ -95,6 +95,20 @@ void lib_pool_keep(uint64_t bytes) {
     cudaGetLastError();
 }
 
+// A small device value to host memory, after the stream's work: through pinned memory of the host
+// thread's own (a copy into pageable memory stages through the driver first). Synchronises.
+nrb_status read_back(void *host, const void *dev, size_t bytes, cudaStream_t st) {
+    static thread_local void *pinned = nullptr;
+    constexpr size_t kBytes = 256;
+    if (bytes > kBytes) return fail(NRB_ERR_INVALID, "read_back: value too large");
+    // portable across devices, kept for the thread's lifetime
+    if (!pinned) NRB_CUDA(cudaHostAlloc(&pinned, kBytes, cudaHostAllocPortable));
+    NRB_CUDA(cudaMemcpyAsync(pinned, dev, bytes, cudaMemcpyDeviceToHost, st));
+    NRB_CUDA(cudaStreamSynchronize(st));
+    memcpy(host, pinned, bytes);
+    return NRB_OK;
+}
+
 // ---- per-kernel timing ----------------------------------------------------------------------
 namespace {
 struct Pending {
@@ -320,20 +334,19 @@ nrb_status f3d_objective(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geometry *g,
         return fail(NRB_ERR_UNSUPPORTED, "fused evaluation: the grid must be aligned with the reference");
     int n_be = 0;
     const bool overlap = be_weight > 0 && sim_weight > 0;
+    // the bending energy reads only the grid: it runs beside the voxel pass, which is launched first
+    // (the device starts on it while the host still queues the rest)
+    if (overlap) NRB_CUDA(cudaEventRecord(ws->ev_fork, st));
+    if (sim_weight > 0)
+        NRB_TRY(launch_fused_objective(ws, nmi, g, ref, flo, mask, cpp, padding, st, nullptr, nullptr, flo_margin));
     if (be_weight > 0) {
-        // the bending energy reads only the grid: it runs beside the voxel pass
-        if (overlap) NRB_TRY(fork_side(ws, st));
+        if (overlap) NRB_CUDA(cudaStreamWaitEvent(ws->side, ws->ev_fork, 0));
         NRB_TRY(launch_be_value(ws, g, cpp, overlap ? ws->side : st));
         n_be = be_partial_count(g);
     }
-    if (sim_weight > 0)
-        NRB_TRY(launch_fused_objective(ws, nmi, g, ref, flo, mask, cpp, padding, st, nullptr, nullptr, flo_margin));
     if (overlap) NRB_TRY(join_side(ws, st));
     NRB_TRY(launch_nmi_finalize(nmi, ws->be_partials, n_be, 3 * nvox(g->cpp_dim), sim_weight, be_weight, obj, st));
-    if (obj_host) {
-        NRB_CUDA(cudaMemcpyAsync(obj_host, obj ? obj : nmi->last, sizeof(nrb_objective), cudaMemcpyDeviceToHost, st));
-        NRB_CUDA(cudaStreamSynchronize(st));
-    }
+    if (obj_host) NRB_TRY(read_back(obj_host, obj ? obj : nmi->last, sizeof(nrb_objective), st));
     return NRB_OK;
 }
 
@@ -343,14 +356,15 @@ nrb_status f3d_gradient(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geometry *g, 
     if (ws->general)
         return fail(NRB_ERR_UNSUPPORTED, "fused evaluation: the grid must be aligned with the reference");
     const bool overlap = be_weight > 0 && sim_weight > 0;
-    if (overlap) {
-        // the bending-energy derivatives read only the grid: they run beside the voxel passes
-        NRB_TRY(fork_side(ws, st));
-        NRB_TRY(launch_be_derivatives(ws, g, cpp, ws->side));
-    }
+    if (overlap) NRB_CUDA(cudaEventRecord(ws->ev_fork, st));
     if (sim_weight > 0) {
         // the histogram of the current position feeds the log table of the voxel gradient
         NRB_TRY(launch_fused_objective(ws, nmi, g, ref, flo, mask, cpp, padding, st, nullptr, nullptr, flo_margin));
+        if (overlap) {
+            // the bending-energy derivatives read only the grid: they run beside the voxel passes
+            NRB_CUDA(cudaStreamWaitEvent(ws->side, ws->ev_fork, 0));
+            NRB_TRY(launch_be_derivatives(ws, g, cpp, ws->side));
+        }
         NRB_TRY(launch_nmi_finalize(nmi, nullptr, 0, 3 * nvox(g->cpp_dim), sim_weight, 0.0, nullptr, st));
         NRB_TRY(launch_fused_gradient(ws, nmi, g, ref, flo, mask, cpp, padding, 1.0, vgrad, st, nullptr, flo_margin));
         NRB_TRY(launch_convolve_to_nodes(ws, g, vgrad, (float)sim_weight, node_grad, st));

@@ -101,6 +101,8 @@ inline void dev_free(void *p, cudaStream_t st) {
     else cudaFree(p);
 }
 
+nrb_status read_back(void *host, const void *dev, size_t bytes, cudaStream_t st);
+
 // Optional per-kernel CUDA-event timing (nrb_timing_enable). A KernelTimer brackets one launch
 // with events on its stream and records the algorithmic bytes that launch must move.
 enum TimedKernel {

@@ -1859,10 +1859,7 @@ extern "C" nrb_status nrb_approx_bending_energy(nrb_workspace *ws, const nrb_geo
     }
     k_be_sum<<<1, NRB_RED_THREADS, 0, st>>>(ws->be_partials, be_grid(g), 3.0 * (double)nvox(g->cpp_dim), o);
     NRB_LAUNCHED("k_be_sum");
-    if (be_host) {
-        NRB_CUDA(cudaMemcpyAsync(be_host, &o->be, sizeof(double), cudaMemcpyDeviceToHost, st));
-        NRB_CUDA(cudaStreamSynchronize(st));
-    }
+    if (be_host) NRB_TRY(read_back(be_host, &o->be, sizeof(double), st));
     if (tmp) NRB_CUDA(cudaFreeAsync(tmp, st));
     return NRB_OK;
 }
@@ -2057,10 +2054,7 @@ extern "C" nrb_status nrb_get_maximal_length(const float *node_grad, int64_t nno
     NRB_LAUNCHED("k_maxlen");
     k_maxlen_finish<<<1, NRB_RED_BLOCKS, 0, st>>>(pm, np, obj, dm);
     NRB_LAUNCHED("k_maxlen_finish");
-    if (max_host) {
-        NRB_CUDA(cudaMemcpyAsync(max_host, dm, sizeof(double), cudaMemcpyDeviceToHost, st));
-        NRB_CUDA(cudaStreamSynchronize(st));
-    }
+    if (max_host) NRB_TRY(read_back(max_host, dm, sizeof(double), st));
     NRB_CUDA(cudaFreeAsync(pm, st));
     NRB_CUDA(cudaFreeAsync(dm, st));
     return NRB_OK;

@@ -2247,8 +2247,7 @@ extern "C" nrb_status nrb_nmi_value(nrb_nmi *nmi, const nrb_geometry *g, const f
     NRB_TRY(launch_nmi_finalize(nmi, nullptr, 0, 1, 1.0, 0.0, obj, st));
     if (nmi_host) {
         nrb_objective o;
-        NRB_CUDA(cudaMemcpyAsync(&o, nmi->last, sizeof(o), cudaMemcpyDeviceToHost, st));
-        NRB_CUDA(cudaStreamSynchronize(st));
+        NRB_TRY(read_back(&o, nmi->last, sizeof(o), st));
         *nmi_host = o.nmi;
     }
     return NRB_OK;
