@@ -98,35 +98,35 @@ __device__ __forceinline__ void stage_item(const WalkParams& P, const float *__r
     const int nc = pre_of(I.z1 - 1, P.gsz) + 4 - I.zc0;
     const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
     __syncthreads();  // the previous item's readers are done
-    // one pass: the node planes of one (component, row, column) are independent loads, batched
-    // four at a time so their latencies overlap
+    // one pass over the (component, row) pairs, shared among the warps: the node planes of a pair are
+    // independent loads, batched four at a time so their latencies overlap
     const int gplane = P.cx * P.cy, splane = P.sb * P.sa;
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        for (int jb = ly; jb < nb; jb += P.ty)
-            for (int ia = lx; ia < na; ia += 32) {
-                const int src = c * P.cnv + (I.zc0 * P.cy + I.yb0 + jb) * P.cx + I.xa0 + ia;
-                float *dst = cp + (c * P.sc * P.sb + jb) * P.sa + ia;
-                const float *g = kTrial ? grad : nullptr;
-                // the identity position of this node row (component c varies along axis c only)
-                const double io = (double)P.io[c], is = (double)P.is[c];
-                const double rowid = c == 0 ? io + is * (double)(I.xa0 + ia)
-                                   : c == 1 ? io + is * (double)(I.yb0 + jb) : io + is * (double)I.zc0;
-                const double kstep = c == 2 ? is : 0.0;
-                int kc = 0;
-                for (; kc + 4 <= nc; kc += 4) {
-                    const float v0 = trial_cp(cpp, g, scale, src + kc * gplane);
-                    const float v1 = trial_cp(cpp, g, scale, src + (kc + 1) * gplane);
-                    const float v2 = trial_cp(cpp, g, scale, src + (kc + 2) * gplane);
-                    const float v3 = trial_cp(cpp, g, scale, src + (kc + 3) * gplane);
-                    dst[kc * splane] = (float)((double)v0 - (rowid + kstep * kc));
-                    dst[(kc + 1) * splane] = (float)((double)v1 - (rowid + kstep * (kc + 1)));
-                    dst[(kc + 2) * splane] = (float)((double)v2 - (rowid + kstep * (kc + 2)));
-                    dst[(kc + 3) * splane] = (float)((double)v3 - (rowid + kstep * (kc + 3)));
-                }
-                for (; kc < nc; ++kc)
-                    dst[kc * splane] = (float)((double)trial_cp(cpp, g, scale, src + kc * gplane) - (rowid + kstep * kc));
+    for (int e = ly; e < 3 * nb; e += P.ty) {
+        const int c = e >= 2 * nb ? 2 : (e >= nb ? 1 : 0), jb = e - c * nb;
+        // the identity position of this node row (component c varies along axis c only)
+        const double io = (double)(c == 0 ? P.io[0] : (c == 1 ? P.io[1] : P.io[2]));
+        const double is = (double)(c == 0 ? P.is[0] : (c == 1 ? P.is[1] : P.is[2]));
+        const double kstep = c == 2 ? is : 0.0;
+        for (int ia = lx; ia < na; ia += 32) {
+            const int src = c * P.cnv + (I.zc0 * P.cy + I.yb0 + jb) * P.cx + I.xa0 + ia;
+            float *dst = cp + (c * P.sc * P.sb + jb) * P.sa + ia;
+            const float *g = kTrial ? grad : nullptr;
+            const double rowid = io + is * (double)(c == 0 ? I.xa0 + ia : (c == 1 ? I.yb0 + jb : I.zc0));
+            int kc = 0;
+            for (; kc + 4 <= nc; kc += 4) {
+                const float v0 = trial_cp(cpp, g, scale, src + kc * gplane);
+                const float v1 = trial_cp(cpp, g, scale, src + (kc + 1) * gplane);
+                const float v2 = trial_cp(cpp, g, scale, src + (kc + 2) * gplane);
+                const float v3 = trial_cp(cpp, g, scale, src + (kc + 3) * gplane);
+                dst[kc * splane] = (float)((double)v0 - (rowid + kstep * kc));
+                dst[(kc + 1) * splane] = (float)((double)v1 - (rowid + kstep * (kc + 1)));
+                dst[(kc + 2) * splane] = (float)((double)v2 - (rowid + kstep * (kc + 2)));
+                dst[(kc + 3) * splane] = (float)((double)v3 - (rowid + kstep * (kc + 3)));
             }
+            for (; kc < nc; ++kc)
+                dst[kc * splane] = (float)((double)trial_cp(cpp, g, scale, src + kc * gplane) - (rowid + kstep * kc));
+        }
+    }
     for (int zi = threadIdx.x; zi < I.z1 - I.z0; zi += blockDim.x) {
         const int z = I.z0 + zi;
         const int pz = pre_of(z, P.gsz);
@@ -136,7 +136,6 @@ __device__ __forceinline__ void stage_item(const WalkParams& P, const float *__r
         split_hi_lo(identity_coord(P.io[2], P.is[2], pz, frac_of_d(z, P.gsz, pz)), h.x, h.y);
         zid[zi] = h;
     }
-    __syncthreads();
 }
 
 // Per-thread walker: x/y weights of the thread's column and the rolling window of the four
@@ -502,6 +501,7 @@ __device__ __forceinline__ void objective_item(const WalkParams& P, const WalkSm
     stage_item<true>(P, cpp, item, S.cp, S.zb, S.zk, S.zid, I, grad, scale);
     Column C;
     column_init(P, I, S.cp, C);
+    __syncthreads();
     if (kXs) build_xrows(P, C, S.cp, X);
     const int nzi = I.z1 - I.z0;
     const int zstride = P.nx * P.ny;
@@ -740,6 +740,7 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
     stage_item(P, cpp, item, S.cp, S.zb, S.zk, S.zid, I);
     Column C;
     column_init(P, I, S.cp, C);
+    __syncthreads();
     if (kXs) build_xrows(P, C, S.cp, X);
     const int nzi = I.z1 - I.z0;
     const int zstride = P.nx * P.ny;
@@ -810,6 +811,7 @@ k_deformation(WalkParams P, const int32_t *__restrict__ mask, const float *__res
         stage_item(P, cpp, item, S.cp, S.zb, S.zk, S.zid, I);
         Column C;
         column_init(P, I, S.cp, C);
+        __syncthreads();
         if (kXs) build_xrows(P, C, S.cp, X);
         const int nzi = I.z1 - I.z0;
         int idx = (I.z0 * P.ny + C.y) * P.nx + C.x;
@@ -1293,6 +1295,7 @@ k_warp_order(WalkParams P, const float *__restrict__ cpp, const float *__restric
         stage_item(P, cpp, item, S.cp, S.zb, S.zk, S.zid, I);
         Column C;
         column_init(P, I, S.cp, C);
+        __syncthreads();
         const int nzi = I.z1 - I.z0;
         for (int zi = 0; zi < nzi; ++zi) {
             float pos[3];
