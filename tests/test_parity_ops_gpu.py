@@ -192,6 +192,30 @@ def test_convolve_to_nodes(O, case):
     assert np.abs(host(node) - ref).max() <= 1e-5 * scale
 
 
+@pytest.mark.parametrize("dim,spacing", [((33, 5, 3), 5.0), ((3, 34, 7), 2.5), ((2, 9, 65), 40.0), ((700, 3, 2), 5.0),
+                                         ((3, 1100, 5), 5.0), ((5, 2, 1500), 5.0), ((7000, 2, 2), 5.0), ((2, 7000, 3), 5.0)])
+def test_kernel_convolution_cubic_line_lengths(O, dim, spacing):
+    """Lines held 32, 16 and 8 at a time with remainders, windows longer than the line, and lines too
+    long for a block; NaN voxels. The bar of the op above; the allocation-free entry point gives the
+    same floats."""
+    import ctypes
+    rng = np.random.default_rng(sum(dim))
+    pix = (1.0, 1.0, 1.0)
+    img = rng.normal(0, 1, 2 * int(np.prod(dim))).astype(np.float32)
+    img[rng.random(img.size) < 0.02] = np.nan
+    for axis in range(3):
+        t, u = dev(img), dev(img)
+        nrb.kernel_convolution_cubic(t, 2, dim, pix, spacing, axis)
+        nrb.check(nrb.lib().nrb_kernel_convolution_cubic_static(
+            ctypes.c_void_p(u.data_ptr()), 2, nrb._I3(*dim), nrb._F3(*pix), ctypes.c_float(spacing), axis, None))
+        ref = O.kernel_convolution_cubic(img, 2, dim, pix, spacing, axis)
+        out = host(t)
+        assert np.array_equal(out, host(u), equal_nan=True)
+        assert np.array_equal(np.isnan(out), np.isnan(ref))
+        ok = np.isfinite(ref)
+        assert np.abs(out[ok] - ref[ok]).max() <= 1e-5 * np.abs(ref[ok]).max()
+
+
 @pytest.mark.parametrize("fdim", [(2, 2, 2), (1, 5, 4), (3, 2, 9), (40, 7, 5)])
 @pytest.mark.parametrize("pad", [np.nan, 0.0, 3.5])
 def test_trilinear_warp_at_the_volume_border(O, fdim, pad):
