@@ -7,6 +7,7 @@
 #include <cfloat>
 #include <climits>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -1499,17 +1500,24 @@ static nrb_status make_sampling(const nrb_geometry *g, AxisSampling ax[3]) {
     return NRB_OK;
 }
 
-// The source vectors live as long as the workspace, so the stream-ordered copy may finish later.
+// A workspace's memory: on its owner's stream when it has one; otherwise from the library's pool as
+// well, usable on any stream once the creator has synchronised, and given back only after the device
+// has finished with it, as cudaFree would wait (mapping and unmapping fresh memory took most of a
+// creation).
 template <typename T>
-static nrb_status upload(T *&dst, const std::vector<T>& src, size_t& bytes, cudaStream_t st) {
-    NRB_CUDA(dev_alloc(&dst, std::max<size_t>(1, src.size()) * sizeof(T), st));
-    if (!src.empty()) {
-        if (st) NRB_CUDA(cudaMemcpyAsync(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-        else NRB_CUDA(cudaMemcpy(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
-    }
-    bytes += src.size() * sizeof(T);
-    return NRB_OK;
+static cudaError_t ws_alloc(T **p, size_t bytes, cudaStream_t st) {
+    return st ? dev_alloc(p, bytes, st) : tmp_alloc(p, bytes, nullptr);
 }
+
+// Consecutive 256-byte aligned parts of one allocation
+struct Arena {
+    size_t bytes = 0;
+    size_t add(size_t n) {
+        const size_t at = bytes;
+        bytes += (std::max<size_t>(1, n) + 255) & ~size_t(255);
+        return at;
+    }
+};
 
 // Items of the voxel walk. The persistent grid holds slots_for(shared bytes) co-resident blocks
 // and every block walks ceil(items / slots) items, so the z-chunk count is chosen to minimise a
@@ -1599,7 +1607,7 @@ static nrb_status workspace_alloc(nrb_workspace *ws) {
         // the whole-volume convolution and per-node sampling replace the separable passes
         ws->general = true;
         const size_t vb = (size_t)3 * nvox(g->ref_dim) * 4;
-        if (dev_alloc(&ws->general_vox, vb, ws->st) != cudaSuccess) {
+        if (ws_alloc(&ws->general_vox, vb, ws->st) != cudaSuccess) {
             cudaGetLastError();
             return fail(NRB_ERR_OOM, "workspace allocation failed");
         }
@@ -1612,33 +1620,59 @@ static nrb_status workspace_alloc(nrb_workspace *ws) {
     } else {
         NRB_TRY(make_sampling(g, ws->ax));
     }
+    cudaStream_t st = ws->st;
+    // the sampling tables: one allocation and one copy (its host image lives as long as the
+    // workspace, so the stream-ordered copy may finish later)
+    Arena t;
+    size_t at[3][4];
     for (int d = 0; d < 3; ++d) {
-        NRB_TRY(upload(ws->d_samples[d], ws->ax[d].samples, bytes, ws->st));
-        NRB_TRY(upload(ws->d_tap_slot[d], ws->ax[d].tap_slot, bytes, ws->st));
-        NRB_TRY(upload(ws->d_tap_weight[d], ws->ax[d].tap_weight, bytes, ws->st));
-        NRB_TRY(upload(ws->d_kernel[d], ws->ax[d].kernel, bytes, ws->st));
+        const AxisSampling& x = ws->ax[d];
+        at[d][0] = t.add(x.samples.size() * sizeof(int));
+        at[d][1] = t.add(x.tap_slot.size() * sizeof(int));
+        at[d][2] = t.add(x.tap_weight.size() * sizeof(float));
+        at[d][3] = t.add(x.kernel.size() * sizeof(float));
     }
-    const long long nx = g->ref_dim[0], ny = g->ref_dim[1], nz = g->ref_dim[2];
+    ws->table_host.assign(t.bytes, 0);
+    // scratch: one allocation
+    const long long ny = g->ref_dim[1], nz = g->ref_dim[2];
     const long long c1 = 3LL * nz * ny * ws->ax[0].nsamples;
     const long long c2 = 3LL * nz * ws->ax[1].nsamples * ws->ax[0].nsamples;
     const long long c3 = 3LL * ws->ax[2].nsamples * ws->ax[1].nsamples * ws->ax[0].nsamples;
-    (void)nx;
-    const size_t sz1 = (size_t)std::max(c1, c3) * 4, sz2 = (size_t)c2 * 4;
     const size_t be_bytes = (size_t)18 * BePad(g->cpp_dim[0], g->cpp_dim[1], g->cpp_dim[2]).size * 4;
-    cudaStream_t st = ws->st;
-    if (dev_alloc(&ws->conv1, sz1, st) != cudaSuccess || dev_alloc(&ws->conv2, sz2, st) != cudaSuccess ||
-        dev_alloc(&ws->be_deriv, be_bytes, st) != cudaSuccess ||
-        dev_alloc(&ws->red, 2 * NRB_RED_BLOCKS * sizeof(double), st) != cudaSuccess ||
-        dev_alloc(&ws->be_partials, NRB_RED_BLOCKS * sizeof(double), st) != cudaSuccess ||
-        dev_alloc(&ws->fred, 2 * NRB_RED_BLOCKS * sizeof(float), st) != cudaSuccess) {
+    Arena m;
+    const size_t o_conv1 = m.add((size_t)std::max(c1, c3) * 4), o_conv2 = m.add((size_t)c2 * 4), o_be = m.add(be_bytes);
+    const size_t o_red = m.add(2 * NRB_RED_BLOCKS * sizeof(double)), o_bep = m.add(NRB_RED_BLOCKS * sizeof(double));
+    const size_t o_fred = m.add(2 * NRB_RED_BLOCKS * sizeof(float));
+    if (ws_alloc(&ws->tables, t.bytes, st) != cudaSuccess || ws_alloc(&ws->scratch, m.bytes, st) != cudaSuccess) {
         cudaGetLastError();
         return fail(NRB_ERR_OOM, "workspace allocation failed");
     }
+    for (int d = 0; d < 3; ++d) {
+        const AxisSampling& x = ws->ax[d];
+        char *h = ws->table_host.data();
+        auto put = [&](size_t off, const void *src, size_t n) {
+            if (n) memcpy(h + off, src, n);
+        };
+        put(at[d][0], x.samples.data(), x.samples.size() * sizeof(int));
+        put(at[d][1], x.tap_slot.data(), x.tap_slot.size() * sizeof(int));
+        put(at[d][2], x.tap_weight.data(), x.tap_weight.size() * sizeof(float));
+        put(at[d][3], x.kernel.data(), x.kernel.size() * sizeof(float));
+        ws->d_samples[d] = reinterpret_cast<int *>(ws->tables + at[d][0]);
+        ws->d_tap_slot[d] = reinterpret_cast<int *>(ws->tables + at[d][1]);
+        ws->d_tap_weight[d] = reinterpret_cast<float *>(ws->tables + at[d][2]);
+        ws->d_kernel[d] = reinterpret_cast<float *>(ws->tables + at[d][3]);
+    }
+    ws->conv1 = reinterpret_cast<float *>(ws->scratch + o_conv1);
+    ws->conv2 = reinterpret_cast<float *>(ws->scratch + o_conv2);
+    ws->be_deriv = reinterpret_cast<float *>(ws->scratch + o_be);
+    ws->red = reinterpret_cast<double *>(ws->scratch + o_red);
+    ws->be_partials = reinterpret_cast<double *>(ws->scratch + o_bep);
+    ws->fred = reinterpret_cast<float *>(ws->scratch + o_fred);
+    NRB_CUDA(cudaMemcpyAsync(ws->tables, ws->table_host.data(), t.bytes, cudaMemcpyHostToDevice, st));
     // the ring of zeros around every derivative plane
     NRB_CUDA(cudaMemsetAsync(ws->be_deriv, 0, be_bytes, st));
     if (!st) NRB_CUDA(cudaStreamSynchronize(st));  // the workspace may be used on any stream at once
-    bytes += sz1 + sz2 + be_bytes + 3 * NRB_RED_BLOCKS * sizeof(double) + 2 * NRB_RED_BLOCKS * 4;
-    ws->bytes = bytes;
+    ws->bytes = bytes + t.bytes + m.bytes;
     NRB_CUDA(cudaStreamCreateWithFlags(&ws->side, cudaStreamNonBlocking));
     NRB_CUDA(cudaEventCreateWithFlags(&ws->ev_fork, cudaEventDisableTiming));
     NRB_CUDA(cudaEventCreateWithFlags(&ws->ev_join, cudaEventDisableTiming));
@@ -1659,19 +1693,19 @@ nrb_status join_side(nrb_workspace *ws, cudaStream_t st) {
 
 void workspace_free(nrb_workspace *ws) {
     cudaStream_t st = ws->st;
-    for (int d = 0; d < 3; ++d) {
-        dev_free(ws->d_samples[d], st);
-        dev_free(ws->d_tap_slot[d], st);
-        dev_free(ws->d_tap_weight[d], st);
-        dev_free(ws->d_kernel[d], st);
+    if (st) {
+        dev_free(ws->tables, st);
+        dev_free(ws->scratch, st);
+        dev_free(ws->general_vox, st);
+    } else {
+        int cur = ws->device;
+        cudaGetDevice(&cur);
+        if (cur != ws->device) cudaSetDevice(ws->device);
+        cudaDeviceSynchronize();
+        for (void *p : { (void *)ws->tables, (void *)ws->scratch, (void *)ws->general_vox })
+            if (p) cudaFreeAsync(p, nullptr);
+        if (cur != ws->device) cudaSetDevice(cur);
     }
-    dev_free(ws->conv1, st);
-    dev_free(ws->conv2, st);
-    dev_free(ws->general_vox, st);
-    dev_free(ws->be_deriv, st);
-    dev_free(ws->red, st);
-    dev_free(ws->be_partials, st);
-    dev_free(ws->fred, st);
     // the side stream's work is ordered before st's last join; its frees above are on st
     if (ws->ev_fork) cudaEventDestroy(ws->ev_fork);
     if (ws->ev_join) cudaEventDestroy(ws->ev_join);

@@ -512,11 +512,15 @@ struct nrb_workspace {
     nrb_geometry g{};
     int device = 0;
     nrb::WalkPlan walk_obj, walk_grad;
+    // the allocations: sampling tables (with their host image) and scratch; the pointers below lie in
+    // them
+    char *tables = nullptr, *scratch = nullptr;
+    std::vector<char> table_host;
     // reduction partials (double pairs) and scalars
     double *red = nullptr;          // 2 * NRB_RED_BLOCKS doubles
     double *be_partials = nullptr;  // NRB_RED_BLOCKS doubles
     float *fred = nullptr;          // 2 * NRB_RED_BLOCKS floats (min | max partials)
-    // bending-energy gradient: 18 derivative values per node
+    // bending-energy gradient: 18 derivative values per node, planes with a ring of zeros
     float *be_deriv = nullptr;
     // convolution-at-nodes scratch
     AxisSampling ax[3];
