@@ -369,9 +369,11 @@ __global__ void __launch_bounds__(256, 2) k_velocity_flow_table(const float *__r
     if (kExtrema) flow_extrema(lo, hi, minmax);
 }
 
-// The flow of a field in any orientation: one voxel per thread, its basis evaluated in full
+// The flow of a field in any orientation: one voxel per thread, its basis evaluated in full. 64
+// registers for four blocks per SM: an exponentiation of an oblique 160x192x160 field takes 603 us,
+// 613 at 80 registers (2.2 ms before the pairs layout and the pool).
 template <bool kExtrema>
-__global__ void __launch_bounds__(256, 3) k_velocity_flow(const float *__restrict__ vel, int gx, int gy, int gz,
+__global__ void __launch_bounds__(256, 4) k_velocity_flow(const float *__restrict__ vel, int gx, int gy, int gz,
                                                       Mat34 gxyz, Mat34 gijk, FieldGeom f, float *__restrict__ out,
                                                       float scale, unsigned *__restrict__ minmax) {
     const long long n = (long long)f.nx * f.ny * f.nz;
@@ -543,9 +545,11 @@ struct Mat33f {
 // `reorient` and divided by the real spacing per column; then reg_tools_addImageToImage, and on
 // the last step the division by 2^N (scale = 2^-N, exact).
 // def is in the pairs layout, g in it when kInPairs, out when kOutPairs. A division by the spacing
-// is a product where the spacing is a power of two (the same float).
+// is a product where the spacing is a power of two (the same float). Waits on its gathers: 40
+// registers for six blocks per SM; a transport of 160x192x160 (N = 6, the squarings included) takes
+// 1154 us, 1240 at 64 registers, 3.9 ms or more planar with the buffers mapped by each call.
 template <bool kInPairs, bool kOutPairs, typename I>
-__global__ void __launch_bounds__(256) k_gradient_exp_step(const float *__restrict__ g, const float *__restrict__ def,
+__global__ void __launch_bounds__(256, 6) k_gradient_exp_step(const float *__restrict__ g, const float *__restrict__ def,
                                                           float *__restrict__ out, FieldGeom f, Mat33f R, float spx,
                                                           float spy, float spz, int unit, float scale) {
     const I n = (I)f.nx * f.ny * f.nz;
