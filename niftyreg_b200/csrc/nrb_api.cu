@@ -95,17 +95,55 @@ void lib_pool_keep(uint64_t bytes) {
     cudaGetLastError();
 }
 
-// A small device value to host memory, after the stream's work: through pinned memory of the host
-// thread's own (a copy into pageable memory stages through the driver first). Synchronises.
+// ---- small values read back ------------------------------------------------------------------
+// Pinned slots of kPinnedBytes, portable across devices: one per call in flight, of which up to
+// kPinnedKept are kept for the next calls and the rest given back.
+namespace {
+constexpr size_t kPinnedBytes = 256;
+constexpr int kPinnedKept = 32;
+std::mutex g_pin_mu;
+void *g_pin_free[kPinnedKept];
+int g_pin_count = 0;
+
+struct PinnedSlot {
+    void *p = nullptr;
+    PinnedSlot(const PinnedSlot &) = delete;
+    PinnedSlot() {
+        {
+            std::lock_guard<std::mutex> lock(g_pin_mu);
+            if (g_pin_count) {
+                p = g_pin_free[--g_pin_count];
+                return;
+            }
+        }
+        if (cudaHostAlloc(&p, kPinnedBytes, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    ~PinnedSlot() {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lock(g_pin_mu);
+            if (g_pin_count < kPinnedKept) {
+                g_pin_free[g_pin_count++] = p;
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+};
+}  // namespace
+
+// A small device value to host memory, after the stream's work: through pinned memory (a copy into
+// pageable memory stages through the driver first; it serves when no pinned memory is to be had).
+// Synchronises.
 nrb_status read_back(void *host, const void *dev, size_t bytes, cudaStream_t st) {
-    static thread_local void *pinned = nullptr;
-    constexpr size_t kBytes = 256;
-    if (bytes > kBytes) return fail(NRB_ERR_INVALID, "read_back: value too large");
-    // portable across devices, kept for the thread's lifetime
-    if (!pinned) NRB_CUDA(cudaHostAlloc(&pinned, kBytes, cudaHostAllocPortable));
-    NRB_CUDA(cudaMemcpyAsync(pinned, dev, bytes, cudaMemcpyDeviceToHost, st));
+    PinnedSlot slot;
+    void *to = slot.p && bytes <= kPinnedBytes ? slot.p : host;
+    NRB_CUDA(cudaMemcpyAsync(to, dev, bytes, cudaMemcpyDeviceToHost, st));
     NRB_CUDA(cudaStreamSynchronize(st));
-    memcpy(host, pinned, bytes);
+    if (to != host) memcpy(host, to, bytes);
     return NRB_OK;
 }
 

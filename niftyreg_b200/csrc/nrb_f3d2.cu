@@ -800,12 +800,8 @@ nrb_status velocity_to_deformation(const nrb_geometry *g, const float *vel, bool
         NRB_LAUNCHED("k_velocity_flow");
     }
     if (update) {
-        // the extrema land in pinned host memory (a pageable copy would stage through the driver):
-        // 8 bytes per host thread, portable across devices, kept for the thread's lifetime
-        static thread_local unsigned *mm = nullptr;
-        if (!mm) NRB_CUDA(cudaHostAlloc((void **)&mm, 2 * sizeof(unsigned), cudaHostAllocPortable));
-        NRB_CUDA(cudaMemcpyAsync(mm, minmax, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-        NRB_CUDA(cudaStreamSynchronize(st));
+        unsigned mm[2];
+        NRB_TRY(read_back(mm, minmax, sizeof(mm), st));
         N = velocity_squaring_steps(fkey_inv(mm[0]), fkey_inv(mm[1]));
         *steps = N;
         // scaled into the buffer an even or odd chain starts from (another one when the parity of N
