@@ -1719,7 +1719,7 @@ int64_t velocity_field_stride(int64_t nvox);
 nrb_status velocity_to_deformation(const nrb_geometry *g, const float *vel, bool update, int *steps, float *def,
                                    float *fields, float *scratch, unsigned *minmax, cudaStream_t st);
 nrb_status exponentiate_gradient(const nrb_geometry *g, const float *vel_other, int steps, float *vgrad,
-                                 float *fields, float *scratch, unsigned *minmax, cudaStream_t st);
+                                 float *fields, int64_t fields_n, float *scratch, unsigned *minmax, cudaStream_t st);
 nrb_status symmetrise_velocity(const int32_t cdim[3], const float fw_xyz[16], float *fw, const float bw_xyz[16],
                                float *bw, cudaStream_t st);
 
@@ -1839,16 +1839,21 @@ private:
         NRB_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));
         return NRB_OK;
     }
-    // intermediate fields of both gradient exponentiations
+    // intermediate fields of both gradient exponentiations, for the squaring number as it stands. A
+    // buffer that grows is allocated on st_, so the side stream waits for it. Called between a fork
+    // and its join.
     nrb_status Fields(int64_t nref, int64_t nflo) {
         const int64_t need[2] = { (int64_t)steps_ * velocity_field_stride(nref), (int64_t)steps_ * velocity_field_stride(nflo) };
         DevBuf *const buf[2] = { &fields_, &fields_b_ };
+        bool grown = false;
         for (int i = 0; i < 2; ++i)
             if (need[i] > fields_n_[i]) {
+                fields_n_[i] = 0;
                 NRB_TRY(buf[i]->alloc(need[i], st_));
                 fields_n_[i] = need[i];
+                grown = true;
             }
-        return NRB_OK;
+        return grown ? Fork() : NRB_OK;
     }
     // reg_f3d2::GetDeformationField + WarpFloatingImage (_reg_f3d2.cpp:144-181): the forward
     // field (squaring number updated when the optimiser runs), the backward one with the same
@@ -1899,7 +1904,6 @@ private:
     // (:244-305), ExponentiateGradient (:637-650) and NormaliseGradient (:369-391)
     nrb_status GetObjectiveFunctionGradient() {
         const int64_t nr = nvox(gfw_.ref_dim), nf = nvox(gbw_.ref_dim);
-        if (sim_w_ > 0) NRB_TRY(Fields(nr, nf));
         NRB_TRY(Fork());
         if (sim_w_ > 0) {
             // the fields and warped images at the best position: those of the accepted trial when
@@ -1928,17 +1932,21 @@ private:
                 NRB_TRY(nmi_voxel_gradient(nmi_bw_.h, &gbw_, flo_.p, war_bw_.p, wg_bw_.p, nullptr, 1.0, vg_bw_.p, side_,
                                            true));
             }
-            // forward gradient along the backward transformation on the reference grid, and back
+            // forward gradient along the backward transformation on the reference grid, and back; the
+            // squaring number is the best position's from here on
+            NRB_TRY(Fields(nr, nf));
             nrb_geometry gx = gfw_;
             for (int i = 0; i < 3; ++i) gx.cpp_dim[i] = gbw_.cpp_dim[i], gx.cpp_pixdim[i] = gbw_.cpp_pixdim[i];
             memcpy(gx.cpp_xyz, gbw_.cpp_xyz, sizeof(gx.cpp_xyz));
             memcpy(gx.cpp_ijk, gbw_.cpp_ijk, sizeof(gx.cpp_ijk));
-            NRB_TRY(exponentiate_gradient(&gx, bw(cur_), steps_, vg_fw_.p, fields_.p, scr_r_.p, mm_, st_));
+            NRB_TRY(exponentiate_gradient(&gx, bw(cur_), steps_, vg_fw_.p, fields_.p, fields_n_[0], scr_r_.p, mm_,
+                                          st_));
             gx = gbw_;
             for (int i = 0; i < 3; ++i) gx.cpp_dim[i] = gfw_.cpp_dim[i], gx.cpp_pixdim[i] = gfw_.cpp_pixdim[i];
             memcpy(gx.cpp_xyz, gfw_.cpp_xyz, sizeof(gx.cpp_xyz));
             memcpy(gx.cpp_ijk, gfw_.cpp_ijk, sizeof(gx.cpp_ijk));
-            NRB_TRY(exponentiate_gradient(&gx, fw(cur_), steps_, vg_bw_.p, fields_b_.p, scr_f_.p, mm_, side_));
+            NRB_TRY(exponentiate_gradient(&gx, fw(cur_), steps_, vg_bw_.p, fields_b_.p, fields_n_[1], scr_f_.p, mm_,
+                                          side_));
             KernelTimer kt(TK_F2_NODES, 0.0, st_);
             NRB_TRY(nrb_convolve_voxel_based_gradient(ws_fw_.h, &gfw_, vg_fw_.p, sim_w_, fw(grad_), st_));
             NRB_TRY(nrb_convolve_voxel_based_gradient(ws_bw_.h, &gbw_, vg_bw_.p, sim_w_, bw(grad_), side_));

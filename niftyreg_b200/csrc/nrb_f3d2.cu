@@ -902,10 +902,13 @@ static void real_spacing(const float xyz[16], float sp[3]) {
 // Compute::ExponentiateGradient (reg-lib/Compute.cpp:288-330) for the voxel-based gradient
 // `vgrad` on g->ref_* and the opposite transformation's velocity grid g->cpp_*: the intermediate
 // fields of that grid (N squarings), then N gradient resampling steps, then the division by 2^N.
-// fields: N * velocity_field_stride(nvox) floats, scratch: 3 * nvox floats, both 8-byte aligned.
+// fields: fields_n floats, of which N * velocity_field_stride(nvox) are used (refused when there are
+// fewer), scratch: 3 * nvox floats, both 8-byte aligned.
 nrb_status exponentiate_gradient(const nrb_geometry *g, const float *vel_other, int steps, float *vgrad,
-                                 float *fields, float *scratch, unsigned *minmax, cudaStream_t st) {
+                                 float *fields, int64_t fields_n, float *scratch, unsigned *minmax, cudaStream_t st) {
     if (steps < 1) return fail(NRB_ERR_INVALID, "gradient exponentiation: the squaring number must be >= 1");
+    if (steps * velocity_field_stride(nvox(g->ref_dim)) > fields_n)
+        return fail(NRB_ERR_INVALID, "gradient exponentiation: the intermediate fields exceed their buffer");
     KernelTimer stage(TK_F2_GRADIENT_EXP, 0.0, st);
     int N = steps;
     NRB_TRY(velocity_to_deformation(g, vel_other, false, &N, nullptr, fields, scratch, minmax, st));
@@ -1052,8 +1055,9 @@ extern "C" nrb_status nrb_exponentiate_gradient(const nrb_geometry *g, const flo
     Scratch s(st), fields(st);
     NRB_CUDA(tmp_alloc(&s.p, 3 * n * sizeof(float), st));
     NRB_CUDA(tmp_alloc(&s.mm, 2 * sizeof(unsigned), st));
-    NRB_CUDA(tmp_alloc(&fields.p, (size_t)steps * velocity_field_stride(n) * sizeof(float), st));
-    return exponentiate_gradient(g, vel_other, steps, vgrad, fields.p, s.p, s.mm, st);
+    const int64_t fields_n = steps * velocity_field_stride(n);
+    NRB_CUDA(tmp_alloc(&fields.p, (size_t)fields_n * sizeof(float), st));
+    return exponentiate_gradient(g, vel_other, steps, vgrad, fields.p, fields_n, s.p, s.mm, st);
 }
 
 extern "C" nrb_status nrb_symmetrise_velocity_fields(const nrb_geometry *g_fw, float *fw, const nrb_geometry *g_bw,

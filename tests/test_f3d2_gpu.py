@@ -326,3 +326,48 @@ def test_f3d2_file_request_writes_both_directions(tmp_path):
     w, _, _ = nrb.read_image(tmp_path / "res.nii")
     wbk, _, _ = nrb.read_image(tmp_path / "res_backward.nii")
     assert np.array_equal(w[0], wf, equal_nan=True) and np.array_equal(wbk[0], wb, equal_nan=True)
+
+
+def test_squaring_number_that_rises_with_a_level():
+    """The intermediate fields cover the squaring number of the gradient they serve. The finer
+    level samples the flow at more points, so its first gradient can need one squaring more than
+    the last trial of the coarser level: the voxel size (which scales the displacements, and
+    nothing else) is scanned for a pair where it does, by the coarse level registered alone and
+    its grid's flow on the fine voxels. The whole registration then runs, and ends as the same
+    pair does at a voxel size 10% smaller (the end-point bar)."""
+    ensure_built()
+    pair = phantom.blobs_pair((64, 64, 64), seed=6, disp_sigma_vox=4.0)
+    dim = (64, 64, 64)
+
+    def register(ref, flo, mm, levels, maxit):
+        params = nrb.default_params(levels=levels, max_iterations=maxit, bending_energy=0.0, spacing=(-2.0,),
+                                    ref_bins=32, flo_bins=32)
+        pix = (mm,) * 3
+        xyz = nrb.identity_header(pix)
+        return nrb.f3d2_register_images(ref, pix, xyz, flo, pix, xyz, params, warped=False)
+
+    def coarse(img):
+        xyz = nrb.identity_header((1.0, 1.0, 1.0))
+        dims, _, total = nrb.image_pyramid_headers(dim, (1.0, 1.0, 1.0), xyz, 2)
+        out = torch.empty(total, dtype=torch.float32, device="cuda")
+        nrb.image_pyramid(dev(img.ravel()), dim, (1.0, 1.0, 1.0), xyz, 2, out)
+        assert tuple(dims[0]) == (32, 32, 32)
+        return host(out)[:32 ** 3].reshape(32, 32, 32).copy()
+
+    ref, flo = coarse(pair.reference), coarse(pair.floating)
+    rising = []
+    field = torch.empty(3 * 64 ** 3, dtype=torch.float32, device="cuda")
+    for mm in np.geomspace(4.0, 10.0, 150):
+        mm = float(np.float32(mm))
+        gf, _, (xf, _), last, _, _, _ = register(ref, flo, 2 * mm, 1, 30)
+        pix = (mm,) * 3
+        xyz = nrb.identity_header(pix)
+        g = nrb.make_geometry(dim, pix, xyz, dim, pix, xyz, gf.shape[:0:-1], (4 * mm,) * 3, xf)
+        if nrb.get_def_field_from_velocity_grid(g, dev(gf.ravel()), last, field, update=True) > last:
+            rising.append(mm)
+    print("voxel sizes (mm) at which the finer level raises the squaring number:", rising)
+    assert rising
+    mm = rising[len(rising) // 2]
+    r = register(pair.reference, pair.floating, mm, 2, 15)[-1]
+    s = register(pair.reference, pair.floating, 0.9 * mm, 2, 15)[-1]
+    assert abs(r.final_nmi - s.final_nmi) <= 5e-3 * s.final_nmi
