@@ -1466,6 +1466,7 @@ struct BatchLevelRunner {
         const int np = (int)hp.size();
         BatchLaunch L;
         NRB_TRY(batch_plan(hp, L));
+        NRB_TRY(batch_node_plan(hp, L));
         BatchPair *d_pairs = nullptr;
         OptState *d_states = nullptr;
         BatchCtl *d_ctl = nullptr;
@@ -1521,7 +1522,7 @@ struct BatchLevelRunner {
             const Arg *x = static_cast<const Arg *>(a);
             return launch_batch_gradient(d, states, *x->L, st, x->bytes);
         };
-        NRB_TRY(launch_batch_node_stage(hp, d_pairs, d_states, s, side, ev_fork, ev_join, voxels, &arg));
+        NRB_TRY(launch_batch_node_stage(hp, L, d_pairs, d_states, s, side, ev_fork, ev_join, voxels, &arg));
         k_b_node_tail<<<TAIL_CTAS * L.npairs, TAIL_THREADS, 0, s>>>(d_pairs, d_states, L.npairs, d_ctl, in_graph ? 1 : 0,
                                                                   h_outer);
         NRB_CUDA(cudaGetLastError());

@@ -1748,9 +1748,16 @@ static void conv_kernels(const nrb_workspace *ws, const nrb_geometry *g, int R[3
         K[i] = ws->d_kernel[i] + (ws->ax[i].radius - R[i]);
     }
 }
+// Above 48 KB a block's shared memory, static arrays included, is opted into: the batched passes hold
+// a BatchList beside their tile. The opt-in belongs to the function, not to the launch, and other
+// host threads launch it too, so it is one constant and never this launch's size.
+constexpr size_t CONV_STATIC_BYTES = 2048, CONV_SHARED_MAX = 227 * 1024 - CONV_STATIC_BYTES;
+static_assert(sizeof(BatchList) + 128 <= CONV_STATIC_BYTES, "static shared memory of the batched convolution passes");
 template <typename K>
 static nrb_status conv_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (bytes > CONV_SHARED_MAX) return fail(NRB_ERR_UNSUPPORTED, "convolution: rows and kernel exceed shared memory");
+    if (bytes + CONV_STATIC_BYTES > 48 * 1024)
+        NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SHARED_MAX));
     return NRB_OK;
 }
 
@@ -2078,8 +2085,38 @@ nrb_status launch_batch_be_value(const std::vector<BatchPair>& hp, const BatchPa
     return NRB_OK;
 }
 
-nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const BatchPair *d, const OptState *states,
-                                   cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
+static auto batch_conv_x(int rows) { return rows == 32 ? k_b_conv_x<32> : rows == 16 ? k_b_conv_x<16> : k_b_conv_x<8>; }
+
+// Rows, shared memory and grids of the convolution passes for the largest pair, opted into before a
+// capture begins (a launch refused inside one would abort the level)
+nrb_status batch_node_plan(const std::vector<BatchPair>& hp, BatchLaunch& L) {
+    long long xb = 0, yb = 0, zb = 0;
+    L.conv_rows = 32;
+    L.conv_xsm = L.conv_ysm = 0;
+    for (const BatchPair& b : hp) L.conv_rows = std::min(L.conv_rows, conv_x_rows(b.rdim[0], b.radius[0], b.ns[0]));
+    for (const BatchPair& b : hp) {
+        L.conv_xsm = std::max(L.conv_xsm, conv_x_bytes(L.conv_rows, b.rdim[0], b.radius[0], b.ns[0]));
+        L.conv_ysm = std::max(L.conv_ysm, conv_y_bytes(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]));
+        xb += conv_x_units(L.conv_rows, b.rdim[1], b.rdim[2]);
+        yb += conv_y_units(b.rdim[1], b.rdim[2], b.ns[0], b.radius[1]);
+        zb += conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]);
+    }
+    auto plan = [](auto kernel, long long units, int threads, size_t smem, int& grid) -> nrb_status {
+        int per = 0;
+        NRB_TRY(conv_smem(kernel, smem));
+        NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
+        if (per < 1) return fail(NRB_ERR_UNSUPPORTED, "batched level: the convolution does not fit in shared memory");
+        grid = (int)std::max(1LL, std::min(units, (long long)per * sm_count()));
+        return NRB_OK;
+    };
+    NRB_TRY(plan(batch_conv_x(L.conv_rows), xb, CONV_X_THREADS, L.conv_xsm, L.conv_xgrid));
+    NRB_TRY(plan(k_b_conv_y, yb, CONV_Y_THREADS, L.conv_ysm, L.conv_ygrid));
+    L.conv_zgrid = grid_for(std::max(1LL, zb), 256);
+    return NRB_OK;
+}
+
+nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const BatchLaunch& L, const BatchPair *d,
+                                   const OptState *states, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
                                    nrb_status (*gradient)(const BatchPair *, const OptState *, cudaStream_t, void *),
                                    void *gradient_arg) {
     const int np = (int)hp.size();
@@ -2095,34 +2132,15 @@ nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const Batch
         NRB_LAUNCHED("k_b_be_derivatives");
     }
     NRB_TRY(gradient(d, states, st, gradient_arg));
-    // shared memory and rows per block for the largest pair
-    size_t xsm = 0, ysm = 0;
-    long long xb = 0, yb = 0, zb = 0;
-    int rows = 32;
-    for (const BatchPair& b : hp) rows = std::min(rows, conv_x_rows(b.rdim[0], b.radius[0], b.ns[0]));
-    for (const BatchPair& b : hp) {
-        xsm = std::max(xsm, conv_x_bytes(rows, b.rdim[0], b.radius[0], b.ns[0]));
-        ysm = std::max(ysm, conv_y_bytes(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]));
-        xb += conv_x_units(rows, b.rdim[1], b.rdim[2]);
-        yb += conv_y_units(b.rdim[1], b.rdim[2], b.ns[0], b.radius[1]);
-        zb += conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]);
-    }
-    auto launch = [&](auto kernel, long long units, int threads, size_t smem) -> nrb_status {
-        int per = 0;
-        NRB_TRY(conv_smem(kernel, smem));
-        NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
-        const int grid = (int)std::max(1LL, std::min(units, (long long)std::max(1, per) * sm_count()));
-        kernel<<<grid, threads, smem, st>>>(d, states, np);
-        NRB_CUDA(cudaGetLastError());
-        return NRB_OK;
-    };
     {
     KernelTimer timer(TK_CONV, 0.0, st);
-    NRB_TRY(launch(rows == 32 ? k_b_conv_x<32> : rows == 16 ? k_b_conv_x<16> : k_b_conv_x<8>, xb, CONV_X_THREADS, xsm));
+    batch_conv_x(L.conv_rows)<<<L.conv_xgrid, CONV_X_THREADS, L.conv_xsm, st>>>(d, states, np);
+    NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_conv_x");
-    NRB_TRY(launch(k_b_conv_y, yb, CONV_Y_THREADS, ysm));
+    k_b_conv_y<<<L.conv_ygrid, CONV_Y_THREADS, L.conv_ysm, st>>>(d, states, np);
+    NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_conv_y");
-    k_b_conv_z<<<grid_for(std::max(1LL, zb), 256), 256, 0, st>>>(d, states, np);
+    k_b_conv_z<<<L.conv_zgrid, 256, 0, st>>>(d, states, np);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_conv_z");
     const int gn = batch_grid(hp, [](const BatchPair& b) { return b.nnode; }, 256, 16);

@@ -211,6 +211,9 @@ struct BatchLaunch {
     int fetch = 0;  // how the floating images are read (Fetch)
     size_t obj_smem = 0, grad_smem = 0, fin_smem = 0;
     int obj_grid = 0, grad_grid = 0;
+    // the node stage's convolution (batch_node_plan)
+    int conv_rows = 0, conv_xgrid = 0, conv_ygrid = 0, conv_zgrid = 0;
+    size_t conv_xsm = 0, conv_ysm = 0;
 };
 
 // The pairs a batched stage serves (their phase is in `mask`) with the cost of their work units,
@@ -633,8 +636,10 @@ nrb_status batch_node_stage(const nrb_workspace *ws, const nrb_geometry *g, floa
                             BatchPair& b);
 nrb_status launch_batch_be_value(const std::vector<BatchPair>& hp, const BatchPair *d, const OptState *states,
                                  cudaStream_t st);
-nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const BatchPair *d, const OptState *states,
-                                   cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
+nrb_status batch_node_plan(const std::vector<BatchPair>& hp, BatchLaunch& L);
+nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const BatchLaunch& L, const BatchPair *d,
+                                   const OptState *states, cudaStream_t st, cudaStream_t side, cudaEvent_t fork,
+                                   cudaEvent_t join,
                                    nrb_status (*gradient)(const BatchPair *, const OptState *, cudaStream_t, void *),
                                    void *gradient_arg);
 // batched registrations (csrc/nrb_f3d.cu): n pairs advanced together level by level on `st`
