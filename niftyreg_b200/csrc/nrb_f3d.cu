@@ -277,6 +277,30 @@ struct GraphHolder {
     }
 };
 
+// Ends the capture into `top` or one of its bodies. Where it turns out invalid, what became of the
+// graph it wrote to is not defined: `top` is then left alone, not destroyed.
+nrb_status end_capture(cudaStream_t cap, GraphHolder& top) {
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(cap, &g);
+    if (e != cudaSuccess) top.g = nullptr;
+    NRB_CUDA(e);
+    return NRB_OK;
+}
+
+// The same after a step failed with `s`, which is returned. A stream still forked into the capture is
+// joined first: a capture that ends without it is invalid, and leaves the stream referring to a
+// graph about to be destroyed.
+nrb_status abort_capture(cudaStream_t cap, cudaStream_t side, cudaEvent_t join, GraphHolder& top, nrb_status s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (side && cudaStreamIsCapturing(side, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive &&
+        cudaEventRecord(join, side) == cudaSuccess)
+        cudaStreamWaitEvent(cap, join, 0);
+    cudaGraph_t g = nullptr;
+    if (cudaStreamEndCapture(cap, &g) != cudaSuccess) top.g = nullptr;
+    cudaGetLastError();
+    return s;  // with the failed step's message
+}
+
 // Appends a WHILE node driven by `h` to the graph `st` is capturing, after everything captured
 // so far, and returns its body graph; capture then continues after the node.
 nrb_status capture_while(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t *body) {
@@ -772,22 +796,17 @@ nrb_status F3dRegistration::RunLevelGraph(float max_step, float smallest_size, f
     NRB_CUDA(cudaGraphCreate(&top.g, 0));
     NRB_CUDA(cudaGraphConditionalHandleCreate(&h_outer, top.g, 0, 0));
     const long long c0 = g_launch_count.load();
-    auto abort_capture = [&](nrb_status s) {
-        cudaGraph_t dummy = nullptr;
-        cudaStreamEndCapture(cap_st_, &dummy);
-        cudaGetLastError();
-        return s;
-    };
+    auto abort_level = [&](nrb_status s) { return abort_capture(cap_st_, ws_.h->side, ws_.h->ev_join, top, s); };
     // top level
     NRB_CUDA(cudaStreamBeginCaptureToGraph(cap_st_, top.g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     k_ctl_level<<<1, 1, 0, cap_st_>>>(dstate_, init, h_outer);
-    if (cudaGetLastError() != cudaSuccess) return abort_capture(fail(NRB_ERR_CUDA, "registration: level init launch"));
+    if (cudaGetLastError() != cudaSuccess) return abort_level(fail(NRB_ERR_CUDA, "registration: level init launch"));
     g_launch_count.fetch_add(1);
     {
         nrb_status s = capture_while(cap_st_, h_outer, &outer_body);
-        if (s != NRB_OK) return abort_capture(s);
+        if (s != NRB_OK) return abort_level(s);
     }
-    NRB_CUDA(cudaStreamEndCapture(cap_st_, &top.g));
+    NRB_TRY(end_capture(cap_st_, top));
     const long long c_top = g_launch_count.load() - c0;
     // one iteration
     NRB_CUDA(cudaGraphConditionalHandleCreate(&h_inner, outer_body, 0, 0));
@@ -824,17 +843,17 @@ nrb_status F3dRegistration::RunLevelGraph(float max_step, float smallest_size, f
             g_launch_count.fetch_add(1);
             if (cudaGetLastError() != cudaSuccess) s = fail(NRB_ERR_CUDA, "registration: line end launch");
         }
-        if (s != NRB_OK) return abort_capture(s);
+        if (s != NRB_OK) return abort_level(s);
     }
-    NRB_CUDA(cudaStreamEndCapture(cap_st_, &outer_body));
+    NRB_TRY(end_capture(cap_st_, top));
     const long long c_outer = g_launch_count.load() - c0 - c_top;
     // one line-search step
     NRB_CUDA(cudaStreamBeginCaptureToGraph(cap_st_, inner_body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     {
         nrb_status s = CaptureLineStep(cap_st_, h_inner);
-        if (s != NRB_OK) return abort_capture(s);
+        if (s != NRB_OK) return abort_level(s);
     }
-    NRB_CUDA(cudaStreamEndCapture(cap_st_, &inner_body));
+    NRB_TRY(end_capture(cap_st_, top));
     const long long c_inner = g_launch_count.load() - c0 - c_top - c_outer;
     g_launch_count.fetch_sub(c_top + c_outer + c_inner);  // counted again below, per execution
 
@@ -1573,38 +1592,32 @@ struct BatchLevelRunner {
         cudaGraphConditionalHandle h_outer, h_grad;
         NRB_CUDA(cudaGraphCreate(&top.g, 0));
         NRB_CUDA(cudaGraphConditionalHandleCreate(&h_outer, top.g, 0, 0));
-        auto abort_capture = [&](nrb_status e) {
-            cudaGraph_t dummy = nullptr;
-            cudaStreamEndCapture(cap, &dummy);
-            if (dummy && dummy != top.g && dummy != while_body && dummy != if_body) cudaGraphDestroy(dummy);
-            cudaGetLastError();
-            return e;
-        };
+        auto abort_level = [&](nrb_status e) { return abort_capture(cap, side, ev_join, top, e); };
         const long long c0 = g_launch_count.load();
         NRB_CUDA(cudaStreamBeginCaptureToGraph(cap, top.g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
         {
             k_b_level_start<<<1, 1, 0, cap>>>(h_outer);
             nrb_status e = cudaGetLastError() == cudaSuccess ? NRB_OK : fail(NRB_ERR_CUDA, "batched level: start launch");
             if (e == NRB_OK) e = capture_while(cap, h_outer, &while_body);
-            if (e != NRB_OK) return abort_capture(e);
+            if (e != NRB_OK) return abort_level(e);
         }
-        NRB_CUDA(cudaStreamEndCapture(cap, &top.g));
+        NRB_TRY(end_capture(cap, top));
         NRB_CUDA(cudaGraphConditionalHandleCreate(&h_grad, while_body, 0, 0));
         // the line-search stage, then the IF node of the gradient stage
         NRB_CUDA(cudaStreamBeginCaptureToGraph(cap, while_body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
         {
             nrb_status e = line_stage(hp, L, d_pairs, d_states, d_ctl, cap, true, h_grad, h_outer, 0.0);
             if (e == NRB_OK) e = capture_if(cap, h_grad, &if_body);
-            if (e != NRB_OK) return abort_capture(e);
+            if (e != NRB_OK) return abort_level(e);
         }
-        NRB_CUDA(cudaStreamEndCapture(cap, &while_body));
+        NRB_TRY(end_capture(cap, top));
         const long long c_line = g_launch_count.load() - c0;
         NRB_CUDA(cudaStreamBeginCaptureToGraph(cap, if_body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
         {
             nrb_status e = gradient_stage(hp, L, d_pairs, d_states, d_ctl, cap, true, h_outer, 0.0);
-            if (e != NRB_OK) return abort_capture(e);
+            if (e != NRB_OK) return abort_level(e);
         }
-        NRB_CUDA(cudaStreamEndCapture(cap, &if_body));
+        NRB_TRY(end_capture(cap, top));
         const long long c_grad = g_launch_count.load() - c0 - c_line;
         g_launch_count.fetch_sub(c_line + c_grad);  // counted per execution below
         const auto t_inst = std::chrono::steady_clock::now();

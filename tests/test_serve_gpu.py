@@ -107,6 +107,27 @@ def test_batches_of_wide_volumes_equal_plain(shapes):
             _same(srv.wait(t)[:2], b)
 
 
+def test_a_refused_launch_inside_a_level_comes_back_as_a_status(pairs, plain):
+    """A convolution too wide for shared memory (2048 voxels, nodes 2300 voxels apart) is refused
+    when the gradient stage of a plain registration is captured, with the bending energy already
+    forked off on its side stream: an error, and the process registers on as before. A batch and a
+    server refuse it too."""
+    p = phantom.blobs_pair((8, 8, 2048), seed=50)
+    params = nrb.default_params(levels=1, max_iterations=10, bending_energy=0.005, spacing=(-2300.0, -5.0, -5.0),
+                                ref_bins=32, flo_bins=32)
+    for _ in range(3):
+        with pytest.raises(nrb.NrbError, match="convolution"):
+            nrb.register_host(p.reference, p.floating, p.pixdim, params)
+        with pytest.raises(nrb.NrbError, match="convolution"):
+            nrb.register_batch([(p.reference, p.floating, p.pixdim)] * 2, params, concurrency=2)
+        with nrb.Server(slots=1) as srv:
+            with pytest.raises(nrb.NrbError, match="convolution"):
+                srv.wait(srv.submit(p.reference, p.floating, p.pixdim, params))
+            q = pairs[1]
+            _same(srv.wait(srv.submit(q.reference, q.floating, q.pixdim, _params()))[:2], plain[1])
+        _same(nrb.register_host(q.reference, q.floating, q.pixdim, _params()), plain[1])
+
+
 def test_server_mix_equals_plain(pairs, plain):
     """Requests submitted while others run; each result as when run alone."""
     with nrb.Server(slots=3) as srv:
