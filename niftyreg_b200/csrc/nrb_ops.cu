@@ -738,13 +738,14 @@ struct EverySample {
     __device__ __forceinline__ int operator[](int j) const { return j; }
 };
 constexpr int CONV_LINE_THREADS = 256;
+constexpr size_t CONV_LINE_SHARED_MAX = 200 * 1024;
 // shared bytes of a block of `cols` lines; along x the lines are transposed (one column of padding)
 inline size_t conv_line_bytes(int cols, int n, int R, bool along_x) {
     return 4 * ((size_t)conv_weight_floats(R, n) + (size_t)(n + 2 * R) * (cols + (along_x ? 1 : 0)));
 }
 inline int conv_line_cols(int n, int R, bool along_x) {
     for (int cols : { 32, 16, 8 })
-        if (conv_line_bytes(cols, n, R, along_x) <= (cols == 8 ? 200 : 64) * 1024) return cols;
+        if (conv_line_bytes(cols, n, R, along_x) <= (cols == 8 ? CONV_LINE_SHARED_MAX : 64 * 1024)) return cols;
     return 0;
 }
 
@@ -811,7 +812,8 @@ static bool conv_lines(float *img, int nvol, const int32_t dim[3], int axis, con
     std::copy(taps.k + (radius - R), taps.k + (radius + R + 1), K.k);
     const size_t smem = conv_line_bytes(cols, n, R, axis == 0);
     auto go = [&](auto kernel) -> nrb_status {
-        NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // one constant: the opt-in is the function's, and other host threads launch it too
+        NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_LINE_SHARED_MAX));
         kernel<<<(unsigned)blocks, CONV_LINE_THREADS, smem, st>>>(img, outer, n, inner, K, R);
         NRB_LAUNCHED("k_conv_lines");
         return NRB_OK;

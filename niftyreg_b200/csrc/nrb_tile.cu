@@ -1567,9 +1567,13 @@ static void set_floating_margin(WalkParams& P, int margin, unsigned long long te
     P.fv = floating_view(P.fv.nx, P.fv.ny, P.fv.nz, margin, margin >= 2 ? tex : 0ull);
 }
 
+// Dynamic shared memory the kernels here are opted into (a launch that would need more is refused).
+// One constant: the opt-in is the function's, and other host threads launch it with other sizes.
+constexpr int SHARED_OPT_IN = 200 * 1024;
+
 template <typename K>
 static nrb_status persistent_grid(K kernel, int threads, size_t smem, int nitems, int& grid, int resident = 0) {
-    NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN));
     if (resident <= 0) {
         int per_sm = 0;
         NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
@@ -1586,7 +1590,7 @@ static nrb_status persistent_grid(K kernel, int threads, size_t smem, int nitems
 template <typename K>
 static long long blocks_resident(K kernel, int threads, size_t smem) {
     int per_sm = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -1899,7 +1903,7 @@ nrb_status launch_nmi_finalize(nrb_nmi *nmi, const double *be_partials, int n_be
                                long long acc_n) {
     const int rpc = (nmi->fb + FIN_CLUSTER - 1) / FIN_CLUSTER;
     const size_t smem = (size_t)(2 * rpc + 2) * nmi->rb * sizeof(double);
-    NRB_CUDA(cudaFuncSetAttribute(k_nmi_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NRB_CUDA(cudaFuncSetAttribute(k_nmi_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN));
     KernelTimer timer(TK_FINALIZE, (double)nmi->rb * nmi->fb * 8 + (double)nmi->total * 16, st);
     FinArgs A;
     A.rb = nmi->rb;
@@ -1997,13 +2001,13 @@ nrb_status batch_plan(std::vector<BatchPair>& pairs, BatchLaunch& L) {
     auto ko = with_flags<>(BatchObjectiveKernel{}, L.obj_xs, L.obj_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
     auto kg = with_flags<>(BatchGradientKernel{}, L.grad_f32, L.grad_xs, L.grad_diag, L.fetch == FETCH_NAN, L.fetch == FETCH_TEX);
     int per = 0;
-    NRB_CUDA(cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    NRB_CUDA(cudaFuncSetAttribute(ko, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN));
     NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ko, 32 * TY_OBJECTIVE, L.obj_smem));
     L.obj_grid = std::max(1, per) * sm_count();
-    NRB_CUDA(cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    NRB_CUDA(cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN));
     NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kg, 32 * TY_GRADIENT, L.grad_smem));
     L.grad_grid = std::max(1, per) * sm_count();
-    NRB_CUDA(cudaFuncSetAttribute(k_b_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.fin_smem));
+    NRB_CUDA(cudaFuncSetAttribute(k_b_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN));
     return NRB_OK;
 }
 
@@ -2244,7 +2248,7 @@ extern "C" nrb_status nrb_nmi_value(nrb_nmi *nmi, const nrb_geometry *g, const f
     const int threads = HIST_THREADS;
     const int grid = (int)std::min<long long>((nv + threads * HIST_VOX - 1) / (threads * HIST_VOX), 2LL * sm_count());
     const size_t smem = (size_t)nmi->rb * nmi->fb * 4;
-    NRB_CUDA(cudaFuncSetAttribute(k_histogram, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    NRB_CUDA(cudaFuncSetAttribute(k_histogram, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN));
     k_histogram<<<grid, threads, smem, st>>>(nv, nmi->rb, nmi->fb, ref, warped, mask, nmi->hist);
     NRB_LAUNCHED("k_histogram");
     NRB_TRY(launch_nmi_finalize(nmi, nullptr, 0, 1, 1.0, 0.0, obj, st));
@@ -2269,7 +2273,7 @@ nrb_status nmi_voxel_gradient(nrb_nmi *nmi, const nrb_geometry *g, const float *
     const bool f32 = !fp64 && log_bytes <= 96 * 1024;
     auto kernel = f32 ? k_nmi_voxel_gradient<true> : k_nmi_voxel_gradient<false>;
     const size_t smem = f32 ? log_bytes : 0;
-    if (f32) NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)log_bytes));
+    if (f32) NRB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_OPT_IN));
     int per = 0;
     NRB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
     const int grid = (int)std::min<long long>((nv + threads - 1) / threads, (long long)std::max(1, per) * sm_count());

@@ -216,6 +216,59 @@ def test_kernel_convolution_cubic_line_lengths(O, dim, spacing):
         assert np.abs(out[ok] - ref[ok]).max() <= 1e-5 * np.abs(ref[ok]).max()
 
 
+def test_threads_with_different_sizes_do_not_disturb_each_other():
+    """Two host threads, each on its own stream, run the same kernels with different shared-memory
+    sizes (line lengths, volume widths, bin counts) at once: every call succeeds and gives the floats
+    that it gives alone."""
+    import threading
+    pix = (1.0, 1.0, 1.0)
+    xyz = nrb.identity_header(pix)
+
+    class Work:
+        def __init__(self, line, width, bins, seed):
+            rng = np.random.default_rng(seed)
+            self.line = (40, line, 3)
+            self.img = dev(rng.normal(0, 1, int(np.prod(self.line))).astype(np.float32))
+            dim = (width, width, 2)
+            cdim, cpix, cxyz = nrb.control_grid_header(dim, pix, (5.0, 5.0, 5.0))
+            self.g = nrb.make_geometry(dim, pix, xyz, dim, pix, xyz, cdim, cpix, cxyz)
+            n = int(np.prod(dim))
+            self.ws, self.nmi = nrb.Workspace(self.g), nrb.Nmi(bins, bins)
+            self.vg = dev(rng.normal(0, 1e-3, 3 * n).astype(np.float32))
+            self.node = torch.empty(3 * int(np.prod(cdim)), dtype=torch.float32, device="cuda")
+            self.ref, self.war = (dev(rng.uniform(2, bins - 3, n).astype(np.float32)) for _ in range(2))
+            self.stream = torch.cuda.Stream()
+            torch.cuda.synchronize()
+            self.want = self.run()
+
+        def run(self):
+            with torch.cuda.stream(self.stream):
+                img, out = self.img.clone(), torch.zeros_like(self.vg)
+                nrb.kernel_convolution_cubic(img, 1, self.line, pix, 5.0, 1, stream=self.stream)
+                nrb.convolve_voxel_based_gradient(self.ws, self.vg, self.node, 0.995, stream=self.stream)
+                v = nrb.nmi_value(self.nmi, self.g, self.ref, self.war, stream=self.stream)
+                nrb.nmi_voxel_gradient(self.nmi, self.g, self.ref, self.war, self.vg, out, stream=self.stream)
+                self.stream.synchronize()
+                return [t.cpu().numpy() for t in (img, self.node, out)] + [v]
+
+        def loop(self):
+            try:
+                for _ in range(200):
+                    assert all(np.array_equal(a, b) for a, b in zip(self.run(), self.want))
+            except BaseException as e:  # reported by the test's own thread
+                self.error = e
+
+    work = [Work(400, 256, 132, 1), Work(150, 240, 68, 2)]
+    threads = [threading.Thread(target=w.loop) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for w in work:
+        if getattr(w, "error", None):
+            raise w.error
+
+
 @pytest.mark.parametrize("fdim", [(2, 2, 2), (1, 5, 4), (3, 2, 9), (40, 7, 5)])
 @pytest.mark.parametrize("pad", [np.nan, 0.0, 3.5])
 def test_trilinear_warp_at_the_volume_border(O, fdim, pad):
