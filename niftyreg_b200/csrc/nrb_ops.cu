@@ -299,12 +299,18 @@ __device__ __forceinline__ void conv_weights(int n, int R, const float *__restri
     __syncthreads();
 }
 
+// Above 48 KB a block's shared memory, static arrays included, is opted into: the batched passes hold
+// a BatchList beside their tile. The opt-in belongs to the function, not to the launch, and other
+// host threads launch it too, so it is one constant and never this launch's size.
+constexpr size_t CONV_STATIC_BYTES = 2048, CONV_SHARED_MAX = 227 * 1024 - CONV_STATIC_BYTES;
+static_assert(sizeof(BatchList) + 128 <= CONV_STATIC_BYTES, "static shared memory of the batched convolution passes");
+
 // Pass along x. A block takes kRows consecutive rows of one component, transposes them into shared
 // memory (column stride kRows + 1: no bank conflict either way; R columns of zeros on either side),
 // and each lane convolves one row; its warps share the outputs, four at a time. The outputs go out
 // through shared memory as one contiguous run. 32 rows while the tile stays small enough for
-// several blocks per SM; long rows take 16 or 8, the warp's other lanes then working on other
-// outputs of the same rows.
+// several blocks per SM; long rows take 16 or 8 (4 when the window is as long as the row, too), the
+// warp's other lanes then working on other outputs of the same rows.
 //
 // One load and a quarter of a weight load per multiply-add, rows copied asynchronously: 182x218x182
 // with a 5-voxel grid (37 samples, 21 taps) takes 55 us (37.7 M warp instructions, issue-bound); it
@@ -317,7 +323,7 @@ __host__ __device__ inline size_t conv_x_bytes(int rows, int nx, int R, int ns) 
 inline int conv_x_rows(int nx, int R, int ns) {
     for (int rows : { 32, 16 })
         if (conv_x_bytes(rows, nx, R, ns) <= 48 * 1024) return rows;
-    return 8;
+    return conv_x_bytes(8, nx, R, ns) <= CONV_SHARED_MAX ? 8 : 4;
 }
 __host__ __device__ inline long long conv_x_units(int rows, int ny, int nz) {
     return 3 * (((long long)ny * nz + rows - 1) / rows);
@@ -1750,11 +1756,7 @@ static void conv_kernels(const nrb_workspace *ws, const nrb_geometry *g, int R[3
         K[i] = ws->d_kernel[i] + (ws->ax[i].radius - R[i]);
     }
 }
-// Above 48 KB a block's shared memory, static arrays included, is opted into: the batched passes hold
-// a BatchList beside their tile. The opt-in belongs to the function, not to the launch, and other
-// host threads launch it too, so it is one constant and never this launch's size.
-constexpr size_t CONV_STATIC_BYTES = 2048, CONV_SHARED_MAX = 227 * 1024 - CONV_STATIC_BYTES;
-static_assert(sizeof(BatchList) + 128 <= CONV_STATIC_BYTES, "static shared memory of the batched convolution passes");
+// opts a convolution kernel into its shared memory (CONV_SHARED_MAX)
 template <typename K>
 static nrb_status conv_smem(K kernel, size_t bytes) {
     if (bytes > CONV_SHARED_MAX) return fail(NRB_ERR_UNSUPPORTED, "convolution: rows and kernel exceed shared memory");
@@ -1788,7 +1790,7 @@ nrb_status launch_convolve_to_nodes(nrb_workspace *ws, const nrb_geometry *g, co
     // x pass: [3][nz][ny][nx] -> [3][nz][ny][nsx]
     const int rows = conv_x_rows(nx, R[0], nsx);
     const size_t xsm = conv_x_bytes(rows, nx, R[0], nsx), ysm = conv_y_bytes(ny, nsx, R[1], nsy);
-    auto kx = rows == 32 ? k_conv_x<32> : rows == 16 ? k_conv_x<16> : k_conv_x<8>;
+    auto kx = rows == 32 ? k_conv_x<32> : rows == 16 ? k_conv_x<16> : rows == 8 ? k_conv_x<8> : k_conv_x<4>;
     NRB_TRY(conv_smem(kx, xsm));
     kx<<<(unsigned)conv_x_units(rows, ny, nz), CONV_X_THREADS, xsm, st>>>(nx, ny, nz, vgrad, ws->d_samples[0], nsx,
                                                                          K[0], R[0], ws->conv1);
@@ -2087,7 +2089,9 @@ nrb_status launch_batch_be_value(const std::vector<BatchPair>& hp, const BatchPa
     return NRB_OK;
 }
 
-static auto batch_conv_x(int rows) { return rows == 32 ? k_b_conv_x<32> : rows == 16 ? k_b_conv_x<16> : k_b_conv_x<8>; }
+static auto batch_conv_x(int rows) {
+    return rows == 32 ? k_b_conv_x<32> : rows == 16 ? k_b_conv_x<16> : rows == 8 ? k_b_conv_x<8> : k_b_conv_x<4>;
+}
 
 // Rows, shared memory and grids of the convolution passes for the largest pair, opted into before a
 // capture begins (a launch refused inside one would abort the level)

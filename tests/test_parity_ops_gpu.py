@@ -329,9 +329,9 @@ def convolve_then_sample(O, v, dim, pix, cdim, cpix, weight):
 
 
 @pytest.mark.parametrize("shape,spacing", [((3, 11, 200), 5.0), ((2, 5, 401), 5.0), ((2, 3, 900), 7.3), ((3, 301, 222), 3.0),
-                                           ((33, 6, 7), 2.5), ((9, 10, 12), 30.0)])
+                                           ((33, 6, 7), 2.5), ((9, 10, 12), 30.0), ((2, 3, 2040), 1020.0)])
 def test_convolve_to_nodes_at_tile_edges(O, shape, spacing):
-    """Rows staged 32, 16 and 8 at a time with a remainder, a y pass in column chunks, outputs not a
+    """Rows staged 32, 16, 8 and 4 at a time with a remainder, a y pass in column chunks, outputs not a
     multiple of four, two samples per node (a spacing that is no whole number of voxels), windows
     longer than the lines; finite gradients, then NaN and infinite ones. The bar of the op above."""
     rng = np.random.default_rng(shape[2])

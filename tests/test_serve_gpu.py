@@ -89,20 +89,23 @@ def test_batch_without_bending_energy_and_one_level(pairs):
         _same(a, b)
 
 
-@pytest.mark.parametrize("shapes", [[(8, 256, 256)] * 2, [(8, 290, 290), (6, 262, 300)], [(4, 40, 400), (5, 36, 500)],
-                                    [(3, 40, 900)]])
-def test_batches_of_wide_volumes_equal_plain(shapes):
+@pytest.mark.parametrize("shapes,spacing", [([(8, 256, 256)] * 2, -5.0), ([(8, 290, 290), (6, 262, 300)], -5.0),
+                                            ([(4, 40, 400), (5, 36, 500)], -5.0), ([(3, 40, 900)], -5.0),
+                                            ([(4, 9, 2040)], -1020.0)])
+def test_batches_of_wide_volumes_equal_plain(shapes, spacing):
     """The batched node convolution at the widths where a block's shared memory nears 48 KB (a y
-    pass in column chunks, 32 rows staged along x), and with 16 and 8 rows: as a batch and as a
+    pass in column chunks, 32 rows staged along x), and with 16, 8 and 4 rows: as a batch and as a
     server's group, bit for bit the plain results."""
     ensure_built()
+    params = _params()
+    params.spacing[0] = spacing
     vols = [phantom.blobs_pair(s, seed=40 + i) for i, s in enumerate(shapes)]
-    want = [nrb.register_host(p.reference, p.floating, p.pixdim, _params()) for p in vols]
-    out = nrb.register_batch([(p.reference, p.floating, p.pixdim) for p in vols], _params(), concurrency=4)
+    want = [nrb.register_host(p.reference, p.floating, p.pixdim, params) for p in vols]
+    out = nrb.register_batch([(p.reference, p.floating, p.pixdim) for p in vols], params, concurrency=4)
     for a, b in zip(out, want):
         _same(a, b)
     with nrb.Server(slots=1) as srv:
-        tickets = [srv.submit(p.reference, p.floating, p.pixdim, _params()) for p in vols]
+        tickets = [srv.submit(p.reference, p.floating, p.pixdim, params) for p in vols]
         for t, b in zip(tickets, want):
             _same(srv.wait(t)[:2], b)
 
