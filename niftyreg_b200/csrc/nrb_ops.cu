@@ -806,14 +806,15 @@ k_conv_lines(float *__restrict__ img, long long outer, int n, int inner, const _
 // not fit a block (the caller then runs the separate passes)
 static bool conv_lines(float *img, int nvol, const int32_t dim[3], int axis, const ConvTaps& taps, int radius,
                        cudaStream_t st, nrb_status *status) {
+    if ((long long)dim[0] * dim[1] >= (1LL << 31)) return false;  // a slice is addressed with an int
     // taps further out than a line is long meet no voxel
     const int n = dim[axis], R = std::min(radius, n - 1);
     const int cols = conv_line_cols(n, R, axis == 0);
+    if (cols == 0) return false;
     const int inner = axis == 0 ? 1 : axis == 1 ? dim[0] : dim[0] * dim[1];
     const long long lines = (long long)nvol * dim[0] * dim[1] * dim[2] / n, outer = lines / inner;
-    const long long blocks = axis == 0 ? (lines + std::max(1, cols) - 1) / std::max(1, cols)
-                                       : outer * ((inner + std::max(1, cols) - 1) / std::max(1, cols));
-    if (cols == 0 || blocks >= (1LL << 31) || (long long)dim[0] * dim[1] >= (1LL << 31)) return false;
+    const long long blocks = axis == 0 ? (lines + cols - 1) / cols : outer * ((inner + cols - 1LL) / cols);
+    if (blocks >= (1LL << 31)) return false;
     ConvTaps K;
     std::copy(taps.k + (radius - R), taps.k + (radius + R + 1), K.k);
     const size_t smem = conv_line_bytes(cols, n, R, axis == 0);

@@ -128,3 +128,23 @@ def test_library_has_no_undefined_internal_symbols():
     out = subprocess.run(["nm", "-C", "-u", nrb.LIB_PATH], capture_output=True, text=True, check=True).stdout
     missing = [l.strip() for l in out.splitlines() if "nrb::" in l]
     assert not missing, missing
+
+
+def test_convolution_of_slices_beyond_32_bits_is_no_division_by_zero():
+    """A slice of 2^32 voxels: the whole-line convolution, whose slices are addressed with 32 bits,
+    leaves it to the separate passes, which here find no device. Host only: with a device the
+    passes would run on the stand-in buffer."""
+    import pytest
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("needs a machine without a device")
+    ensure_built()
+    code = ("import ctypes, niftyreg_b200 as nrb\n"
+            "b = (ctypes.c_float * 8)()\n"
+            "for axis in range(3):\n"
+            "    s = nrb.lib().nrb_kernel_convolution_cubic(b, 1, nrb._I3(65536, 65536, 2), nrb._F3(1, 1, 1),\n"
+            "                                               ctypes.c_float(5.0), axis, None)\n"
+            "    assert s != 0, axis\n")
+    import sys
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stderr)
