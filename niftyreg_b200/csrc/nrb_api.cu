@@ -410,8 +410,8 @@ nrb_status f3d_gradient(nrb_workspace *ws, nrb_nmi *nmi, const nrb_geometry *g, 
         NRB_CUDA(cudaMemsetAsync(node_grad, 0, 3 * nvox(g->cpp_dim) * sizeof(float), st));
     }
     if (be_weight > 0) {
-        if (overlap) NRB_TRY(join_side(ws, st));
-        else NRB_TRY(launch_be_derivatives(ws, g, cpp, st));
+        if (!overlap) return be_gradient(ws, g, cpp, (float)be_weight, node_grad, st);
+        NRB_TRY(join_side(ws, st));
         NRB_TRY(launch_be_accumulate(ws, g, (float)be_weight, node_grad, st));
     }
     return NRB_OK;

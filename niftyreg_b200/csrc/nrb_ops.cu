@@ -2016,26 +2016,51 @@ extern "C" nrb_status nrb_approx_bending_energy(nrb_workspace *ws, const nrb_geo
 namespace nrb {
 // reg_spline_approxBendingEnergyGradient3D, first half: the 18 second-derivative values of
 // every node (grid read, derivatives written)
-nrb_status launch_be_derivatives(nrb_workspace *ws, const nrb_geometry *g, const float *cpp, cudaStream_t st) {
+static nrb_status be_derivatives(const nrb_geometry *g, const float *cpp, float *der, cudaStream_t st) {
     const long long nc = nvox(g->cpp_dim);
     KernelTimer timer(TK_BE_GRADIENT, (12.0 + 72.0) * (double)nc, st);
     k_be_derivatives<<<dim3(grid_for(nc, 128), 3), 128, 0, st>>>(g->cpp_dim[0], g->cpp_dim[1], g->cpp_dim[2],
-                                                        to_mat34(g->cpp_xyz), cpp, be_basis(), ws->be_deriv);
+                                                        to_mat34(g->cpp_xyz), cpp, be_basis(), der);
     NRB_LAUNCHED("k_be_derivatives");
     return NRB_OK;
 }
 
 // second half: the adjoint stencil, node_grad += weight / #nodes * sum (derivatives read,
 // gradient read-modify-write)
-nrb_status launch_be_accumulate(nrb_workspace *ws, const nrb_geometry *g, float weight, float *node_grad,
-                                cudaStream_t st) {
+static nrb_status be_accumulate(const nrb_geometry *g, const float *der, float weight, float *node_grad, cudaStream_t st) {
     const long long nc = nvox(g->cpp_dim);
     KernelTimer timer(TK_BE_GRADIENT, (72.0 + 24.0) * (double)nc, st);
     const float ratio = weight / (float)nc;
-    k_be_accumulate<<<dim3(grid_for(nc, 128), 3), 128, 0, st>>>(g->cpp_dim[0], g->cpp_dim[1], g->cpp_dim[2], ws->be_deriv,
-                                                       be_basis(), ratio, node_grad);
+    k_be_accumulate<<<dim3(grid_for(nc, 128), 3), 128, 0, st>>>(g->cpp_dim[0], g->cpp_dim[1], g->cpp_dim[2], der, be_basis(),
+                                                       ratio, node_grad);
     NRB_LAUNCHED("k_be_accumulate");
     return NRB_OK;
+}
+
+nrb_status launch_be_derivatives(nrb_workspace *ws, const nrb_geometry *g, const float *cpp, cudaStream_t st) {
+    return be_derivatives(g, cpp, ws->be_deriv, st);
+}
+nrb_status launch_be_accumulate(nrb_workspace *ws, const nrb_geometry *g, float weight, float *node_grad,
+                                cudaStream_t st) {
+    return be_accumulate(g, ws->be_deriv, weight, node_grad, st);
+}
+
+// Both halves. The workspace's derivative planes fit the grid that it was made for, with zeros around
+// that grid alone; the planes of any other grid are the call's own.
+nrb_status be_gradient(nrb_workspace *ws, const nrb_geometry *g, const float *cpp, float weight, float *node_grad,
+                       cudaStream_t st) {
+    if (std::equal(g->cpp_dim, g->cpp_dim + 3, ws->g.cpp_dim)) {
+        NRB_TRY(launch_be_derivatives(ws, g, cpp, st));
+        return launch_be_accumulate(ws, g, weight, node_grad, st);
+    }
+    float *der = nullptr;
+    const size_t bytes = (size_t)18 * BePad(g->cpp_dim[0], g->cpp_dim[1], g->cpp_dim[2]).size * 4;
+    NRB_CUDA(tmp_alloc(&der, bytes, st));
+    nrb_status s = check_cuda(cudaMemsetAsync(der, 0, bytes, st), "cudaMemsetAsync");
+    if (s == NRB_OK) s = be_derivatives(g, cpp, der, st);
+    if (s == NRB_OK) s = be_accumulate(g, der, weight, node_grad, st);
+    cudaFreeAsync(der, st);
+    return s;
 }
 
 // ---- batched levels -------------------------------------------------------------------------
@@ -2172,9 +2197,7 @@ extern "C" nrb_status nrb_approx_bending_energy_gradient(nrb_workspace *ws, cons
                                                          const float *cpp, float weight, float *node_grad,
                                                          void *stream) {
     if (!ws || !g || !cpp || !node_grad) return fail(NRB_ERR_INVALID, "nrb_approx_bending_energy_gradient: null pointer");
-    cudaStream_t st = as_stream(stream);
-    NRB_TRY(launch_be_derivatives(ws, g, cpp, st));
-    return launch_be_accumulate(ws, g, weight, node_grad, st);
+    return be_gradient(ws, g, cpp, weight, node_grad, as_stream(stream));
 }
 
 // fred holds two partial arrays of NRB_RED_BLOCKS floats (min | max)

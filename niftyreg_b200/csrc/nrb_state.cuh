@@ -614,6 +614,8 @@ nrb_status launch_be_value(nrb_workspace *ws, const nrb_geometry *g, const float
 nrb_status launch_be_derivatives(nrb_workspace *ws, const nrb_geometry *g, const float *cpp, cudaStream_t st);
 nrb_status launch_be_accumulate(nrb_workspace *ws, const nrb_geometry *g, float weight, float *node_grad,
                                 cudaStream_t st);
+nrb_status be_gradient(nrb_workspace *ws, const nrb_geometry *g, const float *cpp, float weight, float *node_grad,
+                       cudaStream_t st);
 int be_partial_count(const nrb_geometry *g);
 // batched levels (csrc/nrb_tile.cu): a pair's walks as its plain registration would launch them
 nrb_status batch_walks(nrb_workspace *ws, const nrb_nmi *nmi, const nrb_geometry *g, float padding, int flo_margin,

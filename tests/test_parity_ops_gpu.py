@@ -12,7 +12,7 @@ import pytest
 
 import niftyreg_b200 as nrb
 import oracle
-from tests.helpers import ensure_built, make_case
+from tests.helpers import ensure_built, identity_grid, make_case
 
 pytestmark = pytest.mark.gpu
 
@@ -214,6 +214,40 @@ def test_kernel_convolution_cubic_line_lengths(O, dim, spacing):
         assert np.array_equal(np.isnan(out), np.isnan(ref))
         ok = np.isfinite(ref)
         assert np.abs(out[ok] - ref[ok]).max() <= 1e-5 * np.abs(ref[ok]).max()
+
+
+def test_bending_energy_gradient_with_another_grids_workspace(O):
+    """The gradient's scratch comes from any workspace: grids of other dims (longer and thinner, larger,
+    smaller) through one made for 9x10x11 nodes, and that grid again after each. The oracle's bar
+    of the op below, and bit for bit what a workspace of the grid's own gives."""
+    import ctypes
+    pix, rng = (1.0, 1.0, 1.0), np.random.default_rng(8)
+    xyz = nrb.identity_header(pix)
+
+    class Grid:
+        def __init__(self, cdim):
+            rdim = tuple(5 * (n - 3) for n in cdim)
+            cxyz = nrb.identity_header((5.0,) * 3, (-5.0,) * 3)
+            self.g = nrb.make_geometry(rdim, pix, xyz, rdim, pix, xyz, cdim, (5.0,) * 3, cxyz)
+            self.n = 3 * int(np.prod(cdim))
+            cpp = (identity_grid(cdim, cxyz) + rng.normal(0, 2, self.n)).astype(np.float32)
+            self.cpp = dev(cpp)
+            self.ws = nrb.Workspace(self.g)
+            self.own = self.gradient(self.ws)
+            want = O.be_gradient(cpp, cdim, cxyz, 0.05)
+            assert np.abs(self.own - want).max() <= 1e-5 * np.abs(want).max()
+
+        def gradient(self, ws):
+            t = torch.zeros(self.n, dtype=torch.float32, device="cuda")
+            nrb.check(nrb.lib().nrb_approx_bending_energy_gradient(ws.h, ctypes.byref(self.g), nrb._p(self.cpp),
+                                                                   ctypes.c_float(0.05), nrb._p(t), None))
+            return host(t)
+
+    first = Grid((9, 10, 11))
+    for cdim in ((40, 5, 4), (14, 13, 12), (4, 4, 4), (11, 10, 9)):
+        other = Grid(cdim)
+        assert np.array_equal(other.gradient(first.ws), other.own)
+        assert np.array_equal(first.gradient(first.ws), first.own)
 
 
 def test_threads_with_different_sizes_do_not_disturb_each_other():
