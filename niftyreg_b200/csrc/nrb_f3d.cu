@@ -1842,7 +1842,8 @@ private:
 
     // The two directions share nothing but the grids and the squaring number, and at most sizes a
     // kernel of one leaves most of the device idle: the backward direction runs on a stream of its
-    // own between a fork and a join, in the order and with the arithmetic of one stream.
+    // own between a fork and a join, in the order and with the arithmetic of one stream. With the
+    // stage timers on both run on st_, so that a stage's time is that of both directions.
     nrb_status Fork() {
         NRB_CUDA(cudaEventRecord(ev_fork_, st_));
         NRB_CUDA(cudaStreamWaitEvent(side_, ev_fork_, 0));
@@ -2061,7 +2062,7 @@ private:
     bool best_fields_ = false;
     int best_steps_ = 6;
     int64_t fields_n_[2] = { 0, 0 };
-    cudaStream_t side_ = nullptr;  // the backward direction's stream
+    cudaStream_t side_ = nullptr, own_side_ = nullptr;  // the backward direction's stream: own_side_ or st_
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
     unsigned *mm_ = nullptr;
     nrb_objective *obj_ = nullptr;    // device: BE forward, BE backward, NMI forward, NMI backward
@@ -2080,10 +2081,10 @@ private:
 public:
     ~F3d2Registration() {
         // buffers go back on st_: an evaluation that failed between fork and join may still be running
-        if (side_) cudaStreamSynchronize(side_);
+        if (own_side_) cudaStreamSynchronize(own_side_);
         if (ev_fork_) cudaEventDestroy(ev_fork_);
         if (ev_join_) cudaEventDestroy(ev_join_);
-        if (side_) cudaStreamDestroy(side_);
+        if (own_side_) cudaStreamDestroy(own_side_);
         dev_free(mm_, st_);
         dev_free(obj_, st_);
         if (obj_h_) cudaFreeHost(obj_h_);
@@ -2175,7 +2176,8 @@ nrb_status F3d2Registration::Run(const float *ref, const float *flo, const Image
     } else {
         sim_w_ = 1 - penalty;
     }
-    NRB_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
+    NRB_CUDA(cudaStreamCreateWithFlags(&own_side_, cudaStreamNonBlocking));
+    side_ = timing_enabled() ? st_ : own_side_;
     NRB_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     NRB_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
     NRB_CUDA(dev_alloc(&mm_, 2 * sizeof(unsigned), st_));

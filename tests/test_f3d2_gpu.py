@@ -371,3 +371,30 @@ def test_squaring_number_that_rises_with_a_level():
     r = register(pair.reference, pair.floating, mm, 2, 15)[-1]
     s = register(pair.reference, pair.floating, 0.9 * mm, 2, 15)[-1]
     assert abs(r.final_nmi - s.final_nmi) <= 5e-3 * s.final_nmi
+
+
+def test_stage_timers_cover_both_directions():
+    """A pair of very different volumes, and the same pair swapped: a stage's time per evaluation is
+    that of both directions, so it is the same within a factor of two (one direction alone differs
+    by the ratio of the volumes), and timing changes no result."""
+    ensure_built()
+    small, big = phantom.blobs_pair((24, 24, 24), seed=7).reference, phantom.blobs_pair((176, 176, 176), seed=7).reference
+    spix, bpix = (176 / 24,) * 3, (1.0,) * 3
+    sxyz, bxyz = nrb.identity_header(spix), nrb.identity_header(bpix)
+    params = nrb.default_params(levels=1, max_iterations=8, bending_energy=0.005, spacing=(20.0,), ref_bins=32,
+                                flo_bins=32)
+    per = []
+    for a, b in (((small, spix, sxyz), (big, bpix, bxyz)), ((big, bpix, bxyz), (small, spix, sxyz))):
+        plain = nrb.f3d2_register_images(*a, *b, params, warped=False)
+        nrb.timing_enable(True)
+        try:
+            timed = nrb.f3d2_register_images(*a, *b, params, warped=False)
+            stages = {k: nrb.timing_read("f3d2_" + k) for k in ("warp", "nmi", "voxel_gradient", "nodes")}
+        finally:
+            nrb.timing_enable(False)
+        assert np.array_equal(plain[0], timed[0]) and np.array_equal(plain[1], timed[1])
+        assert plain[-1].final_nmi == timed[-1].final_nmi
+        per.append({k: ms / n for k, (n, ms, _) in stages.items()})
+    print("ms per stage:", per)
+    for k in per[0]:
+        assert 0.5 <= per[0][k] / per[1][k] <= 2.0, (k, per)
