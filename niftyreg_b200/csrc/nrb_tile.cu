@@ -266,11 +266,11 @@ __device__ __forceinline__ void column_position(const WalkParams& P, Column& C, 
 // off-diagonal terms the single-precision FMA rounds the same exact value once instead of twice
 // (the two agree except when the exact value falls within 2^-53 of a float rounding boundary)
 // and keeps the conversions off the XU pipe.
-// kDiag: 1 = M has no off-diagonal terms, 0 = general M, -1 = decided by `diag` at run time
-template <int kDiag>
-__device__ __forceinline__ void to_floating_voxel(const Mat34& M, int diag, float x, float y, float z,
-                                                  float& fx, float& fy, float& fz) {
-    if (kDiag == 1 || (kDiag < 0 && diag)) {
+// kDiag: M has no off-diagonal terms
+template <bool kDiag>
+__device__ __forceinline__ void to_floating_voxel(const Mat34& M, float x, float y, float z, float& fx, float& fy,
+                                                  float& fz) {
+    if (kDiag) {
         fx = __fmaf_rn(M.m[0], x, M.m[3]);
         fy = __fmaf_rn(M.m[5], y, M.m[7]);
         fz = __fmaf_rn(M.m[10], z, M.m[11]);
@@ -329,8 +329,8 @@ __device__ __forceinline__ void gather_footprint(unsigned long long tex, int lay
 // fetches each slice's 2x2 footprint with one gather instead of four loads, with no warp vote and
 // no clamped path.
 //
-// A sample is fetched in one step and evaluated in another, so that a walk can have the next
-// slice's fetch in flight while it works on this one.
+// A sample is fetched in one step and evaluated in another: the caller issues its other loads in
+// between.
 struct Footprint {
     float v[2][2][2];  // z, y, x
     float rx, ry, rz;  // position within the footprint
@@ -343,11 +343,11 @@ struct Footprint {
 // runs the clamped path: eight addresses, eight tests). k_objective at 182x218x182: 91 -> 81 us.
 enum Fetch : int { FETCH_ANY = 0, FETCH_NAN = 1, FETCH_TEX = 2 };
 
-template <int kDiag, int kFetch>
+template <bool kDiag, int kFetch>
 __device__ __forceinline__ void fetch_footprint(const float *__restrict__ flo, const FloatingView& V, const Mat34& M,
-                                                int diag, float pad, float x, float y, float z, Footprint& S) {
+                                                float pad, float x, float y, float z, Footprint& S) {
     float fx, fy, fz;
-    to_floating_voxel<kDiag>(M, diag, x, y, z, fx, fy, fz);
+    to_floating_voxel<kDiag>(M, x, y, z, fx, fy, fz);
     float flx, fly, flz;
     const int px = floor_split(fx, flx), py = floor_split(fy, fly), pz = floor_split(fz, flz);
     S.rx = fx - flx;
@@ -487,9 +487,10 @@ __device__ __forceinline__ void flush_hist(const uint32_t *h, int nbins, uint32_
 // count every active voxel's (reference, warped) bin pair into the block's histogram h. Called
 // by every thread of the block.
 //
-// The walk is one slice ahead of itself: the position of slice z + 1 is evaluated and its fetches
-// issued before slice z's are consumed, so a warp always has a slice's gathers in flight. Columns
-// outside the volume walk the nearest inside one and count nothing (no divergence).
+// One slice at a time: the other warps cover a gather's latency. (A walk one slice ahead of itself
+// spilled at 64 registers: registrations of 182x218x182 took 65.1 instead of 66.0 ms, but of 64^3
+// 3.85 instead of 3.73, and an evaluation of 182x218x182 137 instead of 132 us.) Columns outside the
+// volume walk the nearest inside one and count nothing (no divergence).
 template <bool kXs, bool kDiag, int kFetch>
 __device__ __forceinline__ void objective_item(const WalkParams& P, const WalkSmem& S, uint32_t *h, float *X,
                                                int item, const float *__restrict__ ref,
@@ -507,15 +508,13 @@ __device__ __forceinline__ void objective_item(const WalkParams& P, const WalkSm
     const int zstride = P.nx * P.ny;
     int idx = (I.z0 * P.ny + min(C.y, P.ny - 1)) * P.nx + min(C.x, P.nx - 1);
     const float rlim = C.inside ? P.frb : -1.f;  // no reference value counts in an outside column
-    auto issue = [&](int zi, Footprint& F, float& rv) {
+    for (int zi = 0; zi < nzi; ++zi, idx += zstride) {
         float pos[3];
         column_position<kXs>(P, C, S.zb, S.zk, S.zid, zi, pos, X);
-        fetch_footprint<kDiag ? 1 : 0, kFetch>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
-        rv = __ldg(&ref[idx]);
+        Footprint F;
+        fetch_footprint<kDiag, kFetch>(flo, P.fv, P.flo_ijk, P.pad, pos[0], pos[1], pos[2], F);
+        float rv = __ldg(&ref[idx]);
         if (mask != nullptr && __ldg(&mask[idx]) <= -1) rv = -1.f;
-        idx += zstride;
-    };
-    auto count = [&](const Footprint& F, float rv) {
         float w, g[3];
         footprint_value<false>(F, w, g);
         int bin = -1;
@@ -528,12 +527,6 @@ __device__ __forceinline__ void objective_item(const WalkParams& P, const WalkSm
         } else if (bin >= 0) {
             atomicAdd(&h[bin], 1u);
         }
-    };
-    for (int zi = 0; zi < nzi; ++zi) {
-        Footprint F;
-        float rv;
-        issue(zi, F, rv);
-        count(F, rv);
     }
 }
 
@@ -753,7 +746,7 @@ __device__ __forceinline__ void gradient_item(const WalkParams& P, const WalkSme
         if (mask == nullptr || __ldg(&mask[idx]) > -1) {
             Footprint F;
             float w, g[3];
-            fetch_footprint<kDiag ? 1 : 0, kFetch>(flo, P.fv, P.flo_ijk, P.flo_diag, P.pad, pos[0], pos[1], pos[2], F);
+            fetch_footprint<kDiag, kFetch>(flo, P.fv, P.flo_ijk, P.pad, pos[0], pos[1], pos[2], F);
             const float rv = __ldg(&ref[idx]);
             footprint_value<true>(F, w, g);
             if (rv == rv && w == w) {
@@ -1151,7 +1144,7 @@ k_nmi_finalize(FinArgs A, cudaGraphConditionalHandle line) {
 // One voxel per thread and few registers: the kernel waits on its position loads, then on the
 // gather, and the warps of six blocks per SM cover both (a grid-stride loop at
 // 48 registers took 56 us for the warp and 62 us for the gradient of 181x217x181).
-template <bool kGrad, int kDiag, int kFetch>
+template <bool kGrad, bool kDiag, int kFetch>
 __global__ void __launch_bounds__(256, 6)
 k_resample(long long nv, FloatingView V, Mat34 M, float pad, const float *__restrict__ flo, const float *__restrict__ def,
            const int32_t *__restrict__ mask, float *__restrict__ out) {
@@ -1163,7 +1156,7 @@ k_resample(long long nv, FloatingView V, Mat34 M, float pad, const float *__rest
     float w = 0.f, g[3] = { 0.f, 0.f, 0.f };
     if (active) {
         Footprint F;
-        fetch_footprint<kDiag, kFetch>(flo, V, M, 0, pad, x, y, z, F);
+        fetch_footprint<kDiag, kFetch>(flo, V, M, pad, x, y, z, F);
         footprint_value<kGrad>(F, w, g);
     }
     if (kGrad) {
@@ -1249,7 +1242,7 @@ __device__ __forceinline__ float sample_order(const float *__restrict__ flo, int
                                               const Mat34& M, float pad, float x, float y, float z) {
     constexpr int kTaps = kOrder == 3 ? 4 : 2, kOffset = kOrder == 3 ? 1 : 0;
     float fx, fy, fz;
-    to_floating_voxel<0>(M, 0, x, y, z, fx, fy, fz);
+    to_floating_voxel<false>(M, x, y, z, fx, fy, fz);
     const float fp[3] = { fx, fy, fz };
     float w[3][4];
     int first[3];
@@ -1635,7 +1628,7 @@ struct BatchGradientKernel {
 };
 struct ResampleKernel {
     template <bool kGrad, bool kDiag, bool kNan> auto operator()() const {
-        return k_resample<kGrad, kDiag ? 1 : 0, kNan ? FETCH_NAN : FETCH_ANY>;
+        return k_resample<kGrad, kDiag, kNan ? FETCH_NAN : FETCH_ANY>;
     }
 };
 static auto pick_objective(bool trial, bool xs, bool diag, int fetch) {
