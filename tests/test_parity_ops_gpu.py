@@ -392,27 +392,59 @@ def test_convolve_to_nodes_at_tile_edges(O, shape, spacing):
             assert np.abs(out[ok] - ref[ok]).max() <= 1e-5 * np.abs(ref[ok]).max()
 
 
+def nodes_in_float(v, shape, cdim, spacing, weight):
+    """The node gradient of a 1 mm image whose nodes sit on every `spacing`-th voxel, in the float
+    operations of the convolution: per axis and sampled voxel the taps in ascending order, each a
+    fused multiply-add over the values that are not NaN, divided by the sum of their weights; a NaN
+    voxel stays NaN. A node reads one voxel, times the weight. (The product of two floats is exact in
+    long double, and its sum with a third far closer than a float.)"""
+    t = np.abs(np.arange(-2 * spacing, 2 * spacing + 1) / float(spacing))
+    taps = np.where(t < 1, 2.0 / 3.0 - t * t + 0.5 * t * t * t, -(t - 2.0) ** 3 / 6.0).astype(np.float32)
+    out = v.reshape((3,) + shape)
+    for axis in (3, 2, 1):
+        line = np.moveaxis(out, axis, 0)
+        n, res = line.shape[0], []
+        for s in range(0, n, spacing):
+            num, den = np.zeros(line.shape[1:], np.float32), np.zeros(line.shape[1:], np.float32)
+            for k in range(max(0, s - 2 * spacing), min(n - 1, s + 2 * spacing) + 1):
+                w, x = taps[k - s + 2 * spacing], line[k]
+                ok = ~np.isnan(x)
+                fma = (np.longdouble(w) * x.astype(np.longdouble) + num).astype(np.float32)
+                num, den = np.where(ok, fma, num), np.where(ok, den + w, den)
+            res.append(np.where(np.isnan(line[s]), np.float32(np.nan), num / den))
+        out = np.moveaxis(np.stack(res), 0, axis)
+    out = np.where(np.isnan(out).any(0), np.float32(np.nan), out)  # the reorientation mixes the components
+    node = np.zeros((3,) + tuple(cdim[::-1]), np.float32)
+    nz, ny, nx = out.shape[1:]
+    node[:, 1:1 + nz, 1:1 + ny, 1:1 + nx] = out * np.float32(weight * spacing ** 3)
+    return node
+
+
 def test_convolve_to_nodes_nan_free_path_is_exact():
-    """The x pass sums NaN-free rows with a check-free loop and takes the per-tap path (conv_at)
-    for rows holding a NaN; both must give the same bits. A NaN at voxel (0, 3, 0) sends the
-    first block of rows (z = 0, y = 0..7) down the per-tap path; nodes beyond the kernel radius of
-    that voxel along x read those rows' x outputs through the y and z passes, so they must equal
-    the NaN-free run bit for bit."""
+    """Outputs whose window holds no NaN take a check-free sum, the others the per-tap path (conv_at).
+    Against one restatement in float, bit for bit, for a gradient without NaN (the check-free path
+    alone) and with NaN voxels (both paths side by side), and nodes out of a NaN's reach keep their
+    floats."""
     c = make_case(shape=(24, 24, 48), seed=31)
     g = c.geometry()
     rng = np.random.default_rng(31)
     vgrad = rng.normal(0, 1e-3, 3 * c.nvox).astype(np.float32)
     ws = nrb.Workspace(g)
-    a = torch.empty(3 * c.ncp, dtype=torch.float32, device="cuda")
-    b = torch.empty(3 * c.ncp, dtype=torch.float32, device="cuda")
-    nrb.convolve_voxel_based_gradient(ws, dev(vgrad), a, 0.995)
-    v2 = vgrad.copy()
-    v2[3 * 48] = np.nan  # component 0, z = 0, y = 3, x = 0
-    nrb.convolve_voxel_based_gradient(ws, dev(v2), b, 0.995)
+    spoiled = vgrad.copy()
+    spoiled[3 * 48] = np.nan  # component 0, z = 0, y = 3, x = 0
+    scattered = vgrad.copy()
+    scattered[rng.integers(0, 3 * c.nvox, 40)] = np.nan
+    scattered[5 * 48:5 * 48 + 5] = np.nan
     cx, cy, cz = c.cdim
-    na, nb = host(a).reshape(3, cz, cy, cx), host(b).reshape(3, cz, cy, cx)
-    assert not np.array_equal(na[0, :, :, :3], nb[0, :, :, :3])  # the NaN changed the nodes near it
-    assert np.array_equal(na[..., 5:], nb[..., 5:])
+    got = []
+    for v in (vgrad, spoiled, scattered):
+        node = torch.empty(3 * c.ncp, dtype=torch.float32, device="cuda")
+        nrb.convolve_voxel_based_gradient(ws, dev(v), node, 0.5)
+        got.append(host(node).reshape(3, cz, cy, cx))
+        want = nodes_in_float(v, (24, 24, 48), c.cdim, 5, 0.5)
+        assert np.array_equal(got[-1], want, equal_nan=True)
+    assert not np.array_equal(got[0][0, :, :, :3], got[1][0, :, :, :3])  # the NaN changed the nodes near it
+    assert np.array_equal(got[0][..., 5:], got[1][..., 5:])
 
 
 def test_bending_energy(O, case):
