@@ -563,6 +563,10 @@ k_objective(WalkParams P, const float *__restrict__ ref, const float *__restrict
     flush_hist(h, nbins, ghist);
 }
 
+// An intensity as the Parzen windows index with it. Beyond the limits no tap lies in a table (at most
+// 1024 bins), whatever the value; without them the tap indices of an infinite or huge one overflow.
+__device__ __forceinline__ float window_value(float v) { return fminf(fmaxf(v, -16.f), 2048.f); }
+
 // Sum over the 4x4 Parzen window of reg_getVoxelBasedNmiGradient3d (_reg_nmi.cpp:548-571):
 // returns refDeriv + warDeriv - nmi * jointDeriv for a unit spatial gradient. The window's
 // basis values are evaluated once (4 + 4), then its 16 (r, w) pairs are summed in the
@@ -570,6 +574,8 @@ k_objective(WalkParams P, const float *__restrict__ ref, const float *__restrict
 __device__ __forceinline__ double nmi_window(float rv, float wv, const double *logt, int rb, int fb, double nmi) {
     const double *rlog = logt + rb * fb;
     const double *wlog = rlog + rb;
+    rv = window_value(rv);
+    wv = window_value(wv);
     const int r0 = (int)(rv - 1.f), r1 = (int)(rv + 3.f);
     const int w0 = (int)(wv - 1.f), w1 = (int)(wv + 3.f);
     double br[4], dw[4], wl[4];
@@ -653,6 +659,8 @@ __device__ __forceinline__ float nmi_window_f(float rv, float wv, const float *l
         return fmaf(sr, sdw, sbr * sw) - nmi * sj;
     }
     // taps outside the window or the table get weight 0 and a clamped (valid) table index
+    rv = window_value(rv);
+    wv = window_value(wv);
     const int r0 = (int)(rv - 1.f), r1 = (int)(rv + 3.f);
     const int w0 = (int)(wv - 1.f), w1 = (int)(wv + 3.f);
     float rl[4], wl[4];

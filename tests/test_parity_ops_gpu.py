@@ -216,6 +216,45 @@ def test_kernel_convolution_cubic_line_lengths(O, dim, spacing):
         assert np.abs(out[ok] - ref[ok]).max() <= 1e-5 * np.abs(ref[ok]).max()
 
 
+@pytest.mark.parametrize("bins", [68, 212])
+def test_nmi_voxel_gradient_of_intensities_far_outside_the_bins(O, bins):
+    """Infinite and huge intensities on either side lie in no Parzen window: their voxels keep the
+    gradient they had, and the others' floats are those of the same images with NaN in their place
+    (which is skipped). The FP32 window (68 bins) and the FP64 one (a table of 212 is too large for
+    shared memory), and the fused gradient of such a reference."""
+    rng = np.random.default_rng(bins)
+    c = make_case(shape=(12, 14, 16), seed=21, bins=bins)
+    g = c.geometry()
+    far = np.float32([np.inf, -np.inf, 3e9, -3e9, 1e30, 2147483520.0, 2147483648.0, -2147483648.0, 5e3, -40.0])
+    at = rng.permutation(c.nvox)[:4 * far.size].reshape(2, -1)
+    ref, war = c.ref.copy(), rng.uniform(2, bins - 3, c.nvox).astype(np.float32)
+    ref[np.isnan(ref)] = 3.0
+    wgrad, init = (rng.normal(0, 1, 3 * c.nvox).astype(np.float32) for _ in range(2))
+
+    def gradient(r, w):
+        nmi = nrb.Nmi(bins, bins)
+        v = dev(init)
+        nrb.nmi_value(nmi, g, dev(r), dev(w))
+        nrb.nmi_voxel_gradient(nmi, g, dev(r), dev(w), dev(wgrad), v)
+        return host(v).reshape(3, -1)
+
+    def fused(r):
+        nmi, ws = nrb.Nmi(bins, bins), nrb.Workspace(g)
+        v, n = (torch.empty(3 * k, dtype=torch.float32, device="cuda") for k in (c.nvox, c.ncp))
+        nrb.f3d_gradient(ws, nmi, dev(r), dev(c.flo), dev(c.cpp), v, n, 1.0, 0.0)
+        return host(v).reshape(3, -1)
+
+    out = []
+    for values in (np.tile(far, 2), np.full(2 * far.size, np.nan, np.float32)):
+        r, w = ref.copy(), war.copy()
+        r[at[0]], w[at[1]] = values, values
+        out.append((gradient(r, w), fused(r)))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    assert np.array_equal(out[0][0][:, at.ravel()], init.reshape(3, -1)[:, at.ravel()])
+    assert not out[0][1][:, at[0]].any()
+
+
 def test_bending_energy_gradient_with_another_grids_workspace(O):
     """The gradient's scratch comes from any workspace: grids of other dims (longer and thinner, larger,
     smaller) through one made for 9x10x11 nodes, and that grid again after each. The oracle's bar
