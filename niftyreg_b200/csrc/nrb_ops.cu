@@ -379,48 +379,40 @@ k_conv_x(int nx, int ny, int nz, const float *__restrict__ vg, const int *__rest
     conv_x_unit<kRows>(nx, ny, nz, vg, samples, ns, R, out, blockIdx.x, conv_sm, dens, conv_sm + conv_weight_floats(R, ns));
 }
 
-// Pass along y of a [3][nz][ny][inner] array: a block takes `width` columns of one (component, z)
-// slice in shared memory (R rows of zeros above and below), a thread four outputs of a column.
+// Pass along y of a [3][nz][ny][inner] array: a block takes one (component, z) slice in shared memory
+// (R rows of zeros above and below), a thread four outputs of a column.
 constexpr int CONV_Y_THREADS = 256;
-__host__ __device__ inline int conv_y_width(int ny, int inner, int R) {
-    const int most = 48 * 1024 / (4 * (ny + 2 * R));
-    return inner <= most ? inner : (most < 1 ? 1 : most);
-}
-__host__ __device__ inline long long conv_y_units(int ny, int nz, int inner, int R) {
-    const int width = conv_y_width(ny, inner, R);
-    return 3LL * nz * ((inner + width - 1) / width);
-}
 __host__ __device__ inline size_t conv_y_bytes(int ny, int inner, int R, int ns) {
-    return 4 * ((size_t)conv_weight_floats(R, ns) + (size_t)(ny + 2 * R) * conv_y_width(ny, inner, R));
+    return 4 * ((size_t)conv_weight_floats(R, ns) + (size_t)(ny + 2 * R) * inner);
 }
+// A slice pays for its staging where it is small enough for several blocks per SM and gives every
+// thread outputs, and where there are slices enough for the device; the others go through
+// conv_strided_element. 182x218x182 with a 5-voxel grid: 75 us for all passes against 79 without
+// the tile, 181x217x181 with a 2.5-voxel grid 214 against 231. Slices cut into column chunks took
+// 169 against 164 us at 256x256x256 and 596 against 581 at 512x512x320, slices of three columns
+// 40 against 21 at 3x4x1900, and twelve slices 33 against 27 at 512x512x4.
+inline bool conv_y_tile(int ny, int inner, int R, int ns) {
+    return (long long)(ny + 2 * R) * inner <= 12 * 1024 && (ns + 3) / 4 * inner >= CONV_Y_THREADS;
+}
+inline bool conv_y_enough(long long slices) { return slices >= 2LL * sm_count(); }
 
 __device__ __forceinline__ void conv_y_unit(int ny, int inner, const float *__restrict__ in,
                                             const int *__restrict__ samples, int ns, int R, float *__restrict__ out,
-                                            long long unit, const float *w, const float *dens, float *tile) {
-    const int width = conv_y_width(ny, inner, R), chunks = (inner + width - 1) / width;
-    const long long slice = unit / chunks;  // component * nz + z
-    const int i0 = (int)(unit - slice * chunks) * width, wd = min(width, inner - i0);
-    const float *src = in + slice * ny * inner + i0;
-    float *body = tile + R * wd;
-    if (wd == inner) {
+                                            long long slice, const float *w, const float *dens, float *tile) {
+    const float *src = in + slice * ny * inner;
+    float *body = tile + R * inner;
 #pragma unroll 4
-        for (int i = threadIdx.x; i < ny * inner; i += CONV_Y_THREADS) __pipeline_memcpy_async(body + i, src + i, 4);
-    } else {
-        for (int i = threadIdx.x; i < ny * wd; i += CONV_Y_THREADS) {
-            const int y = i / wd;
-            __pipeline_memcpy_async(body + i, src + (long long)y * inner + (i - y * wd), 4);
-        }
-    }
+    for (int i = threadIdx.x; i < ny * inner; i += CONV_Y_THREADS) __pipeline_memcpy_async(body + i, src + i, 4);
     __pipeline_commit();
-    for (int i = threadIdx.x; i < R * wd; i += CONV_Y_THREADS) tile[i] = body[ny * wd + i] = 0.f;
+    for (int i = threadIdx.x; i < R * inner; i += CONV_Y_THREADS) tile[i] = body[ny * inner + i] = 0.f;
     __pipeline_wait_prior(0);
     __syncthreads();
-    float *dst = out + slice * ns * inner + i0;
-    for (int e = threadIdx.x; e < (ns + 3) / 4 * wd; e += CONV_Y_THREADS) {
-        const int q = e / wd, ii = e - q * wd;
+    float *dst = out + slice * ns * inner;
+    for (int e = threadIdx.x; e < (ns + 3) / 4 * inner; e += CONV_Y_THREADS) {
+        const int q = e / inner, ii = e - q * inner;
         const float *col = body + ii;
         float v[4];
-        conv_outputs4(ny, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * wd]; }, v);
+        conv_outputs4(ny, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * inner]; }, v);
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (4 * q + u < ns) dst[(long long)(4 * q + u) * inner + ii] = v[u];
@@ -436,19 +428,19 @@ k_conv_y(int ny, int inner, const float *__restrict__ in, const int *__restrict_
     conv_y_unit(ny, inner, in, samples, ns, R, out, blockIdx.x, conv_sm, dens, conv_sm + conv_weight_floats(R, ns));
 }
 
-// Pass along z of a [3][nz][inner] array, one output per thread, element = (component, sample,
-// column): reads are coalesced over the columns and shared by a column's samples in L1. The array is
-// small by now (y and x are sampled): four outputs per thread left too few warps and staged weights
-// cost more than they saved (14 and 12 us against 9).
-__host__ __device__ inline long long conv_z_elements(int ns, int inner) { return 3LL * ns * inner; }
-
-__device__ __forceinline__ void conv_z_element(int nz, int inner, const float *__restrict__ in,
-                                               const int *__restrict__ samples, int ns, const float *__restrict__ K, int R,
-                                               float *__restrict__ out, long long e) {
+// Pass along the middle axis of an [outer][len][inner] array, one output per thread, element =
+// (outer, sample, column): reads are coalesced over the columns and shared by a column's samples in
+// L1. The z pass (its array is small, y and x being sampled: four outputs per thread left too few
+// warps and staged weights cost more than they saved, 14 and 12 us against 9), and the y pass of
+// the volumes that conv_y_tile leaves.
+__device__ __forceinline__ void conv_strided_element(int len, int inner, const float *__restrict__ in,
+                                                     const int *__restrict__ samples, int ns,
+                                                     const float *__restrict__ K, int R, float *__restrict__ out,
+                                                     long long e) {
     const int i32 = (int)e, rest = i32 / inner, ii = i32 - rest * inner;  // < 3 x voxels, below 2^31
     const int c = rest / ns, s = __ldg(&samples[rest - c * ns]);
-    const float *col = in + (long long)c * nz * inner + ii;
-    const int k0 = max(0, s - R), k1 = min(nz - 1, s + R);
+    const float *col = in + (long long)c * len * inner + ii;
+    const int k0 = max(0, s - R), k1 = min(len - 1, s + R);
     const float *p = col + (long long)k0 * inner, *q = K + (k0 - s + R);
     float num = 0.f, den = 0.f;
 #pragma unroll 8
@@ -458,15 +450,15 @@ __device__ __forceinline__ void conv_z_element(int nz, int inner, const float *_
         den += w;
     }
     float v = num / den;
-    if (num != num) v = conv_at(s, nz, R, K, [&](int k) { return __ldg(col + (long long)k * inner); });
+    if (num != num) v = conv_at(s, len, R, K, [&](int k) { return __ldg(col + (long long)k * inner); });
     out[e] = v;
 }
 
 __global__ void __launch_bounds__(256)
-k_conv_z(int nz, int inner, const float *__restrict__ in, const int *__restrict__ samples, int ns,
-         const float *__restrict__ K, int R, float *__restrict__ out) {
+k_conv_strided(long long elements, int len, int inner, const float *__restrict__ in, const int *__restrict__ samples, int ns,
+               const float *__restrict__ K, int R, float *__restrict__ out) {
     const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e < conv_z_elements(ns, inner)) conv_z_element(nz, inner, in, samples, ns, K, R, out, e);
+    if (e < elements) conv_strided_element(len, inner, in, samples, ns, K, R, out, e);
 }
 
 // reg_voxelCentricToNodeCentric (reg-lib/cpu/_reg_localTrans.cpp:1616-1683): trilinear sample
@@ -614,8 +606,8 @@ __global__ void k_b_be_accumulate(const BatchPair *__restrict__ pairs, const Opt
     });
 }
 
-// x, y and z passes of the node convolution: work unit = one block of the plain k_conv_x and
-// k_conv_y; element-wise along z. A block fills its weights when it comes to a pair's first unit.
+// Passes of the node convolution: work unit = one block of the plain k_conv_x and k_conv_y; or one
+// element. A block fills its weights when it comes to a pair's first unit.
 template <int kRows>
 __global__ void __launch_bounds__(CONV_X_THREADS)
 k_b_conv_x(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
@@ -649,7 +641,7 @@ k_b_conv_y(const BatchPair *__restrict__ pairs, const OptState *__restrict__ sta
     batch_list_build(states, npairs, 1u << PH_GRAD,
                      [&](int q, int& u, int& w) {
                          const BatchPair& b = pairs[q];
-                         u = (int)conv_y_units(b.rdim[1], b.rdim[2], b.ns[0], b.radius[1]);
+                         u = 3 * b.rdim[2];
                          w = 1;
                      }, L);
     int k = 0, have = -1;
@@ -667,17 +659,23 @@ k_b_conv_y(const BatchPair *__restrict__ pairs, const OptState *__restrict__ sta
     }
 }
 
-__global__ void k_b_conv_z(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
+// along y (kAxis 1) or z (kAxis 2), element-wise
+template <int kAxis>
+__global__ void k_b_conv_strided(const BatchPair *__restrict__ pairs, const OptState *__restrict__ states, int npairs) {
     __shared__ BatchList L;
     batch_list_build(states, npairs, 1u << PH_GRAD,
                      [&](int q, int& u, int& w) {
                          const BatchPair& b = pairs[q];
-                         u = (int)conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]);
+                         u = 3 * (kAxis == 1 ? b.rdim[2] : b.ns[2]) * b.ns[1] * b.ns[0];
                          w = 1;
                      }, L);
     batch_elements(L, [&](int p, long long e) {
         const BatchPair& P = pairs[p];
-        conv_z_element(P.rdim[2], P.ns[1] * P.ns[0], P.conv2, P.samples[2], P.ns[2], P.kernel[2], P.radius[2], P.conv1, e);
+        if (kAxis == 1)
+            conv_strided_element(P.rdim[1], P.ns[0], P.conv1, P.samples[1], P.ns[1], P.kernel[1], P.radius[1], P.conv2, e);
+        else
+            conv_strided_element(P.rdim[2], P.ns[1] * P.ns[0], P.conv2, P.samples[2], P.ns[2], P.kernel[2], P.radius[2],
+                                 P.conv1, e);
     });
 }
 
@@ -802,8 +800,23 @@ k_conv_lines(float *__restrict__ img, long long outer, int n, int inner, const _
     }
 }
 
+// Whether the whole-line pass of `blocks` blocks beats the separate ones. It does where it fills the
+// device. With fewer blocks its time is a block's own: the taps of a warp's quads one after the other,
+// and along y and z the positions that it copies (0.075 us a tap, eight taps a position). The
+// separate passes take 9 us more per volume and run their taps in every voxel at once (0.056 us a tap
+// and volume, 8e5 taps a us). All in taps of the first kind; 3x4x1900 along z, 481 taps: 54 us
+// separate, 572 whole; 10x1000x9 along y, 161: 37, 124; 64x64x64, 21: 27, 20; 129x65x33 along x,
+// 161: 55, 36; three volumes of 100x101x3 along y, 201: 87, 59.
+static bool conv_lines_pay(int n, int R, int cols, bool along_x, int nvol, long long nvox, long long blocks) {
+    if (blocks >= sm_count()) return true;
+    const int slots = CONV_LINE_THREADS / cols;  // positions of a line that a block works on at once
+    const double taps = 2.0 * R + 1, quads = (n + 3) / 4;
+    const double chain = std::ceil(quads / slots) * taps + (along_x ? 0.0 : 8 * std::ceil((double)n / slots));
+    return chain <= 27 + nvol * (120 + 0.75 * taps + nvox * taps / 6e4);
+}
+
 // whole-volume convolution of nvol volumes along an axis in place; false when a line and its taps do
-// not fit a block (the caller then runs the separate passes)
+// not fit a block or do not pay (the caller then runs the separate passes)
 static bool conv_lines(float *img, int nvol, const int32_t dim[3], int axis, const ConvTaps& taps, int radius,
                        cudaStream_t st, nrb_status *status) {
     if ((long long)dim[0] * dim[1] >= (1LL << 31)) return false;  // a slice is addressed with an int
@@ -814,7 +827,8 @@ static bool conv_lines(float *img, int nvol, const int32_t dim[3], int axis, con
     const int inner = axis == 0 ? 1 : axis == 1 ? dim[0] : dim[0] * dim[1];
     const long long lines = (long long)nvol * dim[0] * dim[1] * dim[2] / n, outer = lines / inner;
     const long long blocks = axis == 0 ? (lines + cols - 1) / cols : outer * ((inner + cols - 1LL) / cols);
-    if (blocks >= (1LL << 31)) return false;
+    if (blocks >= (1LL << 31) ||
+        !conv_lines_pay(n, R, cols, axis == 0, nvol, (long long)dim[0] * dim[1] * dim[2], blocks)) return false;
     ConvTaps K;
     std::copy(taps.k + (radius - R), taps.k + (radius + R + 1), K.k);
     const size_t smem = conv_line_bytes(cols, n, R, axis == 0);
@@ -1548,9 +1562,12 @@ WalkPlan plan_walk(const nrb_geometry *g, int ty, long long (*slots_for)(size_t 
     p.sb = tile_span(ny, ty, gs[1]);
     long long best_cost = LLONG_MAX;
     WalkPlan best = p;
+    int last_chunk = -1;
     for (int c = 1; c <= std::max(1, nz / min_chunk); ++c) {
         WalkPlan q = p;
         q.zchunk = (nz + c - 1) / c;
+        if (q.zchunk == last_chunk) continue;  // the same plan again (an occupancy query each)
+        last_chunk = q.zchunk;
         q.nchunks = (nz + q.zchunk - 1) / q.zchunk;
         q.nitems = (int)(xy * q.nchunks);
         q.sc = tile_span(nz, q.zchunk, gs[2]);
@@ -1790,21 +1807,29 @@ nrb_status launch_convolve_to_nodes(nrb_workspace *ws, const nrb_geometry *g, co
     conv_kernels(ws, g, R, K);
     // x pass: [3][nz][ny][nx] -> [3][nz][ny][nsx]
     const int rows = conv_x_rows(nx, R[0], nsx);
-    const size_t xsm = conv_x_bytes(rows, nx, R[0], nsx), ysm = conv_y_bytes(ny, nsx, R[1], nsy);
+    const size_t xsm = conv_x_bytes(rows, nx, R[0], nsx);
     auto kx = rows == 32 ? k_conv_x<32> : rows == 16 ? k_conv_x<16> : rows == 8 ? k_conv_x<8> : k_conv_x<4>;
     NRB_TRY(conv_smem(kx, xsm));
     kx<<<(unsigned)conv_x_units(rows, ny, nz), CONV_X_THREADS, xsm, st>>>(nx, ny, nz, vgrad, ws->d_samples[0], nsx,
                                                                          K[0], R[0], ws->conv1);
     NRB_LAUNCHED("k_conv_x");
     // y pass: [3][nz][ny][nsx] -> [3][nz][nsy][nsx]
-    NRB_TRY(conv_smem(k_conv_y, ysm));
-    k_conv_y<<<(unsigned)conv_y_units(ny, nz, nsx, R[1]), CONV_Y_THREADS, ysm, st>>>(ny, nsx, ws->conv1, ws->d_samples[1], nsy,
-                                                                              K[1], R[1], ws->conv2);
-    NRB_LAUNCHED("k_conv_y");
+    if (conv_y_tile(ny, nsx, R[1], nsy) && conv_y_enough(3LL * nz)) {
+        const size_t ysm = conv_y_bytes(ny, nsx, R[1], nsy);
+        NRB_TRY(conv_smem(k_conv_y, ysm));
+        k_conv_y<<<3 * nz, CONV_Y_THREADS, ysm, st>>>(ny, nsx, ws->conv1, ws->d_samples[1], nsy, K[1], R[1], ws->conv2);
+        NRB_LAUNCHED("k_conv_y");
+    } else {
+        const long long ey = 3LL * nz * nsy * nsx;
+        k_conv_strided<<<(unsigned)((ey + 255) / 256), 256, 0, st>>>(ey, ny, nsx, ws->conv1, ws->d_samples[1], nsy, K[1],
+                                                                     R[1], ws->conv2);
+        NRB_LAUNCHED("k_conv_strided(y)");
+    }
     // z pass: [3][nz][nsy * nsx] -> [3][nsz][nsy * nsx] (reuses conv1)
-    k_conv_z<<<(unsigned)((conv_z_elements(nsz, nsy * nsx) + 255) / 256), 256, 0, st>>>(
-        nz, nsy * nsx, ws->conv2, ws->d_samples[2], nsz, K[2], R[2], ws->conv1);
-    NRB_LAUNCHED("k_conv_z");
+    const long long ez = 3LL * nsz * nsy * nsx;
+    k_conv_strided<<<(unsigned)((ez + 255) / 256), 256, 0, st>>>(ez, nz, nsy * nsx, ws->conv2, ws->d_samples[2], nsz, K[2],
+                                                                 R[2], ws->conv1);
+    NRB_LAUNCHED("k_conv_strided(z)");
     // node sampling, reorientation (floating ijk) and weighting
     float w = weight;
     for (int i = 0; i < 3; ++i) w *= g->cpp_pixdim[i] / g->ref_pixdim[i];
@@ -2122,16 +2147,19 @@ static auto batch_conv_x(int rows) {
 // Rows, shared memory and grids of the convolution passes for the largest pair, opted into before a
 // capture begins (a launch refused inside one would abort the level)
 nrb_status batch_node_plan(const std::vector<BatchPair>& hp, BatchLaunch& L) {
-    long long xb = 0, yb = 0, zb = 0;
+    long long xb = 0, yb = 0, ye = 0, ze = 0;
     L.conv_rows = 32;
     L.conv_xsm = L.conv_ysm = 0;
+    L.conv_ytile = true;
     for (const BatchPair& b : hp) L.conv_rows = std::min(L.conv_rows, conv_x_rows(b.rdim[0], b.radius[0], b.ns[0]));
     for (const BatchPair& b : hp) {
         L.conv_xsm = std::max(L.conv_xsm, conv_x_bytes(L.conv_rows, b.rdim[0], b.radius[0], b.ns[0]));
         L.conv_ysm = std::max(L.conv_ysm, conv_y_bytes(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]));
+        L.conv_ytile = L.conv_ytile && conv_y_tile(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]);
         xb += conv_x_units(L.conv_rows, b.rdim[1], b.rdim[2]);
-        yb += conv_y_units(b.rdim[1], b.rdim[2], b.ns[0], b.radius[1]);
-        zb += conv_z_elements(b.ns[2], b.ns[1] * b.ns[0]);
+        yb += 3LL * b.rdim[2];
+        ye += 3LL * b.rdim[2] * b.ns[1] * b.ns[0];
+        ze += 3LL * b.ns[2] * b.ns[1] * b.ns[0];
     }
     auto plan = [](auto kernel, long long units, int threads, size_t smem, int& grid) -> nrb_status {
         int per = 0;
@@ -2142,8 +2170,10 @@ nrb_status batch_node_plan(const std::vector<BatchPair>& hp, BatchLaunch& L) {
         return NRB_OK;
     };
     NRB_TRY(plan(batch_conv_x(L.conv_rows), xb, CONV_X_THREADS, L.conv_xsm, L.conv_xgrid));
-    NRB_TRY(plan(k_b_conv_y, yb, CONV_Y_THREADS, L.conv_ysm, L.conv_ygrid));
-    L.conv_zgrid = grid_for(std::max(1LL, zb), 256);
+    L.conv_ytile = L.conv_ytile && conv_y_enough(yb);
+    if (L.conv_ytile) NRB_TRY(plan(k_b_conv_y, yb, CONV_Y_THREADS, L.conv_ysm, L.conv_ygrid));
+    else L.conv_ygrid = grid_for(std::max(1LL, ye), 256);
+    L.conv_zgrid = grid_for(std::max(1LL, ze), 256);
     return NRB_OK;
 }
 
@@ -2169,12 +2199,13 @@ nrb_status launch_batch_node_stage(const std::vector<BatchPair>& hp, const Batch
     batch_conv_x(L.conv_rows)<<<L.conv_xgrid, CONV_X_THREADS, L.conv_xsm, st>>>(d, states, np);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_conv_x");
-    k_b_conv_y<<<L.conv_ygrid, CONV_Y_THREADS, L.conv_ysm, st>>>(d, states, np);
+    if (L.conv_ytile) k_b_conv_y<<<L.conv_ygrid, CONV_Y_THREADS, L.conv_ysm, st>>>(d, states, np);
+    else k_b_conv_strided<1><<<L.conv_ygrid, 256, 0, st>>>(d, states, np);
     NRB_CUDA(cudaGetLastError());
     NRB_LAUNCHED("k_b_conv_y");
-    k_b_conv_z<<<L.conv_zgrid, 256, 0, st>>>(d, states, np);
+    k_b_conv_strided<2><<<L.conv_zgrid, 256, 0, st>>>(d, states, np);
     NRB_CUDA(cudaGetLastError());
-    NRB_LAUNCHED("k_b_conv_z");
+    NRB_LAUNCHED("k_b_conv_strided(z)");
     const int gn = batch_grid(hp, [](const BatchPair& b) { return b.nnode; }, 256, 16);
     k_b_nodes<<<gn, 256, 0, st>>>(d, states, np);
     NRB_CUDA(cudaGetLastError());

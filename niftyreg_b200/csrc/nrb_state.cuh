@@ -214,6 +214,7 @@ struct BatchLaunch {
     // the node stage's convolution (batch_node_plan)
     int conv_rows = 0, conv_xgrid = 0, conv_ygrid = 0, conv_zgrid = 0;
     size_t conv_xsm = 0, conv_ysm = 0;
+    bool conv_ytile = false;
 };
 
 // The pairs a batched stage serves (their phase is in `mask`) with the cost of their work units,

@@ -193,10 +193,12 @@ def test_convolve_to_nodes(O, case):
 
 
 @pytest.mark.parametrize("dim,spacing", [((33, 5, 3), 5.0), ((3, 34, 7), 2.5), ((2, 9, 65), 40.0), ((700, 3, 2), 5.0),
-                                         ((3, 1100, 5), 5.0), ((5, 2, 1500), 5.0), ((7000, 2, 2), 5.0), ((2, 7000, 3), 5.0)])
+                                         ((3, 1100, 5), 5.0), ((5, 2, 1500), 5.0), ((7000, 2, 2), 5.0), ((2, 7000, 3), 5.0),
+                                         ((700, 50, 51), 5.0), ((50, 700, 51), 5.0), ((41, 30, 1500), 5.0),
+                                         ((1500, 41, 30), 5.0)])
 def test_kernel_convolution_cubic_line_lengths(O, dim, spacing):
-    """Lines held 32, 16 and 8 at a time with remainders, windows longer than the line, and lines too
-    long for a block; NaN voxels. The bar of the op above; the allocation-free entry point gives the
+    """Lines held 32, 16 and 8 at a time with remainders, windows longer than the line, lines too
+    long for a block or too few for the device (the separate passes); NaN voxels. The bar of the op above; the allocation-free entry point gives the
     same floats."""
     import ctypes
     rng = np.random.default_rng(sum(dim))
@@ -300,7 +302,7 @@ def test_threads_with_different_sizes_do_not_disturb_each_other():
     class Work:
         def __init__(self, line, width, bins, seed):
             rng = np.random.default_rng(seed)
-            self.line = (40, line, 3)
+            self.line = (40, line, 80)  # blocks enough for the whole-line pass
             self.img = dev(rng.normal(0, 1, int(np.prod(self.line))).astype(np.float32))
             dim = (width, width, 2)
             cdim, cpix, cxyz = nrb.control_grid_header(dim, pix, (5.0, 5.0, 5.0))
@@ -402,10 +404,11 @@ def convolve_then_sample(O, v, dim, pix, cdim, cpix, weight):
 
 
 @pytest.mark.parametrize("shape,spacing", [((3, 11, 200), 5.0), ((2, 5, 401), 5.0), ((2, 3, 900), 7.3), ((3, 301, 222), 3.0),
-                                           ((33, 6, 7), 2.5), ((9, 10, 12), 30.0), ((2, 3, 2040), 1020.0)])
+                                           ((33, 6, 7), 2.5), ((9, 10, 12), 30.0), ((2, 3, 2040), 1020.0),
+                                           ((100, 60, 61), 2.5)])
 def test_convolve_to_nodes_at_tile_edges(O, shape, spacing):
-    """Rows staged 32, 16, 8 and 4 at a time with a remainder, a y pass in column chunks, outputs not a
-    multiple of four, two samples per node (a spacing that is no whole number of voxels), windows
+    """Rows staged 32, 16, 8 and 4 at a time with a remainder, a y pass by whole slices and by single
+    outputs, outputs not a multiple of four, two samples per node (a spacing that is no whole number of voxels), windows
     longer than the lines; finite gradients, then NaN and infinite ones. The bar of the op above."""
     rng = np.random.default_rng(shape[2])
     nz, ny, nx = shape
