@@ -1526,10 +1526,12 @@ static nrb_status make_sampling(const nrb_geometry *g, AxisSampling ax[3]) {
 // A workspace's memory: on its owner's stream when it has one; otherwise from the library's pool as
 // well, usable on any stream once the creator has synchronised, and given back only after the device
 // has finished with it, as cudaFree would wait (mapping and unmapping fresh memory took most of a
-// creation).
+// creation). Parts beyond what the pool keeps mapped are allocated plainly: from the pool, an oblique
+// 512x512x160 workspace took 3.3 ms instead of 2.8.
+static bool ws_plain(size_t bytes, cudaStream_t st) { return !st && bytes > kLibPoolFloor; }
 template <typename T>
 static cudaError_t ws_alloc(T **p, size_t bytes, cudaStream_t st) {
-    return st ? dev_alloc(p, bytes, st) : tmp_alloc(p, bytes, nullptr);
+    return st || ws_plain(bytes, st) ? dev_alloc(p, bytes, st) : tmp_alloc(p, bytes, nullptr);
 }
 
 // Consecutive 256-byte aligned parts of one allocation
@@ -1633,6 +1635,7 @@ static nrb_status workspace_alloc(nrb_workspace *ws) {
         // the whole-volume convolution and per-node sampling replace the separable passes
         ws->general = true;
         const size_t vb = (size_t)3 * nvox(g->ref_dim) * 4;
+        ws->vox_bytes = vb;
         if (ws_alloc(&ws->general_vox, vb, ws->st) != cudaSuccess) {
             cudaGetLastError();
             return fail(NRB_ERR_OOM, "workspace allocation failed");
@@ -1669,6 +1672,7 @@ static nrb_status workspace_alloc(nrb_workspace *ws) {
     const size_t o_conv1 = m.add((size_t)std::max(c1, c3) * 4), o_conv2 = m.add((size_t)c2 * 4), o_be = m.add(be_bytes);
     const size_t o_red = m.add(2 * NRB_RED_BLOCKS * sizeof(double)), o_bep = m.add(NRB_RED_BLOCKS * sizeof(double));
     const size_t o_fred = m.add(2 * NRB_RED_BLOCKS * sizeof(float));
+    ws->scratch_bytes = m.bytes;
     if (ws_alloc(&ws->tables, t.bytes, st) != cudaSuccess || ws_alloc(&ws->scratch, m.bytes, st) != cudaSuccess) {
         cudaGetLastError();
         return fail(NRB_ERR_OOM, "workspace allocation failed");
@@ -1728,8 +1732,13 @@ void workspace_free(nrb_workspace *ws) {
         cudaGetDevice(&cur);
         if (cur != ws->device) cudaSetDevice(ws->device);
         cudaDeviceSynchronize();
-        for (void *p : { (void *)ws->tables, (void *)ws->scratch, (void *)ws->general_vox })
-            if (p) cudaFreeAsync(p, nullptr);
+        auto give_back = [](void *p, size_t bytes) {
+            if (p && ws_plain(bytes, nullptr)) cudaFree(p);
+            else if (p) cudaFreeAsync(p, nullptr);
+        };
+        give_back(ws->tables, 0);  // a few entries per node and axis
+        give_back(ws->scratch, ws->scratch_bytes);
+        give_back(ws->general_vox, ws->vox_bytes);
         if (cur != ws->device) cudaSetDevice(cur);
     }
     // the side stream's work is ordered before st's last join; its frees above are on st

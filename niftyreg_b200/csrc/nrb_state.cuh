@@ -519,6 +519,7 @@ struct nrb_workspace {
     // the allocations: sampling tables (with their host image) and scratch; the pointers below lie in
     // them
     char *tables = nullptr, *scratch = nullptr;
+    size_t scratch_bytes = 0, vox_bytes = 0;
     std::vector<char> table_host;
     // reduction partials (double pairs) and scalars
     double *red = nullptr;          // 2 * NRB_RED_BLOCKS doubles
