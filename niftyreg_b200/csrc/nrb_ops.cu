@@ -733,8 +733,9 @@ __global__ void k_conv_axis(int nx, int ny, int nz, int axis, const float *__res
 // in shared memory (zeros at both ends, lines side by side so that neighbouring lanes read
 // neighbouring banks), convolves them with conv_outputs4 and writes them back. Each value crosses HBM
 // twice; the separate passes moved 28 bytes per voxel and read the taps, the line and its finite
-// flags from global memory tap by tap (182x218x182, 21 taps: 190 us per volume and axis). Taps
-// travel as a kernel argument.
+// flags from global memory tap by tap (182x218x182, 21 taps: 190 us per volume and axis;
+// 512x512x160 along z, 81 taps: 7.6 ms, 0.92 like this; 1024x1024x2 along y, 241 taps: 731 us, 185).
+// Taps travel as a kernel argument.
 struct ConvTaps {
     float k[NRB_STATIC_CONV_MAX_TAPS];
 };
@@ -743,9 +744,16 @@ struct EverySample {
 };
 constexpr int CONV_LINE_THREADS = 256;
 constexpr size_t CONV_LINE_SHARED_MAX = 200 * 1024;
-// shared bytes of a block of `cols` lines; along x the lines are transposed (one column of padding)
+// Floats from one position of `cols` lines to the next. A warp works on quads 4 positions apart, 32 /
+// cols of them: with 10 and 20 floats for 8 and 16 lines they read different banks (packed lines
+// read the same ones four and two at a time). Along x lines are transposed as they are copied, for
+// which an odd stride has no conflict either.
+__host__ __device__ constexpr int conv_line_stride(int cols, bool along_x) {
+    return along_x ? cols + 1 : cols == 8 ? 10 : cols == 16 ? 20 : cols;
+}
+// shared bytes of a block of `cols` lines
 inline size_t conv_line_bytes(int cols, int n, int R, bool along_x) {
-    return 4 * ((size_t)conv_weight_floats(R, n) + (size_t)(n + 2 * R) * (cols + (along_x ? 1 : 0)));
+    return 4 * ((size_t)conv_weight_floats(R, n) + (size_t)(n + 2 * R) * conv_line_stride(cols, along_x));
 }
 inline int conv_line_cols(int n, int R, bool along_x) {
     for (int cols : { 32, 16, 8 })
@@ -759,7 +767,7 @@ template <int kCols, bool kAlongX>
 __global__ void __launch_bounds__(CONV_LINE_THREADS)
 k_conv_lines(float *__restrict__ img, long long outer, int n, int inner, const __grid_constant__ ConvTaps K, int R) {
     extern __shared__ __align__(16) float conv_sm[];
-    constexpr int kStride = kCols + (kAlongX ? 1 : 0), kWarps = CONV_LINE_THREADS / 32, kSub = 32 / kCols;
+    constexpr int kStride = conv_line_stride(kCols, kAlongX), kWarps = CONV_LINE_THREADS / 32, kSub = 32 / kCols;
     float *dens, *w = conv_sm;
     conv_weights(n, R, K.k, EverySample{}, n, w, dens);
     float *body = conv_sm + conv_weight_floats(R, n) + R * kStride;
@@ -801,14 +809,16 @@ k_conv_lines(float *__restrict__ img, long long outer, int n, int inner, const _
 }
 
 // Whether the whole-line pass of `blocks` blocks beats the separate ones. It does where it fills the
-// device. With fewer blocks its time is a block's own: the taps of a warp's quads one after the other,
+// device, unless that takes thousands of blocks of a few positions each, whose set-up then costs more
+// than their voxels (1024x512 lines of 4, 7 and 12 positions along y or z: 74, 80 and 98 us against
+// 47, 75 and 130; along x of 4, 10 and 12: 91, 108 and 111 against 47, 100 and 136). With fewer blocks its time is a block's own: the taps of a warp's quads one after the other,
 // and along y and z the positions that it copies (0.075 us a tap, eight taps a position). The
 // separate passes take 9 us more per volume and run their taps in every voxel at once (0.056 us a tap
 // and volume, 8e5 taps a us). All in taps of the first kind; 3x4x1900 along z, 481 taps: 54 us
 // separate, 572 whole; 10x1000x9 along y, 161: 37, 124; 64x64x64, 21: 27, 20; 129x65x33 along x,
 // 161: 55, 36; three volumes of 100x101x3 along y, 201: 87, 59.
 static bool conv_lines_pay(int n, int R, int cols, bool along_x, int nvol, long long nvox, long long blocks) {
-    if (blocks >= sm_count()) return true;
+    if (blocks >= sm_count()) return blocks <= 4096 || n >= (along_x ? 11 : 8);
     const int slots = CONV_LINE_THREADS / cols;  // positions of a line that a block works on at once
     const double taps = 2.0 * R + 1, quads = (n + 3) / 4;
     const double chain = std::ceil(quads / slots) * taps + (along_x ? 0.0 : 8 * std::ceil((double)n / slots));
