@@ -455,9 +455,11 @@ __global__ void __launch_bounds__(256) k_flow_scale(const float *d, float *out, 
 // per 32 voxels, whatever the layout) and by latency, so the registers are cut to the full 64 warps
 // per SM: a squaring of 182x218x182 takes 93 us at 32 registers, 104 at 48, 116 at 64 (four voxels
 // per thread in the planar layout at 80: 142). Blocks of 32x8, 32x4x2 or 64x4 voxels instead of
-// runs of 256 measured 3 to 7% slower.
+// runs of 256 measured 3 to 7% slower. Planar fields come from a caller and may leave the volume
+// anywhere: their border path is unrolled, at 48 registers (smooth fields take the same time; a field
+// composed with itself until it has left 256x256x256 594 us, 666 like the pairs).
 template <bool kPairs, bool kOutPairs, typename I>
-__global__ void __launch_bounds__(256, 8) k_compose(const float *__restrict__ apply, const float *pos, float *out,
+__global__ void __launch_bounds__(256, kPairs ? 8 : 5) k_compose(const float *__restrict__ apply, const float *pos, float *out,
                                                 FieldGeom f) {
     const I n = (I)f.nx * f.ny * f.nz;
     const I i = (I)blockIdx.x * 256 + threadIdx.x;
@@ -505,10 +507,10 @@ __global__ void __launch_bounds__(256, 8) k_compose(const float *__restrict__ ap
             }
         }
     } else {
-#pragma unroll 1
+#pragma unroll(kPairs ? 1 : 2)
         for (int c = 0; c < 2; ++c) {
             const int z = z0 + c;
-#pragma unroll 1
+#pragma unroll(kPairs ? 1 : 2)
             for (int b = 0; b < 2; ++b) {
                 const int y = y0 + b;
                 const float tb = (b ? ry[1] : ry[0]) * (c ? rz[1] : rz[0]);
