@@ -379,40 +379,60 @@ k_conv_x(int nx, int ny, int nz, const float *__restrict__ vg, const int *__rest
     conv_x_unit<kRows>(nx, ny, nz, vg, samples, ns, R, out, blockIdx.x, conv_sm, dens, conv_sm + conv_weight_floats(R, ns));
 }
 
-// Pass along y of a [3][nz][ny][inner] array: a block takes one (component, z) slice in shared memory
-// (R rows of zeros above and below), a thread four outputs of a column.
+// Pass along y of a [3][nz][ny][inner] array: a block takes one (component, z) slice, or an even share
+// of its columns, in shared memory (R rows of zeros above and below), a thread four outputs of a
+// column.
 constexpr int CONV_Y_THREADS = 256;
+struct ConvY {
+    int width, chunks;  // columns of a block, blocks of a slice
+    __host__ __device__ ConvY(int ny, int inner, int R) {
+        const int most = 12 * 1024 / (ny + 2 * R);
+        chunks = most < 1 ? inner : (inner + most - 1) / most;
+        width = (inner + chunks - 1) / chunks;
+    }
+};
 __host__ __device__ inline size_t conv_y_bytes(int ny, int inner, int R, int ns) {
-    return 4 * ((size_t)conv_weight_floats(R, ns) + (size_t)(ny + 2 * R) * inner);
+    return 4 * ((size_t)conv_weight_floats(R, ns) + (size_t)(ny + 2 * R) * ConvY(ny, inner, R).width);
 }
-// A slice pays for its staging where it is small enough for several blocks per SM and gives every
-// thread outputs, and where there are slices enough for the device; the others go through
-// conv_strided_element. 182x218x182 with a 5-voxel grid: 75 us for all passes against 79 without
-// the tile, 181x217x181 with a 2.5-voxel grid 214 against 231. Slices cut into column chunks took
-// 169 against 164 us at 256x256x256 and 596 against 581 at 512x512x320, slices of three columns
-// 40 against 21 at 3x4x1900, and twelve slices 33 against 27 at 512x512x4.
-inline bool conv_y_tile(int ny, int inner, int R, int ns) {
-    return (long long)(ny + 2 * R) * inner <= 12 * 1024 && (ns + 3) / 4 * inner >= CONV_Y_THREADS;
+// A block pays for its staging where it has a warp's worth of outputs and, when a thread takes more
+// than one, where there is a block for every SM; other volumes go through conv_strided_element. All
+// passes, with the tile and without: 182x218x182 with a 5-voxel grid 74 and 79 us, 512x512x320 with 3
+// voxels 1024 and 1216; 3x4x1900 (three columns a slice) 39 and 20, 100x101x3 with 1 voxel (nine
+// slices) 33 and 24. Even shares: 256x256x256 with 5 voxels 158 us, 169 with as many columns as fit.
+inline bool conv_y_tile(int ny, int inner, int R, int ns, long long slices) {
+    const ConvY C(ny, inner, R);
+    const int quads = (ns + 3) / 4 * C.width;
+    return quads >= 32 && (C.chunks == 1 || C.width >= 16) && (quads <= CONV_Y_THREADS || slices * C.chunks >= sm_count());
 }
-inline bool conv_y_enough(long long slices) { return slices >= 2LL * sm_count(); }
 
 __device__ __forceinline__ void conv_y_unit(int ny, int inner, const float *__restrict__ in,
                                             const int *__restrict__ samples, int ns, int R, float *__restrict__ out,
-                                            long long slice, const float *w, const float *dens, float *tile) {
-    const float *src = in + slice * ny * inner;
-    float *body = tile + R * inner;
+                                            long long unit, const float *w, const float *dens, float *tile) {
+    const ConvY C(ny, inner, R);
+    const long long slice = unit / C.chunks;  // component * nz + z
+    const int i0 = (int)(unit - slice * C.chunks) * C.width, wd = min(C.width, inner - i0);
+    if (wd <= 0) return;
+    const float *src = in + slice * ny * inner + i0;
+    float *body = tile + R * wd;
+    if (wd == inner) {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < ny * inner; i += CONV_Y_THREADS) __pipeline_memcpy_async(body + i, src + i, 4);
+        for (int i = threadIdx.x; i < ny * inner; i += CONV_Y_THREADS) __pipeline_memcpy_async(body + i, src + i, 4);
+    } else {
+        for (int i = threadIdx.x; i < ny * wd; i += CONV_Y_THREADS) {
+            const int y = i / wd;
+            __pipeline_memcpy_async(body + i, src + (long long)y * inner + (i - y * wd), 4);
+        }
+    }
     __pipeline_commit();
-    for (int i = threadIdx.x; i < R * inner; i += CONV_Y_THREADS) tile[i] = body[ny * inner + i] = 0.f;
+    for (int i = threadIdx.x; i < R * wd; i += CONV_Y_THREADS) tile[i] = body[ny * wd + i] = 0.f;
     __pipeline_wait_prior(0);
     __syncthreads();
-    float *dst = out + slice * ns * inner;
-    for (int e = threadIdx.x; e < (ns + 3) / 4 * inner; e += CONV_Y_THREADS) {
-        const int q = e / inner, ii = e - q * inner;
+    float *dst = out + slice * ns * inner + i0;
+    for (int e = threadIdx.x; e < (ns + 3) / 4 * wd; e += CONV_Y_THREADS) {
+        const int q = e / wd, ii = e - q * wd;
         const float *col = body + ii;
         float v[4];
-        conv_outputs4(ny, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * inner]; }, v);
+        conv_outputs4(ny, R, w, dens, samples, ns, 4 * q, [&](int k) { return col[k * wd]; }, v);
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (4 * q + u < ns) dst[(long long)(4 * q + u) * inner + ii] = v[u];
@@ -641,7 +661,7 @@ k_b_conv_y(const BatchPair *__restrict__ pairs, const OptState *__restrict__ sta
     batch_list_build(states, npairs, 1u << PH_GRAD,
                      [&](int q, int& u, int& w) {
                          const BatchPair& b = pairs[q];
-                         u = 3 * b.rdim[2];
+                         u = 3 * b.rdim[2] * ConvY(b.rdim[1], b.ns[0], b.radius[1]).chunks;
                          w = 1;
                      }, L);
     int k = 0, have = -1;
@@ -1833,10 +1853,11 @@ nrb_status launch_convolve_to_nodes(nrb_workspace *ws, const nrb_geometry *g, co
                                                                          K[0], R[0], ws->conv1);
     NRB_LAUNCHED("k_conv_x");
     // y pass: [3][nz][ny][nsx] -> [3][nz][nsy][nsx]
-    if (conv_y_tile(ny, nsx, R[1], nsy) && conv_y_enough(3LL * nz)) {
+    if (conv_y_tile(ny, nsx, R[1], nsy, 3LL * nz)) {
         const size_t ysm = conv_y_bytes(ny, nsx, R[1], nsy);
         NRB_TRY(conv_smem(k_conv_y, ysm));
-        k_conv_y<<<3 * nz, CONV_Y_THREADS, ysm, st>>>(ny, nsx, ws->conv1, ws->d_samples[1], nsy, K[1], R[1], ws->conv2);
+        k_conv_y<<<3 * nz * ConvY(ny, nsx, R[1]).chunks, CONV_Y_THREADS, ysm, st>>>(ny, nsx, ws->conv1, ws->d_samples[1], nsy,
+                                                                                K[1], R[1], ws->conv2);
         NRB_LAUNCHED("k_conv_y");
     } else {
         const long long ey = 3LL * nz * nsy * nsx;
@@ -2166,7 +2187,7 @@ static auto batch_conv_x(int rows) {
 // Rows, shared memory and grids of the convolution passes for the largest pair, opted into before a
 // capture begins (a launch refused inside one would abort the level)
 nrb_status batch_node_plan(const std::vector<BatchPair>& hp, BatchLaunch& L) {
-    long long xb = 0, yb = 0, ye = 0, ze = 0;
+    long long xb = 0, yb = 0, ye = 0, ze = 0, slices = 0;
     L.conv_rows = 32;
     L.conv_xsm = L.conv_ysm = 0;
     L.conv_ytile = true;
@@ -2174,9 +2195,9 @@ nrb_status batch_node_plan(const std::vector<BatchPair>& hp, BatchLaunch& L) {
     for (const BatchPair& b : hp) {
         L.conv_xsm = std::max(L.conv_xsm, conv_x_bytes(L.conv_rows, b.rdim[0], b.radius[0], b.ns[0]));
         L.conv_ysm = std::max(L.conv_ysm, conv_y_bytes(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]));
-        L.conv_ytile = L.conv_ytile && conv_y_tile(b.rdim[1], b.ns[0], b.radius[1], b.ns[1]);
         xb += conv_x_units(L.conv_rows, b.rdim[1], b.rdim[2]);
-        yb += 3LL * b.rdim[2];
+        yb += 3LL * b.rdim[2] * ConvY(b.rdim[1], b.ns[0], b.radius[1]).chunks;
+        slices += 3LL * b.rdim[2];
         ye += 3LL * b.rdim[2] * b.ns[1] * b.ns[0];
         ze += 3LL * b.ns[2] * b.ns[1] * b.ns[0];
     }
@@ -2189,7 +2210,8 @@ nrb_status batch_node_plan(const std::vector<BatchPair>& hp, BatchLaunch& L) {
         return NRB_OK;
     };
     NRB_TRY(plan(batch_conv_x(L.conv_rows), xb, CONV_X_THREADS, L.conv_xsm, L.conv_xgrid));
-    L.conv_ytile = L.conv_ytile && conv_y_enough(yb);
+    for (const BatchPair& b : hp)
+        L.conv_ytile = L.conv_ytile && conv_y_tile(b.rdim[1], b.ns[0], b.radius[1], b.ns[1], slices);
     if (L.conv_ytile) NRB_TRY(plan(k_b_conv_y, yb, CONV_Y_THREADS, L.conv_ysm, L.conv_ygrid));
     else L.conv_ygrid = grid_for(std::max(1LL, ye), 256);
     L.conv_zgrid = grid_for(std::max(1LL, ze), 256);

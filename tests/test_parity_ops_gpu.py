@@ -405,10 +405,10 @@ def convolve_then_sample(O, v, dim, pix, cdim, cpix, weight):
 
 @pytest.mark.parametrize("shape,spacing", [((3, 11, 200), 5.0), ((2, 5, 401), 5.0), ((2, 3, 900), 7.3), ((3, 301, 222), 3.0),
                                            ((33, 6, 7), 2.5), ((9, 10, 12), 30.0), ((2, 3, 2040), 1020.0),
-                                           ((100, 60, 61), 2.5)])
+                                           ((100, 60, 61), 2.5), ((26, 301, 222), 3.0)])
 def test_convolve_to_nodes_at_tile_edges(O, shape, spacing):
-    """Rows staged 32, 16, 8 and 4 at a time with a remainder, a y pass by whole slices and by single
-    outputs, outputs not a multiple of four, two samples per node (a spacing that is no whole number of voxels), windows
+    """Rows staged 32, 16, 8 and 4 at a time with a remainder, a y pass by whole slices, by shares of
+    their columns and by single outputs, outputs not a multiple of four, two samples per node (a spacing that is no whole number of voxels), windows
     longer than the lines; finite gradients, then NaN and infinite ones. The bar of the op above."""
     rng = np.random.default_rng(shape[2])
     nz, ny, nx = shape

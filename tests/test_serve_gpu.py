@@ -89,13 +89,13 @@ def test_batch_without_bending_energy_and_one_level(pairs):
         _same(a, b)
 
 
-@pytest.mark.parametrize("shapes,spacing", [([(8, 256, 256)] * 2, -5.0), ([(8, 290, 290), (6, 262, 300)], -5.0),
+@pytest.mark.parametrize("shapes,spacing", [([(8, 256, 256)] * 4, -5.0), ([(8, 290, 290), (6, 262, 300)], -5.0),
                                             ([(4, 40, 400), (5, 36, 500)], -5.0), ([(3, 40, 900)], -5.0),
                                             ([(4, 9, 2040)], -1020.0), ([(52, 60, 61), (50, 64, 58)], -2.5)])
 def test_batches_of_wide_volumes_equal_plain(shapes, spacing):
     """The batched node convolution at the widths where a block's shared memory nears 48 KB (32 rows
-    staged along x), with 16, 8 and 4 rows, and with a y pass by whole slices: as a batch and as a
-    server's group, bit for bit the plain results."""
+    staged along x), with 16, 8 and 4 rows, and with a y pass by shares of a slice and by whole slices:
+    as a batch and as a server's group, bit for bit the plain results."""
     ensure_built()
     params = _params()
     params.spacing[0] = spacing
